@@ -72,6 +72,12 @@ int launch_split_reduce_scaled(const float* ws, long long stride, int splits, lo
 int launch_w4a4_gemm(const GemmParams& p, const CUtensorMap& tmP, const CUtensorMap& tmQ, int bn, int grid,
                      bool cta_pair, int epi_warps, cudaStream_t st);
 
+// Per-group GEMM on SM pairs over operands expanded to e4m3 in `scratch` (gemm_f8.cu): p as for launch_w4a4_gemm with
+// cta_pair (P = activations), a / b the packed group-major operands, bn 256, 192 or 128.
+long long group_f8_scratch_bytes(long long M, long long N, int G);
+int launch_w4a4_group_f8(const GemmParams& p, const uint8_t* a, const uint8_t* b, uint8_t* scratch, int bn, int device,
+                         int sm_count, cudaStream_t st);
+
 // CUDA-core weight-streaming kernel for M <= 8 tokens (per-group or per-channel scales, 16-bit output).
 // x / w are the packed operands in either layout (rowmajor: [rows, G * 64]; else [G, rows, 64]).
 bool gemv_applicable(long long M, long long N, long long K, int epi_mode);

@@ -22,6 +22,9 @@ static int epi_warps_for(int epi_mode) {
   return 8;
 }
 
+// The expanded operands take one byte per code: beyond this much scratch a call keeps the in-kernel conversion.
+constexpr long long kF8ScratchLimit = 2ll << 30;
+
 struct Shape {
   int bn;
   bool swap;
@@ -33,7 +36,8 @@ struct Shape {
 // weights); otherwise the candidate with the fewest cost-weighted waves wins.  Weights = measured time per output
 // column relative to 256-wide pair tiles at M = 8192 (per-group | per-channel epilogue): 192-wide pair tiles 1.10 | 1.30,
 // 256-wide single tiles 1.05 | 1.20, 128-wide single tiles 1.25 | 1.45.
-static Shape choose_shape(long long M, long long N, int sms, bool allow_swap, bool group_mode, bool pairs_allowed) {
+static Shape choose_shape(long long M, long long N, int sms, bool allow_swap, bool group_mode, bool pairs_allowed,
+                          double* cost_out = nullptr) {
   Shape s;
   s.pair = false;
   s.swap = allow_swap && M <= 64;
@@ -80,7 +84,34 @@ static Shape choose_shape(long long M, long long N, int sms, bool allow_swap, bo
       s.pair = c.pair;
     }
   }
+  if (cost_out != nullptr) *cost_out = best;
   return s;
+}
+
+// Tile width of the expanded per-group kernel (gemm_f8.cu) for an [M, N] problem with G groups, or 0 where converting
+// inside the GEMM is the better choice.  Both sides are estimated from measured times (B200, 1965 MHz): columns of tile
+// that an SM pair works through one after another x groups x 2.81 ns (192 / 128-column tiles: 2 / 8 % more) here,
+// 3.71 ns per cost unit of choose_shape there, 1.27 and 1.5 times that with the zero-point term; the expansion moves 1.5
+// bytes per code at 8 TB/s (mostly L2) and is one more launch.  Measured on both sides of the line (expanded | in-kernel):
+// [200, 4096] x [6144, 4096] 26.0 | 28.7 us, [384, 12288] x [4096, 12288] 54 | 70, [512, 4096] x [6144, 4096] 32 | 35,
+// [300, 256] x [264, 256] 22 | 14.
+static int choose_f8(long long M, long long N, int G, int sms, bool azp) {
+  if (g_force_bn != 0 || g_force_swap >= 0 || g_force_splits != 0 || g_cta_pairs >= 0 || g_epi_warps != 0 ||
+      g_small_m_path != 0 || !g_pairs_launchable.load() || sms < 2)
+    return 0;   // a pinned configuration means the converting kernel
+  if (M <= 128 || (M + N) * (long long)G >= (1ll << 31) - 65536) return 0;
+  int best_bn = 0;
+  double best = 1e30;
+  const struct { int bn; double w; } cands[3] = {{256, 1.00}, {192, 1.02}, {128, 1.08}};
+  for (const auto& c : cands) {
+    const long long tiles = ((M + 255) / 256) * ((N + c.bn - 1) / c.bn), units = sms / 2;
+    const double cost = (double)((tiles + units - 1) / units) * c.bn * c.w;
+    if (cost < best) { best = cost; best_bn = c.bn; }
+  }
+  double in_kernel = 0;
+  choose_shape(M, N, sms, true, true, true, &in_kernel);
+  const double expanded_us = best * G * 0.00281 * (azp ? 1.27 : 1.0) + 2.0 + (double)(M + N) * G * (128 * 1.5 / 8.0e6);
+  return expanded_us < in_kernel * G * 0.00371 * (azp ? 1.5 : 1.0) ? best_bn : 0;
 }
 
 struct DenseArgs {
@@ -98,6 +129,8 @@ struct DenseArgs {
   // zero-point term (per-group mode only): group g adds azp_adj[g, m] * w_col_sum[g, n] to its integer sum
   const float* azp_adj = nullptr;
   const float* w_col_sum = nullptr;
+  uint8_t* scratch = nullptr;   // room for the expanded operands (per-group mode)
+  long long scratch_bytes = 0;
   bool i8_operands = false;   // a and b are int8 [rows, K] (W4A8): no conversion, accumulator unit 1
 };
 
@@ -124,6 +157,27 @@ static int run_dense(const DenseArgs& d, int device, void* stream) {
     if (gemv_ok)
       return launch_w4a4_gemv(d.a, d.b, d.sa, d.sb, d.out, d.out_dtype, d.M, d.N, d.G, d.rowmajor, d.epi_mode,
                               info->sm_count, static_cast<cudaStream_t>(stream));
+  }
+
+  if (d.scratch != nullptr && d.epi_mode == EPI_GROUP) {
+    const int bn = choose_f8(d.M, d.N, d.G, info->sm_count, d.azp_adj != nullptr);
+    if (bn != 0 && d.scratch_bytes >= group_f8_scratch_bytes(d.M, d.N, d.G) && aligned_to(d.scratch, 16)) {
+      GemmParams p;
+      memset(&p, 0, sizeof(p));
+      p.P_rows = (int)d.M; p.Q_rows = (int)d.N; p.G = d.G;
+      p.sp = d.sa; p.sq = d.sb; p.zp = d.azp_adj; p.zq = d.w_col_sum;
+      p.sp_gstride = d.M; p.sq_gstride = d.N;
+      p.epi_mode = EPI_GROUP; p.out_dtype = d.out_dtype; p.out = d.out; p.ldc = d.N;
+      p.num_p_tiles = (int)((d.M + 255) / 256);
+      p.num_q_tiles = (int)((d.N + bn - 1) / bn);
+      p.splits = 1; p.groups_per_split = d.G;
+      p.status = info->status;
+      const int rc = launch_w4a4_group_f8(p, d.a, d.b, d.scratch, bn, device, info->sm_count, static_cast<cudaStream_t>(stream));
+      if (rc == I4TC_OK) return I4TC_OK;
+      // clusters of two cannot be launched here: the kernel below serves the call
+      cudaGetLastError();
+      g_pairs_launchable = false;
+    }
   }
 
   const bool group_mode = d.epi_mode == EPI_GROUP || d.epi_mode == EPI_GROUP_INT32;
@@ -343,6 +397,33 @@ extern "C" int i4tc_gemm_grouped_azp(const uint8_t* a, const uint8_t* b, const f
   DenseArgs d{a, b, scale_a, scale_b, out, I4TC_BF16, M, N, (int)num_groups, false, 0, EPI_GROUP};
   d.azp_adj = azp_adj;
   d.w_col_sum = w_col_sum;
+  return run_dense(d, device, stream);
+}
+
+extern "C" int64_t i4tc_gemm_grouped_scratch_bytes(int64_t M, int64_t N, int64_t num_groups, int azp, int device) {
+  if (M <= 0 || N <= 0 || num_groups <= 0 || num_groups > 512) return 0;
+  const DeviceInfo* info;
+  if (device_info(device, &info) != I4TC_OK) return 0;
+  if (choose_f8(M, N, (int)num_groups, info->sm_count, azp != 0) == 0) return 0;
+  const long long bytes = group_f8_scratch_bytes(M, N, (int)num_groups);
+  return bytes <= kF8ScratchLimit ? bytes : 0;
+}
+
+extern "C" int i4tc_gemm_grouped_scratch(const uint8_t* a, const uint8_t* b, const float* scale_a, const float* scale_b,
+                                         const float* azp_adj, const float* w_col_sum, void* out, int64_t M, int64_t N,
+                                         int64_t group_size, int64_t num_groups, void* scratch, int64_t scratch_bytes,
+                                         int device, void* stream) {
+  I4TC_REQUIRE(group_size == 128, I4TC_EUNSUPPORTED, "fused grouped GEMM only supports group_size=128");
+  I4TC_REQUIRE(num_groups > 0 && num_groups <= 512, I4TC_EINVAL, "num_groups must be in [1, 512]");
+  int rc = check_dense_common(a, b, out, M, N);
+  if (rc) return rc < 0 ? rc : I4TC_OK;
+  I4TC_REQUIRE(scale_a && scale_b, I4TC_EINVAL, "null scale pointer");
+  I4TC_REQUIRE((azp_adj == nullptr) == (w_col_sum == nullptr), I4TC_EINVAL, "azp_adj and w_col_sum belong together");
+  DenseArgs d{a, b, scale_a, scale_b, out, I4TC_BF16, M, N, (int)num_groups, false, 0, EPI_GROUP};
+  d.azp_adj = azp_adj;
+  d.w_col_sum = w_col_sum;
+  d.scratch = static_cast<uint8_t*>(scratch);
+  d.scratch_bytes = scratch != nullptr ? scratch_bytes : 0;
   return run_dense(d, device, stream);
 }
 

@@ -29,16 +29,13 @@
 // one); each stages and converts its own 128 rows of P and only half of the Q rows.
 // Every wait is bounded: on expiry the kernel sets bit 0 of the status word, all roles leave
 // their loops, TMEM is released and the kernel returns.
-#include "gemm.cuh"
-#include "ptx.cuh"
+#include "gemm_dev.cuh"
 
 namespace i4tc {
 
 using namespace ptx;
 
-constexpr int kBM = 128;             // rows of the P tile == TMEM lanes
 constexpr int kPackedRow = 64;       // bytes of one packed row of one group
-constexpr int kI8Row = 128;          // bytes of one int8 row of one group (the swizzle width)
 constexpr int kConvWarp0 = 4, kConvWarps = 4;
 constexpr int kEpiWarp0 = 8;
 constexpr int kNS = 4;               // scale stages (per-group epilogue)
@@ -51,7 +48,6 @@ template <> struct Regs<8> { static constexpr int WG0 = 56, CONV = 64, EPI = 192
 template <> struct Regs<16> { static constexpr int WG0 = 24, CONV = 40, EPI = 104; static constexpr bool PIPE = false; };
 //  12 epilogue warps, 640 threads x 96: 128*56 + 128*64 + 384*120 = 61440 (192-column tiles: 64 running sums per thread)
 template <> struct Regs<12> { static constexpr int WG0 = 56, CONV = 64, EPI = 120; static constexpr bool PIPE = false; };
-constexpr uint64_t kWaitLimitNs = 2000000000ull;  // 2 s
 
 // CG = 1: one CTA computes a 128 x BN tile.  CG = 2: a pair of CTAs (a cluster of two SMs) computes a
 // 256 x BN tile with tcgen05.mma.cta_group::2; each CTA stages its own 128 P rows and only BN / 2 rows of
@@ -95,141 +91,13 @@ struct Cfg {
   static constexpr int SMEM_BYTES = OFF_MISC + 16 + 1024;              // + alignment slack
 };
 
-struct TileInfo {
-  int p0, q0;        // first row of the P / Q tile
-  int p_lim, q_lim;  // exclusive row limits for output
-  int zq;            // slab offset of the Q operand (MoE: expert * G)
-  long long sq_off;  // float offset into sq (MoE: expert * sq_estride)
-  int g0, g1;        // K groups [g0, g1) of this work item (all of them unless split-K)
-  int split;
-};
-
-// Static persistent schedule: CTA b takes tiles b, b + grid, ...  P tiles vary fastest so that
-// CTAs running together share Q (weight) tiles in L2.
-// With CG = 2 a work item is a 256-row P tile of a CTA pair; rank r of the pair owns rows 128 r .. 128 r + 127
-// of it (p.num_p_tiles then counts 256-row tiles).
-template <int CG = 1>
-struct SchedT {
-  int tile;
-  int e;
-  int tile_base;
-  int rank;
-  __device__ SchedT() : tile(blockIdx.x / CG), e(0), tile_base(0), rank(CG == 2 ? (int)cluster_ctarank() : 0) {}
-  template <int BN>
-  __device__ bool next(const GemmParams& p, TileInfo& ti) {
-    if (p.expert_offsets == nullptr) {
-      const int per_split = p.num_p_tiles * p.num_q_tiles;
-      if (tile >= per_split * p.splits) return false;
-      const int sp = tile / per_split, local = tile - sp * per_split;
-      const int pt = local % p.num_p_tiles, qt = local / p.num_p_tiles;
-      ti.p0 = pt * (kBM * CG) + rank * kBM; ti.q0 = qt * BN; ti.p_lim = p.P_rows; ti.q_lim = p.Q_rows; ti.zq = 0; ti.sq_off = 0;
-      ti.split = sp; ti.g0 = sp * p.groups_per_split;
-      ti.g1 = min(p.G, ti.g0 + p.groups_per_split);
-    } else {
-      for (;;) {
-        if (e >= p.num_experts) return false;
-        const int r0 = __ldg(p.expert_offsets + e), r1 = __ldg(p.expert_offsets + e + 1);
-        const int npt = (r1 - r0 + kBM - 1) / kBM;
-        const int nt = npt * p.num_q_tiles;
-        if (tile < tile_base + nt) {
-          const int local = tile - tile_base;
-          const int pt = local % npt, qt = local / npt;
-          ti.p0 = r0 + pt * kBM; ti.p_lim = r1; ti.q0 = qt * BN; ti.q_lim = p.Q_rows;
-          ti.zq = e * p.G; ti.sq_off = (long long)e * p.sq_estride;
-          ti.split = 0; ti.g0 = 0; ti.g1 = p.G;
-          break;
-        }
-        tile_base += nt; ++e;
-      }
-    }
-    tile += gridDim.x / CG;
-    return true;
-  }
-};
 using Sched = SchedT<1>;
-
-// Bounded mbarrier wait, uniform across the warp.  Returns false (and raises the abort flag)
-// when the limit expires or another role has already aborted.  The common case -- the phase has
-// already completed -- is one non-blocking probe; everything else is the rare path.
-__device__ __forceinline__ bool wait_bar_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  bool ok = mbar_try_wait(bar, parity);
-  if (!ok) {
-    const uint64_t t0 = globaltimer_ns();
-    uint32_t spins = 0;
-    for (;;) {
-      ok = mbar_try_wait(bar, parity);
-      if (ok) break;
-      if ((++spins & 63u) == 0) {
-        if (*abort_flag) break;
-        if (globaltimer_ns() - t0 > kWaitLimitNs) break;
-      }
-    }
-  }
-  ok = __all_sync(0xffffffffu, ok);
-  if (!ok) *abort_flag = 1;
-  return ok;
-}
-// The same wait for a role that runs as a single thread (no warp vote).
-__device__ __forceinline__ bool wait_bar_thread(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  if (mbar_test_wait(bar, parity)) return true;
-  bool ok = mbar_try_wait(bar, parity);
-  if (!ok) {
-    const uint64_t t0 = globaltimer_ns();
-    uint32_t spins = 0;
-    for (;;) {
-      ok = mbar_try_wait(bar, parity);
-      if (ok) break;
-      if ((++spins & 63u) == 0) {
-        if (*abort_flag) break;
-        if (globaltimer_ns() - t0 > kWaitLimitNs) break;
-      }
-    }
-  }
-  if (!ok) *abort_flag = 1;
-  return ok;
-}
-__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  if (__all_sync(0xffffffffu, mbar_test_wait(bar, parity))) return true;
-  return wait_bar_slow(bar, parity, abort_flag);
-}
-
-// Arrival on a barrier that, for CG = 2, may live in the peer CTA (`bar` is then a shared::cluster address).
-template <int CG>
-__device__ __forceinline__ void arrive_bar(uint32_t bar) {
-  if (CG == 2) mbar_arrive_cluster(bar);
-  else mbar_arrive(bar);
-}
-
-__device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
-  // K-major, 128-byte swizzle: rows 128 B apart, 8-row groups 1024 B apart (SBO), LBO unused (1),
-  // descriptor version 1 (sm_100), layout type 2 (SWIZZLE_128B).
-  uint64_t d = (uint64_t)((saddr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
 
 template <int BN, int CG>
 __device__ __forceinline__ constexpr uint32_t make_idesc() {
   // D = S32 (2 << 4), A = B = signed int8 (1 << 7, 1 << 10), both K-major, N >> 3 at bit 17, M >> 4 at bit 24.
   return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((kBM * CG) >> 4) << 24);
 }
-
-// Row order of a converted Q tile.  After tcgen05.ld.16x256b a lane (lr, lq) holds, of every 32-column chunk, the column
-// pairs 8 kk + 2 lq + {0, 1}, kk = 0..3.  The converters therefore store Q row n of a 32-row block at row
-// qperm(n) = 8 * ((n >> 1) & 3) + 2 * (n >> 3) + (n & 1): accumulator column 8 kk + 2 lq + e is then output column
-// 8 lq + 2 kk + e, a lane's four pairs are eight CONSECUTIVE output columns, and a chunk row leaves as one 16-byte store
-// per lane with no exchange between lanes (a 4 x 4 transpose in the quad costs 4 shuffles and 16 selects per chunk row).
-// The map is its own inverse.  Tiles that reach shared memory without the converters (int8 operands) keep the
-// natural order (QP = false below).
-__host__ __device__ constexpr int qperm(int n) {
-  return (n & ~31) | (((n >> 1) & 3) << 3) | (((n >> 3) & 3) << 1) | (n & 1);
-}
-// first of the two output columns (inside a 32-column chunk) of a lane's pair kk
-template <bool QP>
-__device__ __forceinline__ constexpr int pair_col(int kk, int lq) { return QP ? lq * 8 + kk * 2 : kk * 8 + lq * 2; }
 
 // Expand the packed P tile (ROWS_P x 64 B, dense) and Q tile (ROWS_Q x 64 B) of one stage into swizzled int8 tiles
 // (rows x 128 B).  16-byte packed chunk j of a row becomes int8 chunks 2j (even codes) and 2j+1 (odd codes).
@@ -268,13 +136,6 @@ __device__ __forceinline__ void convert_stage(uint32_t pkP, uint32_t i8P, uint32
     }
   }
 }
-
-template <typename OutT>
-__device__ __forceinline__ OutT cast_out(float v);
-template <>
-__device__ __forceinline__ __nv_bfloat16 cast_out<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
-template <>
-__device__ __forceinline__ __half cast_out<__half>(float v) { return __float2half_rn(v); }
 
 // Stores 32 consecutive int32 values of one tile row (normal) or of one tile column spread over 32 rows
 // (swap); the accumulators are 256 x the integer sums.
@@ -322,31 +183,6 @@ __device__ __forceinline__ uint4 quad_transpose(const uint32_t (&x)[4], int lq) 
   uint4 y;
   y.x = hi ? t0 : k0; y.y = hi ? t1 : k1; y.z = hi ? k0 : t0; y.w = hi ? k1 : t1;
   return y;
-}
-
-template <typename OutT>
-__device__ __forceinline__ uint32_t pack_pair(float2 v) {
-  union { OutT h[2]; uint32_t u; } pk;
-  pk.h[0] = cast_out<OutT>(v.x); pk.h[1] = cast_out<OutT>(v.y);
-  return pk.u;
-}
-
-// Writes the column pair (q, q + 1) of tile row prow without any alignment assumption beyond what
-// `pair_ok` promises (even ldc, 4-byte aligned base): 16-bit output, normal or swapped orientation.
-template <typename OutT, bool SWAP>
-__device__ __forceinline__ void store_pair(OutT* out, long long ldc, int prow, int q, int q_lim, float2 v, bool pair_ok) {
-  if (!SWAP) {
-    OutT* dst = out + (long long)prow * ldc + q;
-    if (q + 1 < q_lim && pair_ok) {
-      *reinterpret_cast<uint32_t*>(dst) = pack_pair<OutT>(v);
-    } else {
-      if (q < q_lim) dst[0] = cast_out<OutT>(v.x);
-      if (q + 1 < q_lim) dst[1] = cast_out<OutT>(v.y);
-    }
-  } else {
-    if (q < q_lim) out[(long long)q * ldc + prow] = cast_out<OutT>(v.x);
-    if (q + 1 < q_lim) out[(long long)(q + 1) * ldc + prow] = cast_out<OutT>(v.y);
-  }
 }
 
 // ------------------------------------------------------------------------------------------

@@ -306,6 +306,25 @@ def cutlass_w4a8_scaled_mm(a, b_int8, scale_a, scale_b, out, M: int, N: int, K: 
           "cutlass_w4a8_scaled_mm")
 
 
+def _grouped_gemm(a_packed, b_packed, scale_a, scale_b, azp_adj, w_col_sum, out, M, N, group_size, num_groups, who) -> None:
+    """The per-group GEMM, with scratch from torch's caching allocator where the library asks for some (large M).  When
+    there is no memory for it the library's kernel without scratch serves the call."""
+    dev = _dev(out)
+    scratch, nbytes = None, 0
+    if M > 128:
+        nbytes = lib.i4tc_gemm_grouped_scratch_bytes(M, N, num_groups, azp_adj is not None, dev)
+        if nbytes:
+            try:
+                scratch = torch.empty(nbytes, dtype=torch.uint8, device=out.device)
+            except torch.cuda.OutOfMemoryError:
+                nbytes = 0
+    check(lib.i4tc_gemm_grouped_scratch(a_packed.data_ptr(), b_packed.data_ptr(), scale_a.data_ptr(), scale_b.data_ptr(),
+                                        None if azp_adj is None else azp_adj.data_ptr(),
+                                        None if w_col_sum is None else w_col_sum.data_ptr(), out.data_ptr(), M, N,
+                                        group_size, num_groups, None if scratch is None else scratch.data_ptr(), nbytes,
+                                        dev, _stream(out)), who)
+
+
 def cutlass_int4_fused_grouped_gemm(a_packed, b_packed, scale_a, scale_b, out, M: int, N: int,
                                     group_size: int, num_groups: int) -> None:
     """Per-group-128 fused linear into the caller's bf16 ``out`` [M,N].
@@ -320,9 +339,8 @@ def cutlass_int4_fused_grouped_gemm(a_packed, b_packed, scale_a, scale_b, out, M
     _require(b_packed.numel() == num_groups * N * 64, "b_packed must be [G, N, 64]")
     _f32(scale_a, "scale_a", num_groups * M)
     _f32(scale_b, "scale_b", num_groups * N)
-    check(lib.i4tc_gemm_grouped(a_packed.data_ptr(), b_packed.data_ptr(), scale_a.data_ptr(),
-                                scale_b.data_ptr(), out.data_ptr(), M, N, group_size, num_groups,
-                                _dev(out), _stream(out)), "cutlass_int4_fused_grouped_gemm")
+    _grouped_gemm(a_packed, b_packed, scale_a, scale_b, None, None, out, M, N, group_size, num_groups,
+                  "cutlass_int4_fused_grouped_gemm")
 
 
 # Same contract, different kernels in the reference (int4_gemm.cu:3751, 4073, 4007, 3932).
@@ -360,10 +378,8 @@ def cutlass_int4_fused_grouped_gemm_azp(a_packed, b_packed, scale_a, scale_b, ou
     _f32(scale_b, "scale_b", num_groups * N)
     _f32(azp_adj, "azp_adj", num_groups * M)
     _f32(w_col_sum, "w_col_sum", num_groups * N)
-    check(lib.i4tc_gemm_grouped_azp(a_packed.data_ptr(), b_packed.data_ptr(), scale_a.data_ptr(),
-                                    scale_b.data_ptr(), azp_adj.data_ptr(), w_col_sum.data_ptr(), out.data_ptr(),
-                                    M, N, group_size, num_groups, _dev(out), _stream(out)),
-          "cutlass_int4_fused_grouped_gemm_azp")
+    _grouped_gemm(a_packed, b_packed, scale_a, scale_b, azp_adj, w_col_sum, out, M, N, group_size, num_groups,
+                  "cutlass_int4_fused_grouped_gemm_azp")
 
 
 # Same contract, different kernels in the reference (int4_gemm.cu:3838, 4149).

@@ -203,6 +203,17 @@ int i4tc_gemm_grouped_azp(const uint8_t* a, const uint8_t* b, const float* scale
                           const float* azp_adj, const float* w_col_sum, void* out, int64_t M, int64_t N,
                           int64_t group_size, int64_t num_groups, int device, void* stream);
 
+/* Either of the two GEMMs above (azp_adj = w_col_sum = NULL: the first) with caller-supplied scratch on the device.
+ * With at least i4tc_gemm_grouped_scratch_bytes(...) bytes, 16-byte aligned, large problems expand both operands to
+ * 8-bit floats there and multiply those (the same sums, bit for bit; no conversion inside the GEMM); with less, or
+ * NULL, the call does what i4tc_gemm_grouped(_azp) does.  The scratch is free again when the call's work on `stream` is
+ * done.  i4tc_gemm_grouped_scratch_bytes returns 0 where scratch would not be used. */
+int64_t i4tc_gemm_grouped_scratch_bytes(int64_t M, int64_t N, int64_t num_groups, int azp, int device);
+int i4tc_gemm_grouped_scratch(const uint8_t* a, const uint8_t* b, const float* scale_a, const float* scale_b,
+                              const float* azp_adj, const float* w_col_sum, void* out, int64_t M, int64_t N,
+                              int64_t group_size, int64_t num_groups, void* scratch, int64_t scratch_bytes, int device,
+                              void* stream);
+
 /* int32 partial sums of every group, out [G, M, N]: the integer accumulators that the fused
  * kernel drains.  No reference op exposes them; used to check the integer path bit for bit. */
 int i4tc_gemm_grouped_int32(const uint8_t* a, const uint8_t* b, int32_t* out, int64_t M,

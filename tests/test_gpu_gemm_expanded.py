@@ -1,0 +1,90 @@
+"""GPU: the per-group GEMM over operands expanded to e4m3 (large M, scratch from the caller) gives the same bits as the
+kernel that converts inside, over its three tile widths, both epilogues, ragged and unaligned sizes and extreme codes."""
+import pytest
+import torch
+
+from oracle import w4a4_oracle as O
+from tests.helpers import assert_close_bf16
+
+pytestmark = pytest.mark.gpu
+
+
+def _operands(M, N, G, azp, codes="random", seed=0):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    if codes == "random":
+        a = torch.randint(0, 256, (G, M, 64), dtype=torch.uint8, device="cuda", generator=gen)
+        b = torch.randint(0, 256, (G, N, 64), dtype=torch.uint8, device="cuda", generator=gen)
+    else:   # every code -8 against -8 or 7: the largest sums of either sign
+        a = torch.full((G, M, 64), 0x88, dtype=torch.uint8, device="cuda")
+        b = torch.full((G, N, 64), 0x88, dtype=torch.uint8, device="cuda")
+        b[:, ::2] = 0x77
+    sa = torch.rand(G, M, device="cuda", generator=gen) * 0.1 + 1e-3
+    sb = torch.rand(G, N, device="cuda", generator=gen) * 0.01 + 1e-4
+    z = torch.randint(-8, 9, (G, M), device="cuda", generator=gen).float() if azp else None
+    w = torch.randint(-1024, 897, (G, N), device="cuda", generator=gen).float() if azp else None
+    return a, b, sa, sb, z, w
+
+
+def _call(M, N, G, args, nbytes):
+    from fp8_inference_toolkit_b200 import _cabi
+
+    a, b, sa, sb, z, w = args
+    out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+    # garbage, NaN patterns included: every byte that reaches an output has to be written by the call
+    scratch = torch.full((max(nbytes, 1),), 0x7F, dtype=torch.uint8, device="cuda") if nbytes else None
+    _cabi.check(_cabi.lib.i4tc_gemm_grouped_scratch(
+        a.data_ptr(), b.data_ptr(), sa.data_ptr(), sb.data_ptr(), None if z is None else z.data_ptr(),
+        None if w is None else w.data_ptr(), out.data_ptr(), M, N, 128, G, None if scratch is None else scratch.data_ptr(),
+        nbytes, torch.cuda.current_device(), torch.cuda.current_stream().cuda_stream), "i4tc_gemm_grouped_scratch")
+    return out
+
+
+@pytest.mark.parametrize("azp", [False, True])
+@pytest.mark.parametrize("codes", ["random", "extreme"])
+# tile width 128 (one row tile, ragged N; odd N), 192, 256 (M one past a tile; full tiles and several waves)
+@pytest.mark.parametrize("M,N,G", [(129, 1000, 64), (257, 1001, 20), (512, 512, 32), (130, 9473, 16), (1000, 6144, 32),
+                                   (1537, 2568, 32), (2048, 4096, 32)])
+def test_same_bits_as_the_converting_kernel(M, N, G, codes, azp):
+    from fp8_inference_toolkit_b200 import _cabi, ops
+
+    nbytes = _cabi.lib.i4tc_gemm_grouped_scratch_bytes(M, N, G, int(azp), torch.cuda.current_device())
+    assert nbytes > 0, "this size is meant to take the expanded path"
+    args = _operands(M, N, G, azp, codes, seed=M + N)
+    ref = _call(M, N, G, args, 0)
+    assert torch.equal(_call(M, N, G, args, nbytes), ref)
+    assert torch.equal(_call(M, N, G, args, nbytes - 1), ref)   # too little scratch: the converting kernel again
+    ops.check_status()
+
+
+def test_against_the_oracle():
+    from fp8_inference_toolkit_b200 import ops
+
+    M, N, G = 512, 512, 32
+    a, b, sa, sb, _, _ = _operands(M, N, G, False, seed=5)
+    out = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    ops.cutlass_int4_fused_grouped_gemm(a, b, sa, sb, out, M, N, 128, G)
+    ops.check_status()
+    codes = [O.unpack_int4(t.cpu().numpy().reshape(-1, 64)).reshape(G, -1, 128) for t in (a, b)]
+    ref = O.linear_grouped(codes[0], codes[1], sa.cpu().numpy(), sb.cpu().numpy())
+    assert_close_bf16(out, ref, "expanded")
+    assert torch.equal(out.cpu(), ref)
+
+
+def test_inside_a_captured_graph():
+    """Scratch comes from torch's allocator, so a capture owns it and a replay works on new inputs."""
+    from fp8_inference_toolkit_b200 import ops
+
+    M, N, G = 512, 512, 32
+    a, b, sa, sb, _, _ = _operands(M, N, G, False, seed=6)
+    out = torch.zeros(M, N, dtype=torch.bfloat16, device="cuda")
+    run = lambda: ops.cutlass_int4_fused_grouped_gemm(a, b, sa, sb, out, M, N, 128, G)
+    run()
+    g = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g):
+        run()
+    a.copy_(a.flip(1))
+    g.replay()
+    replayed = out.clone()
+    run()
+    assert torch.equal(replayed, out)
