@@ -202,6 +202,34 @@ def rmsnorm_int4_quant_grouped(input: torch.Tensor, norm_weight: torch.Tensor, e
     return packed, scale
 
 
+def rmsnorm(input: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
+    """``bf16(bf16(x * rsqrt(mean(x^2) + eps)) * weight)`` over the last dimension of contiguous bf16 rows."""
+    _require(input.is_cuda and input.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16, "input and weight must be bfloat16 CUDA tensors")
+    _require(input.is_contiguous() and weight.is_contiguous() and weight.numel() == input.shape[-1], "input and weight must be contiguous")
+    _same_device(input, weight)
+    out = torch.empty_like(input)
+    K = input.shape[-1]
+    check(lib.i4tc_rmsnorm(input.data_ptr(), input.numel() // K if K else 0, K, K, weight.data_ptr(), float(eps), out.data_ptr(),
+                           _dev(input), _stream(input)), "rmsnorm")
+    return out
+
+
+def qk_norm_rope_(qkv: torch.Tensor, q_weight: torch.Tensor, k_weight: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor,
+                  q_heads: int, kv_heads: int, seq: int, eps: float) -> torch.Tensor:
+    """In place on the query and key heads (of 128) of contiguous bf16 ``qkv`` [tokens, heads * 128]: RMSNorm per head, then
+    the rotary embedding at position ``token % seq`` (tables bf16 [seq, 64])."""
+    _cuda2d(qkv, "qkv")
+    for t in (qkv, q_weight, k_weight, cos, sin):
+        _require(t.dtype == torch.bfloat16 and t.is_contiguous(), "operands must be contiguous bfloat16")
+    _same_device(qkv, q_weight, k_weight, cos, sin)
+    _require(q_weight.numel() == 128 and k_weight.numel() == 128, "heads must have 128 elements")
+    _require(cos.numel() == seq * 64 and sin.numel() == seq * 64, "cos and sin must be [seq, 64]")
+    check(lib.i4tc_qk_norm_rope(qkv.data_ptr(), qkv.shape[0], qkv.shape[1], q_heads, kv_heads, seq, q_weight.data_ptr(),
+                                k_weight.data_ptr(), cos.data_ptr(), sin.data_ptr(), float(eps), _dev(qkv), _stream(qkv)),
+          "qk_norm_rope_")
+    return qkv
+
+
 def int4_quant_with_scales(input: torch.Tensor, scale: torch.Tensor, group_size: int = 0):
     """Quantise with caller-supplied divisors (no reference op; the "identical scales" form used to
     compare codes bit for bit).  ``scale`` [M] -> packed [M,K/2]; ``scale`` [G,M] -> packed [G,M,gs/2]."""

@@ -36,6 +36,11 @@ class RMSNorm(nn.Module):
         self.eps = eps
 
     def forward(self, x):
+        K = x.shape[-1]
+        if (x.is_cuda and x.dtype == self.weight.dtype == torch.bfloat16 and x.is_contiguous() and self.weight.is_contiguous()
+                and x.data_ptr() % 16 == 0 and K % 8 == 0 and 1024 <= K <= 16384 and x.numel() < K << 31
+                and not (torch.is_grad_enabled() and (x.requires_grad or self.weight.requires_grad))):
+            return ops.rmsnorm(x, self.weight, self.eps)
         xf = x.float()
         return (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + self.eps)).to(x.dtype) * self.weight
 
@@ -99,11 +104,18 @@ class Block(nn.Module):
 
     def _attention(self, qkv, B, S, cos, sin):
         cfg = self.cfg
+        # (qkv is this layer's own buffer)
+        fused = cfg.head_dim == 128 and cos.shape == (S, 64) and cos.dtype == torch.bfloat16
+        if fused:
+            ops.qk_norm_rope_(qkv.view(B * S, -1), self.q_norm.weight, self.k_norm.weight, cos, sin, cfg.q_heads,
+                              cfg.kv_heads, S, cfg.eps)
         q, k, v = qkv.split([cfg.q_heads * cfg.head_dim, cfg.kv_heads * cfg.head_dim, cfg.kv_heads * cfg.head_dim], -1)
-        q = self.q_norm(q.view(B, S, cfg.q_heads, cfg.head_dim)).transpose(1, 2)
-        k = self.k_norm(k.view(B, S, cfg.kv_heads, cfg.head_dim)).transpose(1, 2)
-        v = v.view(B, S, cfg.kv_heads, cfg.head_dim).transpose(1, 2)
-        q, k = apply_rope(q, cos, sin), apply_rope(k, cos, sin)
+        q, k, v = (t.view(B, S, -1, cfg.head_dim) for t in (q, k, v))
+        if not fused:
+            q, k = self.q_norm(q), self.k_norm(k)
+        q, k, v = q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2)
+        if not fused:
+            q, k = apply_rope(q, cos, sin), apply_rope(k, cos, sin)
         a = F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=True)
         return a.transpose(1, 2).reshape(B, S, -1)
 

@@ -376,6 +376,19 @@ int i4tc_moe_ep_return_rows(const int32_t* pos_of, int64_t rows, int64_t H, cons
 int i4tc_moe_combine(const void* y, const int32_t* inv_pairs, const float* w, int64_t T,
                      int64_t top_k, int64_t H, void* out, int device, void* stream);
 
+/* ---- bf16 ops around the linears of the prefill harness ------------------- */
+
+/* out [rows, K] = bf16(bf16(x * rsqrt(mean(x^2) + eps)) * weight) of bf16 rows x (row stride ldx elements); K a multiple of
+ * 8 and at most 16384, everything 16-byte aligned. */
+int i4tc_rmsnorm(const void* x, int64_t rows, int64_t K, int64_t ldx, const void* weight, float eps, void* out, int device,
+                 void* stream);
+
+/* RMSNorm and rotary embedding (halves rotated) of the first q_heads + k_heads heads of 128 in every row of bf16
+ * qkv [tokens, ld], in place; the position of a token is token % seq; cos_table / sin_table bf16 [seq, 64]. */
+int i4tc_qk_norm_rope(void* qkv, int64_t tokens, int64_t ld, int64_t q_heads, int64_t k_heads, int64_t seq,
+                      const void* q_weight, const void* k_weight, const void* cos_table, const void* sin_table, float eps,
+                      int device, void* stream);
+
 /* Polls the device-side status word written by bounded waits; 0 if no kernel timed out since
  * the last call, else I4TC_EKERNEL.  Synchronises `stream`. */
 int i4tc_check_status(int device, void* stream);
