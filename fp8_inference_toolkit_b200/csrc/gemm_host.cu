@@ -427,6 +427,18 @@ extern "C" int i4tc_gemm_grouped_scratch(const uint8_t* a, const uint8_t* b, con
   return run_dense(d, device, stream);
 }
 
+extern "C" int i4tc_linear(const void* x, int dtype, int64_t M, int64_t K, int64_t ldx, const uint8_t* w, const float* w_scale,
+                           int per_channel, uint8_t* x_packed, float* x_scale, void* out, int64_t N, void* scratch,
+                           int64_t scratch_bytes, int device, void* stream) {
+  if (per_channel) {
+    if (int rc = i4tc_quant_rowwise(x, dtype, M, K, ldx, x_packed, x_scale, I4TC_ROLE_ACTIVATION, device, stream)) return rc;
+    return i4tc_gemm_scaled(x_packed, w, x_scale, w_scale, out, I4TC_BF16, M, N, K, device, stream);
+  }
+  if (int rc = i4tc_quant_grouped(x, dtype, M, K, ldx, 128, x_packed, x_scale, I4TC_ROLE_ACTIVATION, device, stream)) return rc;
+  return i4tc_gemm_grouped_scratch(x_packed, w, x_scale, w_scale, nullptr, nullptr, out, M, N, 128, K / 128, scratch,
+                                   scratch_bytes, device, stream);
+}
+
 extern "C" int i4tc_gemm_grouped_int32(const uint8_t* a, const uint8_t* b, int32_t* out, int64_t M, int64_t N,
                                        int64_t num_groups, int device, void* stream) {
   I4TC_REQUIRE(num_groups > 0 && num_groups <= 512, I4TC_EINVAL, "num_groups must be in [1, 512]");

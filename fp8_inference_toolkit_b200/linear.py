@@ -111,11 +111,10 @@ class W4A4Int4TCLinearMethod:
         N = layer.output_size_per_partition
         x2d = x.reshape(-1, K)
         M = x2d.shape[0]
-        out = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
         if self.per_channel:
-            xp, xs = ops.dynamic_int4_quant(x2d)
-            ops.cutlass_int4_scaled_mm(xp, layer.weight_int4, xs, layer.weight_scale, out, M, N, K)
+            out = ops.linear(x2d, layer.weight_int4, layer.weight_scale, N, True)
         elif self.asymmetric:
+            out = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
             sm = getattr(layer, "smooth_scale", None)
             xp, xs, azp = ops.dynamic_int4_quant_asymmetric_clipped_grouped(
                 x2d, GROUP_SIZE, self.clip_ratio, None if sm is None else sm.to(x2d.dtype))
@@ -126,11 +125,12 @@ class W4A4Int4TCLinearMethod:
             if sm is not None:
                 x2d = x2d / sm.to(x2d.dtype)
             if self.clip_ratio < 1.0:
+                out = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
                 xp, xs = ops.dynamic_int4_quant_clipped_grouped(x2d, GROUP_SIZE, self.clip_ratio)
+                ops.cutlass_int4_fused_grouped_gemm(xp, layer.weight_int4, xs, layer.weight_scale, out, M, N,
+                                                    GROUP_SIZE, K // GROUP_SIZE)
             else:
-                xp, xs = ops.dynamic_int4_quant_grouped(x2d, GROUP_SIZE)
-            ops.cutlass_int4_fused_grouped_gemm(xp, layer.weight_int4, xs, layer.weight_scale, out, M, N,
-                                                GROUP_SIZE, K // GROUP_SIZE)
+                out = ops.linear(x2d, layer.weight_int4, layer.weight_scale, N, False)
         if out.dtype != x.dtype:
             out = out.to(x.dtype)
         if bias is not None:

@@ -353,6 +353,45 @@ def _grouped_gemm(a_packed, b_packed, scale_a, scale_b, azp_adj, w_col_sum, out,
                                         dev, _stream(out)), who)
 
 
+def _pad256(n: int) -> int:
+    return (n + 255) & ~255
+
+
+def linear(x: torch.Tensor, w_packed: torch.Tensor, w_scale: torch.Tensor, N: int, per_channel: bool) -> torch.Tensor:
+    """Quantise the activations [M,K] and multiply, as ``dynamic_int4_quant(_grouped)`` + ``cutlass_int4_scaled_mm`` /
+    ``cutlass_int4_fused_grouped_gemm`` do, through one library call and one buffer for codes, scales and scratch (a single
+    token spends 20 us of host time in the separate ops).  bf16 [M,N]."""
+    _cuda2d(x, "input")
+    M, K = x.shape
+    if per_channel:
+        _require(K % 64 == 0, "K must be a multiple of 64")
+    else:
+        _require(K % 128 == 0, "K must be divisible by group_size")
+    x = _float_input(x, "input")
+    groups = 1 if per_channel else K // 128
+    _packed(w_packed, "b_packed")
+    _require(w_packed.numel() == N * (K // 2), "b_packed does not have N*K/2 bytes")
+    _f32(w_scale, "scale_b", groups * N)
+    dev = _dev(x)
+    _require(w_packed.device == x.device and w_scale.device == x.device, "all tensors must be on the same device")
+    out = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
+    packed_bytes = _pad256(M * (K // 2))
+    base_bytes = packed_bytes + _pad256(groups * M * 4)
+    extra = lib.i4tc_gemm_grouped_scratch_bytes(M, N, groups, 0, dev) if M > 128 and not per_channel else 0
+    if extra:
+        try:
+            buf = torch.empty(base_bytes + extra, dtype=torch.uint8, device=x.device)
+        except torch.cuda.OutOfMemoryError:
+            extra = 0
+    if not extra:
+        buf = torch.empty(base_bytes, dtype=torch.uint8, device=x.device)
+    at = buf.data_ptr()
+    check(lib.i4tc_linear(x.data_ptr(), _DTYPES[x.dtype], M, K, x.stride(0), w_packed.data_ptr(), w_scale.data_ptr(),
+                          int(per_channel), at, at + packed_bytes, out.data_ptr(), N, at + base_bytes if extra else None,
+                          extra, dev, _stream(x)), "linear")
+    return out
+
+
 def cutlass_int4_fused_grouped_gemm(a_packed, b_packed, scale_a, scale_b, out, M: int, N: int,
                                     group_size: int, num_groups: int) -> None:
     """Per-group-128 fused linear into the caller's bf16 ``out`` [M,N].

@@ -214,6 +214,12 @@ int i4tc_gemm_grouped_scratch(const uint8_t* a, const uint8_t* b, const float* s
                               int64_t group_size, int64_t num_groups, void* scratch, int64_t scratch_bytes, int device,
                               void* stream);
 
+/* The symmetric linear in one call: activations x [M, K] (row stride ldx elements) quantised per token (per_channel) or per
+ * group of 128 into x_packed / x_scale, then i4tc_gemm_scaled or i4tc_gemm_grouped_scratch into bf16 out [M, N]. */
+int i4tc_linear(const void* x, int dtype, int64_t M, int64_t K, int64_t ldx, const uint8_t* w, const float* w_scale,
+                int per_channel, uint8_t* x_packed, float* x_scale, void* out, int64_t N, void* scratch,
+                int64_t scratch_bytes, int device, void* stream);
+
 /* int32 partial sums of every group, out [G, M, N]: the integer accumulators that the fused
  * kernel drains.  No reference op exposes them; used to check the integer path bit for bit. */
 int i4tc_gemm_grouped_int32(const uint8_t* a, const uint8_t* b, int32_t* out, int64_t M,
