@@ -118,8 +118,7 @@ w4a4_group_f8_kernel(const __grid_constant__ GemmParams p, const __grid_constant
     } else if (warp == 1) {
       if (leader) {
         // ---------------- MMA issuer ----------------
-        // (elect.sync, not lane == 0: the compiler then keeps descriptors in uniform registers; an MMA costs the thread
-        // 41 cycles instead of 85)
+        // (elect.sync, not lane == 0: timed, an MMA costs the thread 41 cycles instead of 85)
         if (elect_one()) {
           // D = fp32 (1 << 4), A = B = e4m3 (0), K-major, N >> 3 at bit 17, M >> 4 at bit 24
           constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((kBM * 2) >> 4) << 24);

@@ -685,8 +685,8 @@ w4a4_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ C
     // ---------------- MMA issuer (CG = 2: the leader CTA only) ----------------
     // One thread runs the whole loop: the loop is the serial path of every small tile, and a warp-wide version
     // pays a vote and a reconvergence (~250 cycles) per K group for nothing.
-    // elect.sync, not lane == 0: the compiler then keeps the descriptors in uniform registers and an MMA costs the thread
-    // 41 cycles instead of 85 ([2048, 4096] x [4096, 4096] per channel: 46.6 -> 43.2 us).
+    // elect.sync, not lane == 0: timed, an MMA costs the thread 41 cycles instead of 85 ([2048, 4096] x [4096, 4096] per
+    // channel: 46.6 -> 43.2 us).
     if (leader && elect_one()) {
     constexpr uint32_t idesc = make_idesc<BN, CG>();
     const uint32_t sc_ring = (p.zp != nullptr) ? kNS / 2 : kNS;   // scale stages in the ring (see epilogue_group)

@@ -207,8 +207,9 @@ __device__ __forceinline__ uint32_t pack8(const Vec8<T>& x, const Recip& q, bool
 }
 
 // e**t for t clamped to [-87, 87] as a fixed sequence of correctly rounded fp32 operations (never contracted into
-// fused multiply-adds): n = rint(t * log2(e)); r = (t - n * ln2_hi) - n * ln2_lo; degree-7 Taylor polynomial of r by
-// Horner's rule; times 2**n.  A CPU repeats it bit for bit with plain IEEE single-precision arithmetic.
+// fused multiply-adds): n = rint(t * log2(e)); r = (t - n * ln2_hi) - n * ln2_lo (Cody and Waite's reduction: ln2_hi is ln 2
+// cut to 15 significant bits, so n * ln2_hi is exact, ln2_lo the rest); degree-7 Taylor polynomial of r by Horner's rule;
+// times 2**n.  A CPU repeats it bit for bit with plain IEEE single-precision arithmetic.
 __device__ __forceinline__ float exp_reproducible(float t) {
   t = fminf(fmaxf(t, -87.0f), 87.0f);
   const float n = rintf(__fmul_rn(t, 1.4426950408889634f));
