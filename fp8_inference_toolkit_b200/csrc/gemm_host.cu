@@ -162,6 +162,8 @@ static int run_dense(const DenseArgs& d, int device, void* stream) {
   if (d.scratch != nullptr && d.epi_mode == EPI_GROUP) {
     const int bn = choose_f8(d.M, d.N, d.G, info->sm_count, d.azp_adj != nullptr);
     if (bn != 0 && d.scratch_bytes >= group_f8_scratch_bytes(d.M, d.N, d.G) && aligned_to(d.scratch, 16)) {
+      // (the tensor maps of the other tile kernel check this; here the operands are read by the expansion's 16-byte loads)
+      I4TC_REQUIRE(aligned_to(d.a, 16) && aligned_to(d.b, 16), I4TC_EALIGN, "packed operand must be 16-byte aligned");
       GemmParams p;
       memset(&p, 0, sizeof(p));
       p.P_rows = (int)d.M; p.Q_rows = (int)d.N; p.G = d.G;

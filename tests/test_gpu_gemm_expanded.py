@@ -88,3 +88,30 @@ def test_inside_a_captured_graph():
     replayed = out.clone()
     run()
     assert torch.equal(replayed, out)
+
+
+def test_operands_off_a_16_byte_boundary_are_refused():
+    """On the host, before anything is launched: by the GEMMs and by the one-call linear."""
+    from fp8_inference_toolkit_b200 import ops
+
+    M, N, G = 512, 512, 32
+    a, b, sa, sb, z, w = _operands(M, N, G, True, seed=7)
+    x = torch.randn(M, G * 128, device="cuda").to(torch.bfloat16)
+    out = torch.zeros(M, N, dtype=torch.bfloat16, device="cuda")
+
+    def off(t):
+        flat = torch.zeros(t.numel() + 8, dtype=torch.uint8, device="cuda")
+        flat[8:] = t.reshape(-1)
+        return flat[8:].view(t.shape)
+
+    a8, b8 = off(a), off(b)
+    assert a8.data_ptr() % 16 == b8.data_ptr() % 16 == 8 and a8.is_contiguous() and b8.is_contiguous()
+    for p, q in ((a8, b), (a, b8)):
+        with pytest.raises(RuntimeError, match="16-byte aligned"):
+            ops.cutlass_int4_fused_grouped_gemm(p, q, sa, sb, out, M, N, 128, G)
+        with pytest.raises(RuntimeError, match="16-byte aligned"):
+            ops.cutlass_int4_fused_grouped_gemm_azp(p, q, sa, sb, out, z, w, M, N, 128, G)
+    with pytest.raises(RuntimeError, match="16-byte aligned"):
+        ops.linear(x, b8, sb, N, False)
+    torch.cuda.synchronize()
+    assert not out.any()
