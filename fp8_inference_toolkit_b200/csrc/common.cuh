@@ -28,6 +28,7 @@ inline int fail(int code, const char* fmt, ...) {
 
 inline int cuda_fail(cudaError_t e, const char* what) {
   snprintf(err_buf(), 512, "%s: %s (%s)", what, cudaGetErrorName(e), cudaGetErrorString(e));
+  cudaGetLastError();   // reported here and now: the next call's launch check is not to find it again
   return (int)e;
 }
 

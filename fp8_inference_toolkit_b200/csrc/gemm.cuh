@@ -66,17 +66,32 @@ int launch_split_reduce(const float* ws, long long stride, int splits, long long
 int launch_split_reduce_scaled(const float* ws, long long stride, int splits, long long M, long long N, const float* sa,
                                const float* sb, void* out, int out_dtype, cudaStream_t st);
 
+// What became of a launch of CTA pairs (clusters of two) that did not succeed.
+struct PairLaunch {
+  bool failed = false;        // the launch itself (any other failure is the caller's to see)
+  bool unavailable = false;   // no such cluster can be active on this device at all: a restricted SM partition, for instance
+};
+template <typename Kernel, typename... Args>
+int launch_pairs(const cudaLaunchConfig_t& cfg, PairLaunch* pl, Kernel kernel, const Args&... args) {
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  if (e == cudaSuccess) return I4TC_OK;
+  int active = 0;
+  pl->failed = true;
+  pl->unavailable = cudaOccupancyMaxActiveClusters(&active, kernel, &cfg) == cudaSuccess && active == 0;
+  return cuda_fail(e, "launch of thread block pairs");
+}
+
 // cta_pair: pairs of CTAs compute 256 x 256 tiles (dense, unswapped, bn = 256, even grid; p.num_p_tiles counts
 // 256-row tiles and tmQ has 128-row boxes).
-// epi_warps: 8 or 16 epilogue warps per CTA (16 needs bn >= 128).
+// epi_warps: 8 or 16 epilogue warps per CTA (16 needs bn >= 128).  pl: needed with cta_pair.
 int launch_w4a4_gemm(const GemmParams& p, const CUtensorMap& tmP, const CUtensorMap& tmQ, int bn, int grid,
-                     bool cta_pair, int epi_warps, cudaStream_t st);
+                     bool cta_pair, int epi_warps, cudaStream_t st, PairLaunch* pl = nullptr);
 
 // Per-group GEMM on SM pairs over operands expanded to e4m3 in `scratch` (gemm_f8.cu): p as for launch_w4a4_gemm with
 // cta_pair (P = activations), a / b the packed group-major operands, bn 256, 192 or 128.
 long long group_f8_scratch_bytes(long long M, long long N, int G);
 int launch_w4a4_group_f8(const GemmParams& p, const uint8_t* a, const uint8_t* b, uint8_t* scratch, int bn, int device,
-                         int sm_count, cudaStream_t st);
+                         int sm_count, cudaStream_t st, PairLaunch* pl);
 
 // CUDA-core weight-streaming kernel for M <= 8 tokens (per-group or per-channel scales, 16-bit output).
 // x / w are the packed operands in either layout (rowmajor: [rows, G * 64]; else [G, rows, 64]).

@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(256) expand_e4m3_kernel(const uint8_t* __restr
 
 template <int BN, bool AZP>
 static int launch_f8(const GemmParams& p, const CUtensorMap& tmP, const CUtensorMap& tmQ, int p_pitch, int q_pitch, int grid,
-                     cudaStream_t st) {
+                     cudaStream_t st, PairLaunch* pl) {
   using C = F8Cfg<BN>;
   static_assert(C::SMEM_BYTES <= 232448, "shared memory layout exceeds the 227 KB a CTA may use");
   I4TC_CUDA(cudaFuncSetAttribute(w4a4_group_f8_kernel<BN, AZP>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
@@ -343,8 +343,7 @@ static int launch_f8(const GemmParams& p, const CUtensorMap& tmP, const CUtensor
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  I4TC_CUDA(cudaLaunchKernelEx(&cfg, w4a4_group_f8_kernel<BN, AZP>, p, tmP, tmQ, p_pitch, q_pitch));
-  return I4TC_OK;
+  return launch_pairs(cfg, pl, w4a4_group_f8_kernel<BN, AZP>, p, tmP, tmQ, p_pitch, q_pitch);
 }
 
 long long group_f8_scratch_bytes(long long M, long long N, int G) {
@@ -352,7 +351,7 @@ long long group_f8_scratch_bytes(long long M, long long N, int G) {
 }
 
 int launch_w4a4_group_f8(const GemmParams& p, const uint8_t* a, const uint8_t* b, uint8_t* scratch, int bn, int device,
-                         int sm_count, cudaStream_t st) {
+                         int sm_count, cudaStream_t st, PairLaunch* pl) {
   const int M = p.P_rows, N = p.Q_rows;
   const int m_pitch = (M + 31) & ~31, n_pitch = (N + 31) & ~31;
   uint8_t* ea = scratch;
@@ -367,9 +366,9 @@ int launch_w4a4_group_f8(const GemmParams& p, const uint8_t* a, const uint8_t* b
   const long long tiles = (long long)p.num_p_tiles * p.num_q_tiles;
   const int grid = 2 * (int)(tiles < sm_count / 2 ? tiles : sm_count / 2);
   const bool azp = p.zp != nullptr;
-  if (bn == 256) return azp ? launch_f8<256, true>(p, tmP, tmQ, m_pitch, n_pitch, grid, st) : launch_f8<256, false>(p, tmP, tmQ, m_pitch, n_pitch, grid, st);
-  if (bn == 192) return azp ? launch_f8<192, true>(p, tmP, tmQ, m_pitch, n_pitch, grid, st) : launch_f8<192, false>(p, tmP, tmQ, m_pitch, n_pitch, grid, st);
-  return azp ? launch_f8<128, true>(p, tmP, tmQ, m_pitch, n_pitch, grid, st) : launch_f8<128, false>(p, tmP, tmQ, m_pitch, n_pitch, grid, st);
+  if (bn == 256) return azp ? launch_f8<256, true>(p, tmP, tmQ, m_pitch, n_pitch, grid, st, pl) : launch_f8<256, false>(p, tmP, tmQ, m_pitch, n_pitch, grid, st, pl);
+  if (bn == 192) return azp ? launch_f8<192, true>(p, tmP, tmQ, m_pitch, n_pitch, grid, st, pl) : launch_f8<192, false>(p, tmP, tmQ, m_pitch, n_pitch, grid, st, pl);
+  return azp ? launch_f8<128, true>(p, tmP, tmQ, m_pitch, n_pitch, grid, st, pl) : launch_f8<128, false>(p, tmP, tmQ, m_pitch, n_pitch, grid, st, pl);
 }
 
 }  // namespace i4tc

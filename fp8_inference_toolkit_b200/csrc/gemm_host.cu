@@ -13,7 +13,7 @@ static std::atomic<int> g_force_swap{-1};   // -1 = choose automatically
 static std::atomic<int> g_small_m_path{0};  // 0 = automatic, 1 = CUDA-core kernel only, 2 = register-fed tensor-core kernel whenever it applies, 3 = tile kernel only
 static std::atomic<int> g_force_splits{0};  // 0 = choose automatically, 1 = never split, n = n K ranges
 static std::atomic<int> g_cta_pairs{-1};    // -1 = choose automatically, 0 = never, 1 = whenever the problem allows it
-static std::atomic<bool> g_pairs_launchable{true};   // cleared when an automatic cluster launch was refused
+static std::atomic<bool> g_pairs_launchable{true};   // cleared when this device turned out to hold no clusters of two
 static std::atomic<int> g_epi_warps{0};     // 0 = choose automatically, 8 or 16
 
 static int epi_warps_for(int epi_mode) {
@@ -174,11 +174,11 @@ static int run_dense(const DenseArgs& d, int device, void* stream) {
       p.num_q_tiles = (int)((d.N + bn - 1) / bn);
       p.splits = 1; p.groups_per_split = d.G;
       p.status = info->status;
-      const int rc = launch_w4a4_group_f8(p, d.a, d.b, d.scratch, bn, device, info->sm_count, static_cast<cudaStream_t>(stream));
-      if (rc == I4TC_OK) return I4TC_OK;
-      // clusters of two cannot be launched here: the kernel below serves the call
-      cudaGetLastError();
-      g_pairs_launchable = false;
+      PairLaunch pl;
+      const int rc = launch_w4a4_group_f8(p, d.a, d.b, d.scratch, bn, device, info->sm_count, static_cast<cudaStream_t>(stream), &pl);
+      if (!pl.failed) return rc;
+      // the launch of clusters was refused: the kernel below serves the call (or reports what is wrong with it)
+      if (pl.unavailable) g_pairs_launchable = false;
     }
   }
 
@@ -269,13 +269,12 @@ static int run_dense(const DenseArgs& d, int device, void* stream) {
     GemmParams pp = p;
     pp.num_p_tiles = (int)((prow + 255) / 256);
     const int grid = 2 * (int)(pair_tiles < clusters_max ? pair_tiles : clusters_max);
-    const int rc = launch_w4a4_gemm(pp, tmP, tmQ, sh.bn, grid, true, epi_warps_for(d.epi_mode), static_cast<cudaStream_t>(stream));
-    if (rc == I4TC_OK) return I4TC_OK;
-    if (g_cta_pairs == 1) return rc;   // the caller asked for pairs: report why they cannot run
-    // an environment that cannot launch clusters of two (a restricted SM partition, for instance): the launch
-    // was refused before anything ran; remember it and use single thread blocks from now on
-    cudaGetLastError();
-    g_pairs_launchable = false;
+    PairLaunch pl;
+    const int rc = launch_w4a4_gemm(pp, tmP, tmQ, sh.bn, grid, true, epi_warps_for(d.epi_mode), static_cast<cudaStream_t>(stream), &pl);
+    if (!pl.failed || g_cta_pairs == 1) return rc;   // (a caller who asked for pairs sees why they cannot run)
+    // refused before anything ran: single thread blocks serve the call, and every later one where the device cannot
+    // hold clusters of two at all
+    if (pl.unavailable) g_pairs_launchable = false;
     if (sh.bn == 192) {   // that width exists on pairs only: fall back to 256-wide single tiles
       sh.bn = 256;
       p.num_q_tiles = (int)((qrow + sh.bn - 1) / sh.bn);

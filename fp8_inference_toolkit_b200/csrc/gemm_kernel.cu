@@ -900,7 +900,8 @@ w4a4_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ C
 }
 
 template <int BN, int CG, int EW>
-static int launch_bn(const GemmParams& p, const CUtensorMap& tmP, const CUtensorMap& tmQ, int grid, cudaStream_t st) {
+static int launch_bn(const GemmParams& p, const CUtensorMap& tmP, const CUtensorMap& tmQ, int grid, cudaStream_t st,
+                     PairLaunch* pl = nullptr) {
   using C = Cfg<BN, CG, EW>;
   static_assert(C::SMEM_BYTES <= 232448, "shared memory layout exceeds the 227 KB a CTA may use");
   static bool configured[64] = {false};
@@ -925,7 +926,7 @@ static int launch_bn(const GemmParams& p, const CUtensorMap& tmP, const CUtensor
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    I4TC_CUDA(cudaLaunchKernelEx(&cfg, w4a4_gemm_kernel<BN, CG, EW>, p, tmP, tmQ));
+    return launch_pairs(cfg, pl, w4a4_gemm_kernel<BN, CG, EW>, p, tmP, tmQ);
   }
   I4TC_CUDA(cudaGetLastError());
   return I4TC_OK;
@@ -989,15 +990,15 @@ int launch_split_reduce(const float* ws, long long stride, int splits, long long
 }
 
 int launch_w4a4_gemm(const GemmParams& p, const CUtensorMap& tmP, const CUtensorMap& tmQ, int bn, int grid,
-                     bool cta_pair, int epi_warps, cudaStream_t st) {
+                     bool cta_pair, int epi_warps, cudaStream_t st, PairLaunch* pl) {
   const bool wide = epi_warps == 16 && bn >= 128;   // 64-column tiles have only 8 x 32 columns to hand out
   if (cta_pair) {
     I4TC_REQUIRE((bn == 256 || bn == 192) && (grid % 2) == 0 && p.expert_offsets == nullptr && !p.swap && p.splits == 1 &&
                      (p.epi_mode == EPI_CHANNEL || p.epi_mode == EPI_GROUP),
                  I4TC_EINVAL, "CTA-pair launch needs a dense, unswapped 192- or 256-wide problem and an even grid");
     // 192-column tiles: three epilogue warps per scheduler, 64 running sums per thread
-    if (bn == 192) return launch_bn<192, 2, 12>(p, tmP, tmQ, grid, st);
-    return wide ? launch_bn<256, 2, 16>(p, tmP, tmQ, grid, st) : launch_bn<256, 2, 8>(p, tmP, tmQ, grid, st);
+    if (bn == 192) return launch_bn<192, 2, 12>(p, tmP, tmQ, grid, st, pl);
+    return wide ? launch_bn<256, 2, 16>(p, tmP, tmQ, grid, st, pl) : launch_bn<256, 2, 8>(p, tmP, tmQ, grid, st, pl);
   }
   switch (bn) {
     case 64: return launch_bn<64, 1, 8>(p, tmP, tmQ, grid, st);

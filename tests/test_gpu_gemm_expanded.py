@@ -115,3 +115,23 @@ def test_operands_off_a_16_byte_boundary_are_refused():
         ops.linear(x, b8, sb, N, False)
     torch.cuda.synchronize()
     assert not out.any()
+
+
+def test_an_unrelated_error_leaves_the_pair_kernels_on():
+    """A call that failed for its own reasons (a device that is not there) is no reason to run others without SM pairs."""
+    from fp8_inference_toolkit_b200 import _cabi, ops
+
+    M, N, G = 512, 512, 32
+    dev = torch.cuda.current_device()
+    a, b, sa, sb, _, _ = args = _operands(M, N, G, False, seed=8)
+    nbytes = _cabi.lib.i4tc_gemm_grouped_scratch_bytes(M, N, G, 0, dev)
+    assert nbytes > 0
+    ref = _call(M, N, G, args, 0)
+    x = torch.randn(M, G * 128, device="cuda").to(torch.bfloat16)
+    y = ops.linear(x, b, sb, N, False)
+    for call, want in ((lambda: _call(M, N, G, args, nbytes), ref), (lambda: ops.linear(x, b, sb, N, False), y)):
+        # (fails on the host: the runtime knows no such device)
+        assert _cabi.lib.i4tc_gemm_grouped(a.data_ptr(), b.data_ptr(), sa.data_ptr(), sb.data_ptr(), ref.data_ptr(), M, N, 128, G,
+                                           63, torch.cuda.current_stream().cuda_stream) > 0
+        assert torch.equal(call(), want)
+        assert _cabi.lib.i4tc_gemm_grouped_scratch_bytes(M, N, G, 0, dev) == nbytes
