@@ -10,6 +10,9 @@ from dataclasses import dataclass
 import torch
 import torch.nn.functional as F
 from torch import nn
+from torch.autograd import forward_ad
+from torch.overrides import _get_current_function_mode_stack
+from torch.utils._device import DeviceContext
 
 from . import moe as _moe
 from . import ops
@@ -29,6 +32,22 @@ class Qwen3Config:
     eps: float = 1e-6
 
 
+def _plain(*tensors, align: int = 16) -> bool:
+    """Whether an op that reads raw pointers may stand in for torch ops on these tensors: contiguous bf16 on one GPU, and
+    nothing at work (a tracer, a mode, a functional transform, autograd in either direction) that has to see torch ops."""
+    if torch.compiler.is_compiling() or torch.jit.is_tracing():
+        return False
+    if (forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None
+            or torch._C._len_torch_dispatch_stack() or any(type(m) is not DeviceContext for m in _get_current_function_mode_stack())):
+        return False
+    for t in tensors:
+        if (type(t) not in (torch.Tensor, nn.Parameter) or not t.is_cuda or t.device != tensors[0].device
+                or t.dtype != torch.bfloat16 or not t.is_contiguous() or t.is_neg() or t.data_ptr() % align
+                or (t.requires_grad and torch.is_grad_enabled())):
+            return False
+    return True
+
+
 class RMSNorm(nn.Module):
     def __init__(self, dim: int, eps: float, device=None):
         super().__init__()
@@ -36,11 +55,10 @@ class RMSNorm(nn.Module):
         self.eps = eps
 
     def forward(self, x):
-        K = x.shape[-1]
-        if (x.is_cuda and x.dtype == self.weight.dtype == torch.bfloat16 and x.is_contiguous() and self.weight.is_contiguous()
-                and x.data_ptr() % 16 == 0 and K % 8 == 0 and 1024 <= K <= 16384 and x.numel() < K << 31
-                and not (torch.is_grad_enabled() and (x.requires_grad or self.weight.requires_grad))):
-            return ops.rmsnorm(x, self.weight, self.eps)
+        if _plain(x, self.weight) and x.dim() > 0 and self.weight.shape == x.shape[-1:]:
+            K = x.shape[-1]
+            if K % 8 == 0 and 1024 <= K <= 16384 and x.numel() < K << 31:
+                return ops.rmsnorm(x, self.weight, self.eps)
         xf = x.float()
         return (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + self.eps)).to(x.dtype) * self.weight
 
