@@ -63,6 +63,15 @@ class RMSNorm(nn.Module):
         return (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + self.eps)).to(x.dtype) * self.weight
 
 
+def _untouched(norm) -> bool:
+    """An RMSNorm of this file that nobody hooked or patched: calling it is its expression and nothing else."""
+    g = nn.modules.module
+    return (type(norm) is RMSNorm and "forward" not in vars(norm)
+            and not (norm._forward_hooks or norm._forward_pre_hooks or norm._backward_hooks or norm._backward_pre_hooks
+                     or g._global_forward_hooks or g._global_forward_pre_hooks or g._global_backward_hooks
+                     or g._global_backward_pre_hooks))
+
+
 def rope_tables(seq: int, head_dim: int, theta: float, device):
     inv = 1.0 / (theta ** (torch.arange(0, head_dim, 2, device=device, dtype=torch.float32) / head_dim))
     ang = torch.outer(torch.arange(seq, device=device, dtype=torch.float32), inv)
@@ -122,11 +131,15 @@ class Block(nn.Module):
 
     def _attention(self, qkv, B, S, cos, sin):
         cfg = self.cfg
-        # (qkv is this layer's own buffer)
-        fused = cfg.head_dim == 128 and cos.shape == (S, 64) and cos.dtype == torch.bfloat16
+        # norms and rotary embedding in one kernel, in place (qkv is this layer's own buffer), where they are what they were
+        # built as; else through the modules
+        fused = (cfg.head_dim == 128 and _untouched(self.q_norm) and _untouched(self.k_norm)
+                 and self.q_norm.eps == self.k_norm.eps and qkv.numel() > 0
+                 and _plain(qkv, self.q_norm.weight, self.k_norm.weight, cos, sin, align=8)
+                 and self.q_norm.weight.shape == self.k_norm.weight.shape == (128,) and cos.shape == sin.shape == (S, 64))
         if fused:
             ops.qk_norm_rope_(qkv.view(B * S, -1), self.q_norm.weight, self.k_norm.weight, cos, sin, cfg.q_heads,
-                              cfg.kv_heads, S, cfg.eps)
+                              cfg.kv_heads, S, self.q_norm.eps)
         q, k, v = qkv.split([cfg.q_heads * cfg.head_dim, cfg.kv_heads * cfg.head_dim, cfg.kv_heads * cfg.head_dim], -1)
         q, k, v = (t.view(B, S, -1, cfg.head_dim) for t in (q, k, v))
         if not fused:
