@@ -45,6 +45,7 @@ SIGNATURES = {
     "i4tc_quant_rowwise_int8": (_i, [_p, _i, _l, _l, _l, _p, _p, _i, _p]),
     "i4tc_gemm_grouped": (_i, [_p, _p, _p, _p, _p, _l, _l, _l, _l, _i, _p]),
     "i4tc_gemm_grouped_azp": (_i, [_p, _p, _p, _p, _p, _p, _p, _l, _l, _l, _l, _i, _p]),
+    "i4tc_gemm_grouped_expanded_width": (_i, [_l, _l, _l, _i, _i]),
     "i4tc_gemm_grouped_scratch_bytes": (_l, [_l, _l, _l, _i, _i]),
     "i4tc_gemm_grouped_scratch": (_i, [_p, _p, _p, _p, _p, _p, _p, _l, _l, _l, _l, _p, _l, _i, _p]),
     "i4tc_linear": (_i, [_p, _i, _l, _l, _l, _p, _p, _i, _p, _p, _p, _l, _p, _l, _i, _p]),

@@ -2,7 +2,7 @@
 //
 // What bounds the converting kernel (gemm_kernel.cu) with a flush per K group is the drain: an int32 -> fp32 conversion,
 // a multiply and a multiply-add per accumulator, next to converter warps and their shared-memory traffic (96 KB per
-// group tile of 128 x 256).  Every code of -8..7 is an e4m3 number and a group's sum stays below 2^13, so
+// group tile of 128 x 256).  Every code of -8..7 is an e4m3 number and a group's sum is at most 2^13 (128 products of 64), so
 // tcgen05.mma kind::f8f6f4 gives the same integers as exact fp32 values at the same rate: no conversion in the drain.
 // The codes are expanded once per call (expand_e4m3_kernel: 1.5 bytes of traffic per code) instead of once per tile, TMA
 // writes the swizzled operand tiles itself, and the warps that converted drain instead.  Results are bit-identical.

@@ -401,13 +401,16 @@ extern "C" int i4tc_gemm_grouped_azp(const uint8_t* a, const uint8_t* b, const f
   return run_dense(d, device, stream);
 }
 
-extern "C" int64_t i4tc_gemm_grouped_scratch_bytes(int64_t M, int64_t N, int64_t num_groups, int azp, int device) {
+extern "C" int i4tc_gemm_grouped_expanded_width(int64_t M, int64_t N, int64_t num_groups, int azp, int device) {
   if (M <= 0 || N <= 0 || num_groups <= 0 || num_groups > 512) return 0;
   const DeviceInfo* info;
   if (device_info(device, &info) != I4TC_OK) return 0;
-  if (choose_f8(M, N, (int)num_groups, info->sm_count, azp != 0) == 0) return 0;
-  const long long bytes = group_f8_scratch_bytes(M, N, (int)num_groups);
-  return bytes <= kF8ScratchLimit ? bytes : 0;
+  if (group_f8_scratch_bytes(M, N, (int)num_groups) > kF8ScratchLimit) return 0;
+  return choose_f8(M, N, (int)num_groups, info->sm_count, azp != 0);
+}
+
+extern "C" int64_t i4tc_gemm_grouped_scratch_bytes(int64_t M, int64_t N, int64_t num_groups, int azp, int device) {
+  return i4tc_gemm_grouped_expanded_width(M, N, num_groups, azp, device) != 0 ? group_f8_scratch_bytes(M, N, (int)num_groups) : 0;
 }
 
 extern "C" int i4tc_gemm_grouped_scratch(const uint8_t* a, const uint8_t* b, const float* scale_a, const float* scale_b,

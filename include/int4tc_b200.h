@@ -207,7 +207,9 @@ int i4tc_gemm_grouped_azp(const uint8_t* a, const uint8_t* b, const float* scale
  * With at least i4tc_gemm_grouped_scratch_bytes(...) bytes, 16-byte aligned, large problems expand both operands to
  * 8-bit floats there and multiply those (the same sums, bit for bit; no conversion inside the GEMM); with less, or
  * NULL, the call does what i4tc_gemm_grouped(_azp) does.  The scratch is free again when the call's work on `stream` is
- * done.  i4tc_gemm_grouped_scratch_bytes returns 0 where scratch would not be used. */
+ * done.  i4tc_gemm_grouped_scratch_bytes returns 0 where scratch would not be used; i4tc_gemm_grouped_expanded_width
+ * says which tile width (256, 192 or 128 columns) that path would take, or 0. */
+int i4tc_gemm_grouped_expanded_width(int64_t M, int64_t N, int64_t num_groups, int azp, int device);
 int64_t i4tc_gemm_grouped_scratch_bytes(int64_t M, int64_t N, int64_t num_groups, int azp, int device);
 int i4tc_gemm_grouped_scratch(const uint8_t* a, const uint8_t* b, const float* scale_a, const float* scale_b,
                               const float* azp_adj, const float* w_col_sum, void* out, int64_t M, int64_t N,

@@ -41,18 +41,67 @@ def _call(M, N, G, args, nbytes):
 
 @pytest.mark.parametrize("azp", [False, True])
 @pytest.mark.parametrize("codes", ["random", "extreme"])
-# tile width 128 (one row tile, ragged N; odd N), 192, 256 (M one past a tile; full tiles and several waves)
-@pytest.mark.parametrize("M,N,G", [(129, 1000, 64), (257, 1001, 20), (512, 512, 32), (130, 9473, 16), (1000, 6144, 32),
-                                   (1537, 2568, 32), (2048, 4096, 32)])
-def test_same_bits_as_the_converting_kernel(M, N, G, codes, azp):
+# every tile width with a ragged last row tile (one row; one row of the pair's second CTA; none of its rows), ragged and odd N,
+# full tiles, and several waves
+@pytest.mark.parametrize("M,N,G,width", [
+    (129, 1000, 64, 128), (257, 1001, 20, 128), (512, 512, 32, 128), (1537, 2568, 32, 128),
+    (130, 9473, 16, 192), (1000, 6144, 32, 192),
+    (1025, 3001, 16, 256), (1409, 2305, 16, 256), (769, 9465, 16, 256), (2048, 4096, 32, 256)])
+def test_same_bits_as_the_converting_kernel(M, N, G, width, codes, azp):
     from fp8_inference_toolkit_b200 import _cabi, ops
 
-    nbytes = _cabi.lib.i4tc_gemm_grouped_scratch_bytes(M, N, G, int(azp), torch.cuda.current_device())
-    assert nbytes > 0, "this size is meant to take the expanded path"
+    dev = torch.cuda.current_device()
+    assert _cabi.lib.i4tc_gemm_grouped_expanded_width(M, N, G, int(azp), dev) == width
+    nbytes = _cabi.lib.i4tc_gemm_grouped_scratch_bytes(M, N, G, int(azp), dev)
+    assert nbytes > 0
     args = _operands(M, N, G, azp, codes, seed=M + N)
     ref = _call(M, N, G, args, 0)
     assert torch.equal(_call(M, N, G, args, nbytes), ref)
     assert torch.equal(_call(M, N, G, args, nbytes - 1), ref)   # too little scratch: the converting kernel again
+    ops.check_status()
+
+
+def _low_bit_codes(M, N, G, pattern, gen):
+    """Codes of group pairs whose sums are large inside and differ by a few units: where fewer than 14 bits of a sum are kept,
+    or products are aligned to its size and cut, the difference shows it."""
+    def redraw(t):
+        r = torch.randint(-8, 8, t.shape, device="cuda", generator=gen, dtype=torch.int8)
+        return torch.where(torch.rand(t.shape, device="cuda", generator=gen) < 0.05, r, t)
+
+    H = G // 2
+    a = torch.full((H, M, 128), -8, dtype=torch.int8, device="cuda")
+    b = torch.full((H, N, 128), -8, dtype=torch.int8, device="cuda")
+    if pattern == "cancelling":      # half of the products are 64, half -56, in an order of its own in every group
+        for h in range(H):
+            b[h][:, torch.randperm(128, device="cuda", generator=gen)[:64]] = 7
+    a, b = redraw(a), redraw(b)
+    if pattern == "large":
+        a[:, 0], b[:, 0] = -8, -8    # the largest sum of all, 2^13
+    at = torch.randint(0, 128, (H, M, 1), device="cuda", generator=gen)
+    old = a.gather(2, at)
+    return a, b, a.scatter(2, at, torch.where(old < 7, old + 1, old - 1))
+
+
+@pytest.mark.parametrize("pattern", ["large", "cancelling"])
+@pytest.mark.parametrize("M,N,G,width", [(257, 1001, 20, 128), (130, 9473, 16, 192), (1025, 3001, 16, 256)])
+def test_every_bit_of_a_group_sum_counts(M, N, G, width, pattern):
+    from fp8_inference_toolkit_b200 import _cabi, ops
+
+    dev = torch.cuda.current_device()
+    assert _cabi.lib.i4tc_gemm_grouped_expanded_width(M, N, G, 0, dev) == width
+    a, b, a2 = _low_bit_codes(M, N, G, pattern, torch.Generator(device="cuda").manual_seed(N))
+    if pattern == "large":
+        assert int((a[0, 0].int() * b[0, 0].int()).sum()) == 1 << 13
+    pack = lambda t: (t[..., 0::2] & 15) | ((t[..., 1::2] & 15) << 4)
+    both = lambda t, u: torch.stack([t, u], 1).flatten(0, 1).contiguous()     # groups 2 h and 2 h + 1
+    scale = torch.tensor([1.0, -1.0], device="cuda").repeat(G // 2)[:, None]
+    args = (pack(both(a, a2)).view(torch.uint8), pack(both(b, b)).view(torch.uint8), scale.expand(G, M).contiguous(),
+            torch.ones(G, N, device="cuda"), None, None)
+    flat = lambda t: t.transpose(0, 1).flatten(1).double()
+    ref = flat(a - a2) @ flat(b).T            # small integers, every one of them a bf16 value
+    assert ref.abs().max() <= 256
+    nbytes = _cabi.lib.i4tc_gemm_grouped_scratch_bytes(M, N, G, 0, dev)
+    assert torch.equal(_call(M, N, G, args, nbytes).double(), ref)
     ops.check_status()
 
 
@@ -88,6 +137,38 @@ def test_inside_a_captured_graph():
     replayed = out.clone()
     run()
     assert torch.equal(replayed, out)
+
+
+@pytest.mark.parametrize("azp", [False, True])
+def test_without_memory_for_scratch(azp, monkeypatch):
+    """The converting kernel serves the call."""
+    from fp8_inference_toolkit_b200 import _cabi, ops
+
+    M, N, G = 512, 512, 32
+    a, b, sa, sb, z, w = _operands(M, N, G, azp, seed=9)
+    nbytes = _cabi.lib.i4tc_gemm_grouped_scratch_bytes(M, N, G, int(azp), torch.cuda.current_device())
+    x = torch.randn(M, G * 128, device="cuda").to(torch.bfloat16)
+
+    def run():
+        out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+        if azp:
+            ops.cutlass_int4_fused_grouped_gemm_azp(a, b, sa, sb, out, z, w, M, N, 128, G)
+        else:
+            ops.cutlass_int4_fused_grouped_gemm(a, b, sa, sb, out, M, N, 128, G)
+        return out, ops.linear(x, b, sb, N, False)
+
+    ref = run()
+    refused, empty = [], torch.empty
+
+    def small_only(*size, **kwargs):
+        if kwargs.get("dtype") == torch.uint8 and isinstance(size[0], int) and size[0] >= nbytes:
+            refused.append(size[0])
+            raise torch.cuda.OutOfMemoryError("no room")
+        return empty(*size, **kwargs)
+
+    monkeypatch.setattr(torch, "empty", small_only)
+    got = run()
+    assert len(refused) == 2 and all(torch.equal(p, q) for p, q in zip(got, ref))
 
 
 def test_operands_off_a_16_byte_boundary_are_refused():

@@ -54,3 +54,23 @@ def test_one_call_linear_equals_the_ops(M, per_channel):
             ops.cutlass_int4_fused_grouped_gemm(xp, wp, xs, ws, ref, M, N, 128, K // 128)
         assert torch.equal(ops.linear(x, wp, ws, N, per_channel), ref)
     ops.check_status()
+
+
+@pytest.mark.parametrize("per_channel", [False, True])
+def test_one_call_linear_refuses_what_the_ops_refuse(per_channel):
+    from fp8_inference_toolkit_b200 import ops
+
+    M, K, N, G = 4, 256, 24, 1 if per_channel else 2
+    x = torch.zeros(M, K, dtype=torch.bfloat16, device="cuda")
+    w = torch.zeros(N * K // 2, dtype=torch.uint8, device="cuda")
+    s = torch.ones(G * N, device="cuda")
+    assert not ops.linear(x, w, s, N, per_channel).any()
+    odd = K - 32     # neither whole groups nor whole 32-byte rows of codes
+    for args in [(x.cpu(), w, s), (x[0], w, s), (x.int(), w, s), (x[:, :odd].contiguous(), w[: N * odd // 2], s),
+                 (x, w[:-1], s), (x, w.view(torch.int8), s), (x, torch.zeros(N * K, dtype=torch.uint8, device="cuda")[::2], s),
+                 (x, w.cpu(), s), (x, w, s[:-1]), (x, w, s.double()), (x, w, s.cpu()), (x, w, torch.ones(2 * G * N, device="cuda")[::2])]:
+        with pytest.raises(RuntimeError):
+            ops.linear(*args, N, per_channel)
+    with pytest.raises(RuntimeError):
+        ops.linear(x, w, s, N + 1, per_channel)
+    assert ops.linear(x[:0], w, s, N, per_channel).shape == (0, N)
