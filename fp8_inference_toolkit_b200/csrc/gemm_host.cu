@@ -90,28 +90,32 @@ static Shape choose_shape(long long M, long long N, int sms, bool allow_swap, bo
 
 // Tile width of the expanded per-group kernel (gemm_f8.cu) for an [M, N] problem with G groups, or 0 where converting
 // inside the GEMM is the better choice.  Both sides are estimated from measured times (B200, 1965 MHz): columns of tile
-// that an SM pair works through one after another x groups x 2.81 ns (192 / 128-column tiles: 2 / 8 % more) here,
-// 3.71 ns per cost unit of choose_shape there, 1.27 and 1.5 times that with the zero-point term; the expansion moves 1.5
-// bytes per code at 8 TB/s (mostly L2) and is one more launch.  Measured on both sides of the line (expanded | in-kernel):
-// [200, 4096] x [6144, 4096] 26.0 | 28.7 us, [384, 12288] x [4096, 12288] 54 | 70, [512, 4096] x [6144, 4096] 32 | 35,
-// [300, 256] x [264, 256] 22 | 14.
+// that an SM pair works through one after another x groups x 2.70 ns (192 / 128-column tiles: 2 / 8 % more) here,
+// 3.78 ns per cost unit of choose_shape there, 1.24 and 1.53 times that with the zero-point term and 2 ns a column here;
+// the expansion moves 1.5 bytes per code at 7.1 TB/s (part of it in L2) and is one more launch.  Fitted to both kernels
+// at 1046 sizes (M 129..8192, N 264..24576, K 256..12288, with and without zero points): the choice costs 0.34 % on
+// average against the faster of the two, and what is expanded is slower by 5 % at most.  Around the line (expanded | in-kernel):
+// [256, 4096] x [6144, 4096] 28.5 | 27.2 us, with zero points 32.4 | 39.5; [256, 4096] x [24576, 4096] 67 | 71 and one row
+// more 101 | 74; [512, 4096] x [24576, 4096] 102 | 101, with zero points 123 | 152; [1000, 1024] x [1000, 1024] 14.7 | 12.9,
+// with zero points 15.7 | 15.2.
 static int choose_f8(long long M, long long N, int G, int sms, bool azp) {
   if (g_force_bn != 0 || g_force_swap >= 0 || g_force_splits != 0 || g_cta_pairs >= 0 || g_epi_warps != 0 ||
       g_small_m_path != 0 || !g_pairs_launchable.load() || sms < 2)
     return 0;   // a pinned configuration means the converting kernel
   if (M <= 128 || (M + N) * (long long)G >= (1ll << 31) - 65536) return 0;
   int best_bn = 0;
-  double best = 1e30;
+  double best = 1e30, best_columns = 0;
   const struct { int bn; double w; } cands[3] = {{256, 1.00}, {192, 1.02}, {128, 1.08}};
   for (const auto& c : cands) {
     const long long tiles = ((M + 255) / 256) * ((N + c.bn - 1) / c.bn), units = sms / 2;
-    const double cost = (double)((tiles + units - 1) / units) * c.bn * c.w;
-    if (cost < best) { best = cost; best_bn = c.bn; }
+    const double columns = (double)((tiles + units - 1) / units) * c.bn;
+    if (columns * c.w < best) { best = columns * c.w; best_bn = c.bn; best_columns = columns; }
   }
   double in_kernel = 0;
   choose_shape(M, N, sms, true, true, true, &in_kernel);
-  const double expanded_us = best * G * 0.00281 * (azp ? 1.27 : 1.0) + 2.0 + (double)(M + N) * G * (128 * 1.5 / 8.0e6);
-  return expanded_us < in_kernel * G * 0.00371 * (azp ? 1.5 : 1.0) ? best_bn : 0;
+  const double expanded_us = best * G * 0.00270 * (azp ? 1.24 : 1.0) + (azp ? best_columns * 0.002 : 0.0) + 2.7 +
+                             (double)(M + N) * G * (128 * 1.5 / 7.1e6);
+  return expanded_us < in_kernel * G * 0.00378 * (azp ? 1.53 : 1.0) ? best_bn : 0;
 }
 
 struct DenseArgs {

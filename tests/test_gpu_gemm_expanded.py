@@ -44,9 +44,9 @@ def _call(M, N, G, args, nbytes):
 # every tile width with a ragged last row tile (one row; one row of the pair's second CTA; none of its rows), ragged and odd N,
 # full tiles, and several waves
 @pytest.mark.parametrize("M,N,G,width", [
-    (129, 1000, 64, 128), (257, 1001, 20, 128), (512, 512, 32, 128), (1537, 2568, 32, 128),
-    (130, 9473, 16, 192), (1000, 6144, 32, 192),
-    (1025, 3001, 16, 256), (1409, 2305, 16, 256), (769, 9465, 16, 256), (2048, 4096, 32, 256)])
+    (129, 1000, 64, 128), (257, 1001, 32, 128), (512, 512, 32, 128), (1537, 2568, 40, 128),
+    (130, 9473, 32, 192), (1000, 6144, 32, 192),
+    (1025, 3001, 32, 256), (1409, 2305, 32, 256), (769, 9465, 32, 256), (2048, 4096, 32, 256)])
 def test_same_bits_as_the_converting_kernel(M, N, G, width, codes, azp):
     from fp8_inference_toolkit_b200 import _cabi, ops
 
@@ -83,7 +83,7 @@ def _low_bit_codes(M, N, G, pattern, gen):
 
 
 @pytest.mark.parametrize("pattern", ["large", "cancelling"])
-@pytest.mark.parametrize("M,N,G,width", [(257, 1001, 20, 128), (130, 9473, 16, 192), (1025, 3001, 16, 256)])
+@pytest.mark.parametrize("M,N,G,width", [(257, 1001, 32, 128), (130, 9473, 32, 192), (1025, 3001, 32, 256)])
 def test_every_bit_of_a_group_sum_counts(M, N, G, width, pattern):
     from fp8_inference_toolkit_b200 import _cabi, ops
 
