@@ -219,7 +219,7 @@ def run_ours(args) -> None:
     import torch.distributed as dist
 
     import int4_native_tc as tc
-    from fp8_inference_toolkit_b200 import ops, synthetic
+    from fp8_inference_toolkit_b200 import _cabi, ops, synthetic
     from fp8_inference_toolkit_b200.linear import W4A4Linear
 
     world = int(os.environ.get("WORLD_SIZE", "1"))
@@ -345,6 +345,9 @@ def run_ours(args) -> None:
     gemm_ops_rank = ops_per_step / world
     int8_peak = 2.0 * peaks["bf16_tflops"]
     achieved = gemm_ops_rank / gemm_s / 1e12
+    # shapes whose GEMM call expands its operands to e4m3 first (a launch of its own, timed with the GEMM)
+    expanded = [not per_channel and _cabi.lib.i4tc_gemm_grouped_expanded_width(M, N // world, K // GROUP, 0, local) != 0
+                for _, K, N in SHAPES]
 
     # ---- e2e: host buffers through the linear module, copies inside the timed region.  The ranks share one host:
     # each copies M / n rows of the activations from pinned memory and an all-gather over NVLink gives every rank
@@ -413,20 +416,24 @@ def run_ours(args) -> None:
         line = {
             "metric": METRIC_CHANNEL if per_channel else METRIC, "value": value, "unit": UNIT, "n_gpus": world,
             "steps": args.steps, "warmup": max(args.warmup, 3), "ms_per_step": ms_per_step, "higher_is_better": True,
-            "scaling": "strong", "vs_baseline": None, "dtype": "s4*s4->s32, f32 dequant", "data": "synthetic",
+            "scaling": "strong", "vs_baseline": None,
+            "dtype": "s4*s4->f32 (exact), f32 dequant" if all(expanded) else "s4*s4->s32, f32 dequant", "data": "synthetic",
             "config": workload_config(M, world, per_channel), "clocks": clocks,
             "e2e": {"value": e2e_val, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h * 1,
                     "ms_per_step": e2e_s * 1e3},
-            "gpu_launches": args.steps * 2 * len(SHAPES),   # timed region of `value`: quantise + GEMM per linear
+            # timed region of `value`: quantise + GEMM per linear, and the expansion where there is one
+            "gpu_launches": args.steps * (2 * len(SHAPES) + sum(expanded)),
             "roofline": {
                 "bound": "tensor", "achieved": achieved, "peak": int8_peak, "unit": "TOPS",
                 "frac": achieved / int8_peak,
-                # ncu (M=1024 capture, profiles/): DRAM reads of a launch = 1.00 x its operand bytes and the
-                # bf16 output is written back after the kernel ends, so a launch moves its algorithmic bytes
-                "traffic": sum(gemm_bytes(M, N // world, K) for _, K, N in SHAPES) / len(SHAPES),
-                "traffic_unit": "bytes per launch (mean of the 4 shapes), algorithmic; ncu-confirmed at M=1024",
-                "kernel": ("w4a4_gemm_kernel (per-channel epilogue, 256x256 tiles on SM pairs)" if per_channel
-                           else "w4a4_gemm_kernel (per-group-128 epilogue, 256x256 tiles on SM pairs)") + ", 4 launches per step",
+                # operands, scales and output once, and where the operands are expanded one write and one read of a byte
+                # per code (part of which stays in L2); counted, not a counter's reading
+                "traffic": sum(gemm_bytes(M, N // world, K) + (2 * (M + N // world) * K if x else 0)
+                               for (_, K, N), x in zip(SHAPES, expanded)) / len(SHAPES),
+                "traffic_unit": "bytes per GEMM call (mean of the 4 shapes), algorithmic plus the expanded operands",
+                "kernel": ("w4a4_gemm_kernel (per-channel epilogue, 256x256 tiles on SM pairs), 4 launches per step" if per_channel
+                           else "w4a4_group_f8_kernel (per-group-128 epilogue, e4m3 operands on SM pairs), %d launches per step, "
+                                "each behind expand_e4m3_kernel; w4a4_gemm_kernel, %d" % (sum(expanded), len(SHAPES) - sum(expanded))),
                 "peak_source": f"2 x bf16 burst of MEASURED_PEAKS.json ({peaks['source']}); int8 dense = 2 x bf16 on B200",
                 "per_shape_us": {SHAPES[i][0]: statistics.mean(v) * 1e6 for i, v in per_shape.items()},
             },

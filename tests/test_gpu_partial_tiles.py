@@ -1,5 +1,5 @@
 """GPU: row tiles that are mostly padding (a few tokens per expert) give the oracle's bits, whatever part of a warp's rows
-exists; and the one-call linear equals its separate ops."""
+exists; and the one-call linear equals its separate ops and refuses what they refuse."""
 import numpy as np
 import pytest
 import torch
