@@ -7,6 +7,7 @@
 #include <stdint.h>
 #include <stdio.h>
 #include <stdarg.h>
+#include <atomic>
 
 #include "../../include/int4tc_b200.h"
 
@@ -67,6 +68,7 @@ struct DeviceInfo {
   int cc_minor = 0;
   int max_smem_optin = 0;
   unsigned int* status = nullptr;  // device status word written by bounded waits
+  mutable std::atomic<bool> pairs{true};   // cleared when the device turned out to hold no clusters of two
 };
 
 // Cached per-device properties; allocates the status word on first use.

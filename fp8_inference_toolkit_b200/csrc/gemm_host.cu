@@ -13,7 +13,6 @@ static std::atomic<int> g_force_swap{-1};   // -1 = choose automatically
 static std::atomic<int> g_small_m_path{0};  // 0 = automatic, 1 = CUDA-core kernel only, 2 = register-fed tensor-core kernel whenever it applies, 3 = tile kernel only
 static std::atomic<int> g_force_splits{0};  // 0 = choose automatically, 1 = never split, n = n K ranges
 static std::atomic<int> g_cta_pairs{-1};    // -1 = choose automatically, 0 = never, 1 = whenever the problem allows it
-static std::atomic<bool> g_pairs_launchable{true};   // cleared when this device turned out to hold no clusters of two
 static std::atomic<int> g_epi_warps{0};     // 0 = choose automatically, 8 or 16
 
 static int epi_warps_for(int epi_mode) {
@@ -98,9 +97,10 @@ static Shape choose_shape(long long M, long long N, int sms, bool allow_swap, bo
 // [256, 4096] x [6144, 4096] 28.5 | 27.2 us, with zero points 32.4 | 39.5; [256, 4096] x [24576, 4096] 67 | 71 and one row
 // more 101 | 74; [512, 4096] x [24576, 4096] 102 | 101, with zero points 123 | 152; [1000, 1024] x [1000, 1024] 14.7 | 12.9,
 // with zero points 15.7 | 15.2.
-static int choose_f8(long long M, long long N, int G, int sms, bool azp) {
+static int choose_f8(long long M, long long N, int G, const DeviceInfo& dev, bool azp) {
+  const int sms = dev.sm_count;
   if (g_force_bn != 0 || g_force_swap >= 0 || g_force_splits != 0 || g_cta_pairs >= 0 || g_epi_warps != 0 ||
-      g_small_m_path != 0 || !g_pairs_launchable.load() || sms < 2)
+      g_small_m_path != 0 || !dev.pairs.load() || sms < 2)
     return 0;   // a pinned configuration means the converting kernel
   if (M <= 128 || (M + N) * (long long)G >= (1ll << 31) - 65536) return 0;
   int best_bn = 0;
@@ -164,7 +164,7 @@ static int run_dense(const DenseArgs& d, int device, void* stream) {
   }
 
   if (d.scratch != nullptr && d.epi_mode == EPI_GROUP) {
-    const int bn = choose_f8(d.M, d.N, d.G, info->sm_count, d.azp_adj != nullptr);
+    const int bn = choose_f8(d.M, d.N, d.G, *info, d.azp_adj != nullptr);
     if (bn != 0 && d.scratch_bytes >= group_f8_scratch_bytes(d.M, d.N, d.G) && aligned_to(d.scratch, 16)) {
       // (the tensor maps of the other tile kernel check this; here the operands are read by the expansion's 16-byte loads)
       I4TC_REQUIRE(aligned_to(d.a, 16) && aligned_to(d.b, 16), I4TC_EALIGN, "packed operand must be 16-byte aligned");
@@ -182,12 +182,12 @@ static int run_dense(const DenseArgs& d, int device, void* stream) {
       const int rc = launch_w4a4_group_f8(p, d.a, d.b, d.scratch, bn, device, info->sm_count, static_cast<cudaStream_t>(stream), &pl);
       if (!pl.failed) return rc;
       // the launch of clusters was refused: the kernel below serves the call (or reports what is wrong with it)
-      if (pl.unavailable) g_pairs_launchable = false;
+      if (pl.unavailable) info->pairs = false;
     }
   }
 
   const bool group_mode = d.epi_mode == EPI_GROUP || d.epi_mode == EPI_GROUP_INT32;
-  const bool pairs_allowed = (d.epi_mode == EPI_CHANNEL || d.epi_mode == EPI_GROUP) && g_pairs_launchable.load();
+  const bool pairs_allowed = (d.epi_mode == EPI_CHANNEL || d.epi_mode == EPI_GROUP) && info->pairs.load();
   Shape sh = choose_shape(d.M, d.N, info->sm_count, true, group_mode, pairs_allowed);
   I4TC_REQUIRE(sh.bn != 192 || sh.pair, I4TC_EINVAL, "192-wide tiles need a dense problem with scaled outputs (SM pairs)");
   GemmParams p;
@@ -278,7 +278,7 @@ static int run_dense(const DenseArgs& d, int device, void* stream) {
     if (!pl.failed || g_cta_pairs == 1) return rc;   // (a caller who asked for pairs sees why they cannot run)
     // refused before anything ran: single thread blocks serve the call, and every later one where the device cannot
     // hold clusters of two at all
-    if (pl.unavailable) g_pairs_launchable = false;
+    if (pl.unavailable) info->pairs = false;
     if (sh.bn == 192) {   // that width exists on pairs only: fall back to 256-wide single tiles
       sh.bn = 256;
       p.num_q_tiles = (int)((qrow + sh.bn - 1) / sh.bn);
@@ -410,7 +410,7 @@ extern "C" int i4tc_gemm_grouped_expanded_width(int64_t M, int64_t N, int64_t nu
   const DeviceInfo* info;
   if (device_info(device, &info) != I4TC_OK) return 0;
   if (group_f8_scratch_bytes(M, N, (int)num_groups) > kF8ScratchLimit) return 0;
-  return choose_f8(M, N, (int)num_groups, info->sm_count, azp != 0);
+  return choose_f8(M, N, (int)num_groups, *info, azp != 0);
 }
 
 extern "C" int64_t i4tc_gemm_grouped_scratch_bytes(int64_t M, int64_t N, int64_t num_groups, int azp, int device) {
