@@ -8,12 +8,12 @@
 // writes the swizzled operand tiles itself, and the warps that converted drain instead.  Results are bit-identical.
 //   [8192, 4096] x [24576, 4096]: 1282 -> 985 us; with the zero-point term 1900 -> 1260 us
 //   [4096, 12288] x [4096, 12288]: 360 -> 259 us;  [1000, 4096] x [6144, 4096]: 60 -> 51 us
-// A group tile of 256 x 256 takes a pair about 1400 cycles: the tensor cores need 512 of them, the packed fp32
-// arithmetic 570.  What is left is latency between the two: an accumulator is 1000 cycles from its first MMA to its
-// arrival and there are two (four at 128 columns), and shared memory answers the drain slowly under the tensor core's
-// operand reads (LDS throughput a third).  Measured and not kept: accumulators of half the width (two commits per group:
-// a commit needs 480 cycles of its own, +20 %), double-buffered TMEM loads (+4-20 %), all loads before the arithmetic
-// (+3 %), 160-column tiles with three accumulators (+19 %).
+// A group tile of 256 x 256 takes a pair 1258 active cycles (counters of [8192, 4096] x [8192, 4096]): the tensor cores need
+// 512 of them (active 40 %), the packed fp32 arithmetic 570.  What is left is latency between the two: an accumulator is
+// 1000 cycles from its first MMA to its arrival and there are two (four at 128 columns), and shared memory answers the
+// drain slowly under the tensor core's operand reads (LDS throughput a third).  Measured and not kept: accumulators of
+// half the width (two commits per group: a commit needs 480 cycles of its own, +20 %), double-buffered TMEM loads (+4-20 %),
+// all loads before the arithmetic (+3 %), 160-column tiles with three accumulators (+19 %).
 //
 // Roles (BN / 16 + 4 warps): warp 0 TMA producer, warp 1 MMA issuer (leader) or reporter (second CTA), warps 2-3 scale
 // loaders, the others epilogue.  Every wait is bounded as in gemm_kernel.cu.
@@ -30,7 +30,8 @@ struct F8Cfg {
   static constexpr int NT = BN > 128 ? 2 : 4;             // accumulators in the 512 TMEM columns
   static constexpr int EW = BN / 16;                      // epilogue warps: 32 rows x 64 columns of every accumulator
   // registers per thread of warps 0..3 and of the epilogue, within what the launch allocates: 640 threads x 96 (BN 256:
-  // 128 * 56 + 512 * 104), 512 x 128 (BN 192: 128 * 56 + 384 * 152); BN 128 (384 threads x 168) runs as launched
+  // 128 * 56 + 512 * 104), 512 x 128 (BN 192: 128 * 56 + 384 * 152); BN 128 (384 threads x 168) runs as launched.  The
+  // compiler allots by the launch: 256 columns spill 20 bytes (56 with the zero-point term), 192 columns 8, 128 none
   static constexpr int REG_LOW = 56, REG_EPI = BN == 256 ? 104 : (BN == 192 ? 152 : 0);
   static constexpr int THREADS = (kF8EpiWarp0 + EW) * 32;
   static constexpr int QR = BN / 2;                       // Q rows staged by each CTA of the pair

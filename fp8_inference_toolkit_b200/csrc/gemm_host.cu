@@ -93,7 +93,8 @@ static Shape choose_shape(long long M, long long N, int sms, bool allow_swap, bo
 // 3.78 ns per cost unit of choose_shape there, 1.24 and 1.53 times that with the zero-point term and 2 ns a column here;
 // the expansion moves 1.5 bytes per code at 7.1 TB/s (part of it in L2) and is one more launch.  Fitted to both kernels
 // at 1046 sizes (M 129..8192, N 264..24576, K 256..12288, with and without zero points): the choice costs 0.34 % on
-// average against the faster of the two, and what is expanded is slower by 5 % at most.  Around the line (expanded | in-kernel):
+// average against the faster of the two, and what is expanded is slower by 5 % at most (16.4 | 14.9 us in another run of the
+// smallest size below, with zero points).  Around the line (expanded | in-kernel):
 // [256, 4096] x [6144, 4096] 28.5 | 27.2 us, with zero points 32.4 | 39.5; [256, 4096] x [24576, 4096] 67 | 71 and one row
 // more 101 | 74; [512, 4096] x [24576, 4096] 102 | 101, with zero points 123 | 152; [1000, 1024] x [1000, 1024] 14.7 | 12.9,
 // with zero points 15.7 | 15.2.
