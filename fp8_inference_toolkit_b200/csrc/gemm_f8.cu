@@ -6,16 +6,18 @@
 // tcgen05.mma kind::f8f6f4 gives the same integers as exact fp32 values at the same rate: no conversion in the drain.
 // The codes are expanded once per call (expand_e4m3_kernel: 1.5 bytes of traffic per code) instead of once per tile, TMA
 // writes the swizzled operand tiles itself, and the warps that converted drain instead.  Results are bit-identical.
-//   [8192, 4096] x [24576, 4096]: 1282 -> 985 us; with the zero-point term 1900 -> 1260 us
-//   [4096, 12288] x [4096, 12288]: 360 -> 259 us;  [1000, 4096] x [6144, 4096]: 60 -> 51 us
-// A group tile of 256 x 256 takes a pair 1258 active cycles (counters of [8192, 4096] x [8192, 4096]): the tensor cores need
-// 512 of them (active 40 %), the packed fp32 arithmetic 570.  What is left is latency between the two: an accumulator is
-// 1000 cycles from its first MMA to its arrival and there are two (four at 128 columns), and shared memory answers the
-// drain slowly under the tensor core's operand reads (LDS throughput a third).  Measured and not kept: accumulators of
-// half the width (two commits per group: a commit needs 480 cycles of its own, +20 %), double-buffered TMEM loads (+4-20 %),
-// all loads before the arithmetic (+3 %), 160-column tiles with three accumulators (+19 %).
+//   [8192, 4096] x [24576, 4096]: 1282 -> 869 us (expansion included); with the zero-point term 1900 -> 1150 us
+//   [4096, 12288] x [4096, 12288]: 360 -> 262 us;  [1000, 4096] x [6144, 4096]: 60 -> 51 us
+// A group tile of 256 x 256 takes a pair about 1110 cycles: the tensor cores need 512 of them, the packed fp32 arithmetic
+// 570 (640 next to MMAs).  Timed on one SM without barriers, the drain of a 128 x 256 tile takes 690-740 cycles alone and 980-1020
+// next to MMAs, whether by 8 or 16 warps and with one or two TMEM loads in flight: 80 LDS.128 of scales take 150 cycles
+// alone and 580 next to MMAs, whose operand reads go first, and TMEM loads (270) are not slowed.  Knocked out one by one: the arithmetic
+// 80 us of 322 ([8192, 4096] x [8192, 4096]), the multiplies 20, the output stores 16.  Measured and not kept: two MMA-issuing warps,
+// on alternate groups or on the halves of a tile with an accumulator each (+0-8 %), 160-column tiles with three accumulators
+// (+19 %), TMEM loads a step ahead across groups (+5-10 %), scales a group ahead in registers (+30 %), pairs packed by
+// explicit 64-bit registers (+4 %), row scales doubled in shared memory (+2 %).
 //
-// Roles (BN / 16 + 4 warps): warp 0 TMA producer, warp 1 MMA issuer (leader) or reporter (second CTA), warps 2-3 scale
+// Roles (12 warps): warp 0 TMA producer, warp 1 MMA issuer (leader) or reporter (second CTA), warps 2-3 scale
 // loaders, the others epilogue.  Every wait is bounded as in gemm_kernel.cu.
 #include "gemm_dev.cuh"
 
@@ -25,20 +27,30 @@ using namespace ptx;
 
 constexpr int kF8EpiWarp0 = 4;   // warps 0..3: TMA producer, MMA issuer, two scale loaders
 
+// Four consecutive floats of shared memory as two pairs.
+__device__ __forceinline__ void lds_pairs(uint32_t addr, float2& a, float2& b) {
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a.x), "=f"(a.y), "=f"(b.x), "=f"(b.y) : "r"(addr));
+}
+
 template <int BN>
 struct F8Cfg {
   static constexpr int NT = BN > 128 ? 2 : 4;             // accumulators in the 512 TMEM columns
-  static constexpr int EW = BN / 16;                      // epilogue warps: 32 rows x 64 columns of every accumulator
-  // registers per thread of warps 0..3 and of the epilogue, within what the launch allocates: 640 threads x 96 (BN 256:
-  // 128 * 56 + 512 * 104), 512 x 128 (BN 192: 128 * 56 + 384 * 152); BN 128 (384 threads x 168) runs as launched.  The
-  // compiler allots by the launch: 256 columns spill 20 bytes (56 with the zero-point term), 192 columns 8, 128 none
-  static constexpr int REG_LOW = 56, REG_EPI = BN == 256 ? 104 : (BN == 192 ? 152 : 0);
+  // 8 epilogue warps, 32 rows x BN / 2 columns of every accumulator each: what a warp pays per group (probes, arrivals, row
+  // scales, index arithmetic) is spread over 64 to 128 columns.  Against BN / 16 warps of 64 columns, [8192, 4096] x
+  // [24576, 4096]: 981 -> 869 us at 256, 983 -> 924 at 192, 985 -> 928 at 128 columns
+  static constexpr int EW = 8;
+  static constexpr int CW = BN / 2;
+  static constexpr int STEP = BN == 192 ? 16 : 32;        // columns per TMEM load (the other one: 2 to 4 % slower)
+  // registers per thread of warps 0..3 and of the epilogue, within what the launch allocates (384 threads x 168):
+  // 128 * 56 + 256 * 224, CW of the latter for the running sums
+  static constexpr int REG_LOW = 56, REG_EPI = 224;
   static constexpr int THREADS = (kF8EpiWarp0 + EW) * 32;
   static constexpr int QR = BN / 2;                       // Q rows staged by each CTA of the pair
   static constexpr int ST_P = kBM * kI8Row, ST_Q = QR * kI8Row;
   static constexpr int NS = BN > 128 ? 6 : 8;             // stages: operand tiles and scales of one K group
   static_assert(NS >= NT, "the epilogue waits on the barrier ring of the stages");
-  static constexpr int SC_F = 2 * (kBM + BN);             // floats per scale stage (with the zero-point vectors)
+  // floats per scale stage: row scales, column scales; then the rows' zero points (each twice, as a pair) and the columns' sums
+  static constexpr int SC_Z = kBM + BN, SC_F = SC_Z + 2 * kBM + BN;
   static constexpr int OFF_SC = NS * (ST_P + ST_Q);
   static constexpr int OFF_BAR = OFF_SC + NS * SC_F * 4;
   static constexpr int NUM_BARS = 3 * NS + NT;
@@ -84,7 +96,7 @@ w4a4_group_f8_kernel(const __grid_constant__ GemmParams p, const __grid_constant
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp < 4) {
-    if (C::REG_EPI != 0) setmaxnreg_dec<C::REG_LOW>();
+    setmaxnreg_dec<C::REG_LOW>();
     SchedT<2> sched;
     TileInfo ti;
     uint32_t it = 0;
@@ -174,14 +186,20 @@ w4a4_group_f8_kernel(const __grid_constant__ GemmParams p, const __grid_constant
             const int row = ti.p0 + j * 32 + lane;
             const bool v = row < ti.p_lim;
             cp_async_4_zfill(dst + (uint32_t)(j * 32 + rslot) * 4u, v ? p.sp + (long long)g * p.sp_gstride + row : p.sp, v);
-            if (AZP) cp_async_4_zfill(dst + (uint32_t)(kBM + BN + j * 32 + rslot) * 4u, v ? p.zp + (long long)g * p.sp_gstride + row : p.sp, v);
+            if (AZP) {
+              // row 8 a + lr of the 32 at [a / 2][lr][a & 1], so that one 16-byte load gives a lane the pairs of two of its rows
+              const uint32_t at = dst + (uint32_t)(C::SC_Z + j * 64 + ((lane >> 4) * 8 + (lane & 7)) * 4 + ((lane >> 3) & 1) * 2) * 4u;
+              const float* src = v ? p.zp + (long long)g * p.sp_gstride + row : p.sp;
+              cp_async_4_zfill(at, src, v);
+              cp_async_4_zfill(at + 4, src, v);
+            }
           }
 #pragma unroll
           for (int j = 0; j < BN / 32; ++j) {
             const int q = ti.q0 + j * 32 + lane;
             const bool v = q < ti.q_lim;
             cp_async_4_zfill(dst + (uint32_t)(kBM + j * 32 + lane) * 4u, v ? p.sq + (long long)g * p.sq_gstride + q : p.sq, v);
-            if (AZP) cp_async_4_zfill(dst + (uint32_t)(2 * kBM + BN + j * 32 + lane) * 4u, v ? p.zq + (long long)g * p.sq_gstride + q : p.sq, v);
+            if (AZP) cp_async_4_zfill(dst + (uint32_t)(C::SC_Z + 2 * kBM + j * 32 + lane) * 4u, v ? p.zq + (long long)g * p.sq_gstride + q : p.sq, v);
           }
           cp_async_mbar_arrive_noinc(bar_full + ss * 8);   // fires when this lane's copies have landed
         }
@@ -189,79 +207,95 @@ w4a4_group_f8_kernel(const __grid_constant__ GemmParams p, const __grid_constant
       cp_async_wait_all();   // nothing of this warp is in flight into shared memory at teardown
     }
   } else {
-    // ---------------- epilogue: 32 rows x 64 columns of every accumulator per warp ----------------
-    if (C::REG_EPI != 0) setmaxnreg_inc<C::REG_EPI == 0 ? 168 : C::REG_EPI>();
-    const int quad = warp & 3, col_base = ((warp - kF8EpiWarp0) >> 2) * 64;
+    // ---------------- epilogue: 32 rows x CW columns of every accumulator per warp ----------------
+    setmaxnreg_inc<C::REG_EPI>();
+    constexpr int CW = C::CW, NCH = CW / 32, STEP = C::STEP;
+    const int quad = warp & 3, col_base = ((warp - kF8EpiWarp0) >> 2) * CW;
     const int lq = lane & 3, lr = lane >> 2;
-    const float* sc = reinterpret_cast<const float*>(smem + C::OFF_SC);
     const uint32_t arr_tm = mapa_shared(bar_tm, 0);
     const uint32_t tm_warp = tmem_base + ((uint32_t)(quad * 32) << 16) + col_base;
+    const uint32_t sc_row = sbase + C::OFF_SC + (uint32_t)(quad * 32 + lr * 4) * 4u;
+    const uint32_t sc_col = sbase + C::OFF_SC + (uint32_t)(kBM + col_base + lq * 8) * 4u;
+    const uint32_t z_row = sbase + C::OFF_SC + (uint32_t)(C::SC_Z + quad * 64 + lr * 4) * 4u;
+    constexpr uint32_t Z_COL = (uint32_t)(C::SC_Z + kBM) * 4u;   // from a column's scale to its sum
     SchedT<2> sched;
     TileInfo ti;
-    uint32_t it = 0;
+    uint32_t it = 0, s = 0, ph = 0, buf = 0;   // group, its stage, the stage's phase, its accumulator
     bool ok = true, pre = false;   // pre: the next group was seen complete under this one's arithmetic
     __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out);
     while (sched.template next<BN>(p, ti)) {
-      float2 f[32];   // [a][c][kk]: row 8a + lr, columns c * 32 + 8 lq + 2 kk + {0, 1}
+      float2 f[CW / 2];   // [a][c][kk]: row 8a + lr, columns c * 32 + 8 lq + 2 kk + {0, 1}
 #pragma unroll
-      for (int i = 0; i < 32; ++i) f[i] = make_float2(0.f, 0.f);
-      for (int g = ti.g0; g < ti.g1; ++g, ++it) {
-        const float* st = sc + (it % C::NS) * C::SC_F;
-        const uint32_t buf = it % C::NT;
+      for (int i = 0; i < CW / 2; ++i) f[i] = make_float2(0.f, 0.f);
+      for (int g = ti.g0; g < ti.g1; ++g) {
+        const uint32_t st = s * (C::SC_F * 4);
         // (the scales of the group arrived with its operands)
-        if (BN == 256 || !__all_sync(0xffffffffu, pre)) ok = wait_bar(bar_done + (it % C::NS) * 8, (it / C::NS) & 1u, abort_flag);
+        if (!__all_sync(0xffffffffu, pre)) ok = wait_bar(bar_done + s * 8, ph, abort_flag);
         if (!ok) break;
         tc_fence_after_sync();
-        const float4 sp = *reinterpret_cast<const float4*>(st + quad * 32 + lr * 4);
-        float4 zp = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (AZP) zp = *reinterpret_cast<const float4*>(st + kBM + BN + quad * 32 + lr * 4);
+        float2 sp[4], zp[AZP ? 4 : 1];
+        {
+          float2 a, b;
+          lds_pairs(sc_row + st, a, b);
+          sp[0] = make_float2(a.x, a.x); sp[1] = make_float2(a.y, a.y); sp[2] = make_float2(b.x, b.x); sp[3] = make_float2(b.y, b.y);
+        }
+        if constexpr (AZP) { lds_pairs(z_row + st, zp[0], zp[1]); lds_pairs(z_row + st + 128, zp[2], zp[3]); }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {   // 16 columns at a time: half of the 32-column chunk c
-          const int c = u >> 1, half = u & 1;
-          uint32_t r[2][8];
-          tmem_ld_16x256b_x2(tm_warp + buf * BN + u * 16, r[0]);
-          tmem_ld_16x256b_x2(tm_warp + buf * BN + (16u << 16) + u * 16, r[1]);
-          const float* sq_at = st + kBM + col_base + c * 32 + lq * 8 + half * 4;
-          const float4 sq = *reinterpret_cast<const float4*>(sq_at);
-          float4 zq = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (AZP) zq = *reinterpret_cast<const float4*>(sq_at + kBM + BN);
+        for (int u = 0; u < CW / STEP; ++u) {   // STEP columns at a time: a 32-column chunk c, or half of one from pair kk0 on
+          const int c = u * STEP / 32, kk0 = (u * STEP / 8) & 3;
+          uint32_t r[2][STEP / 2];
+          const uint32_t tm = tm_warp + buf * BN + u * STEP;
+          if constexpr (STEP == 32) {
+            tmem_ld_16x256b_x4(tm, r[0]);
+            tmem_ld_16x256b_x4(tm + (16u << 16), r[1]);
+          } else {
+            tmem_ld_16x256b_x2(tm, r[0]);
+            tmem_ld_16x256b_x2(tm + (16u << 16), r[1]);
+          }
+          float2 sq[STEP / 8], zq[AZP ? STEP / 8 : 1];
+#pragma unroll
+          for (int i = 0; i < STEP / 8; i += 2) {
+            const uint32_t at = sc_col + st + (uint32_t)(c * 32 + kk0 * 2 + i * 2) * 4u;
+            lds_pairs(at, sq[i], sq[i + 1]);
+            if constexpr (AZP) lds_pairs(at + Z_COL, zq[i], zq[i + 1]);
+          }
           tmem_ld_wait();
-          if (u == 3) {
-            // all of this warp's part of the accumulator is in registers: hand it back to the MMA thread
+          if (u == CW / STEP - 1) {
+            // all of this warp's part of the accumulator and of the scales is in registers: hand both back
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(arr_tm + buf * 8);
-            // (at 256 columns there is no register left for the early probe: it costs 5 % there and gains 4-8 % at 192 and 128)
-            if (BN != 256) pre = mbar_test_wait(bar_done + ((it + 1) % C::NS) * 8, ((it + 1) / C::NS) & 1u);
+            if (lane == 0) { mbar_arrive_cluster(arr_tm + buf * 8); mbar_arrive(bar_sc_empty + s * 8); }
+            pre = mbar_test_wait(bar_done + ((it + 1) % C::NS) * 8, ((it + 1) / C::NS) & 1u);
           }
+          auto fold = [&](int a, int kk) {
+            const int i = 4 * kk + 2 * (a & 1);
+            float2 d = make_float2(__uint_as_float(r[a >> 1][i]), __uint_as_float(r[a >> 1][i + 1]));
+            if constexpr (AZP) d = __ffma2_rn(zp[a], zq[kk], d);
+            float2& acc = f[(a * NCH + c) * 4 + kk0 + kk];
+            acc = __ffma2_rn(__fmul2_rn(d, sp[a]), sq[kk], acc);
+          };
+          if constexpr (STEP == 32) {
 #pragma unroll
-          for (int a = 0; a < 4; ++a) {
-            const float s = a == 0 ? sp.x : a == 1 ? sp.y : a == 2 ? sp.z : sp.w;
-            const float z = a == 0 ? zp.x : a == 1 ? zp.y : a == 2 ? zp.z : zp.w;
+            for (int kk = 0; kk < 4; ++kk) { fold(0, kk); fold(1, kk); fold(2, kk); fold(3, kk); }
+          } else {
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const int i = 4 * e + 2 * (a & 1);
-              float2 d = make_float2(__uint_as_float(r[a >> 1][i]), __uint_as_float(r[a >> 1][i + 1]));
-              if (AZP) d = __ffma2_rn(make_float2(z, z), e ? make_float2(zq.z, zq.w) : make_float2(zq.x, zq.y), d);
-              float2& acc = f[(a * 2 + c) * 4 + 2 * half + e];
-              acc = __ffma2_rn(__fmul2_rn(d, make_float2(s, s)), e ? make_float2(sq.z, sq.w) : make_float2(sq.x, sq.y), acc);
-            }
+            for (int a = 0; a < 4; ++a) { fold(a, 0); fold(a, 1); }
           }
         }
-        __syncwarp();   // every lane has read its scales of this stage
-        if (lane == 0) mbar_arrive(bar_sc_empty + (it % C::NS) * 8);
+        ++it;
+        s = it % C::NS; ph = (it / C::NS) & 1u; buf = it % C::NT;
       }
       if (!ok) break;
       // ---- write the tile: a lane's four pairs of a 32-column chunk are eight consecutive output columns ----
-      const bool vec_ok = ((p.ldc & 7) == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0) && (ti.q0 + col_base + 64 <= ti.q_lim);
+      const bool vec_ok = ((p.ldc & 7) == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0) && (ti.q0 + col_base + CW <= ti.q_lim);
       const bool pair_ok = ((p.ldc & 1) == 0) && ((reinterpret_cast<uintptr_t>(out) & 3) == 0);
 #pragma unroll
       for (int a = 0; a < 4; ++a) {
         const int prow = ti.p0 + quad * 32 + 8 * a + lr;
         if (prow >= ti.p_lim) continue;
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const float2* v = f + (a * 2 + c) * 4;
+        for (int c = 0; c < NCH; ++c) {
+          const float2* v = f + (a * NCH + c) * 4;
           const int q = ti.q0 + col_base + c * 32 + lq * 8;
           if (vec_ok) {
             *reinterpret_cast<uint4*>(out + (long long)prow * p.ldc + q) =

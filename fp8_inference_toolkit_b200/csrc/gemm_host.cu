@@ -89,15 +89,14 @@ static Shape choose_shape(long long M, long long N, int sms, bool allow_swap, bo
 
 // Tile width of the expanded per-group kernel (gemm_f8.cu) for an [M, N] problem with G groups, or 0 where converting
 // inside the GEMM is the better choice.  Both sides are estimated from measured times (B200, 1965 MHz): columns of tile
-// that an SM pair works through one after another x groups x 2.70 ns (192 / 128-column tiles: 2 / 8 % more) here,
-// 3.78 ns per cost unit of choose_shape there, 1.24 and 1.53 times that with the zero-point term and 2 ns a column here;
+// that an SM pair works through one after another x groups x 2.40 ns (192 / 128-column tiles: 5 / 7 % more) here,
+// 3.78 ns per cost unit of choose_shape there, 1.30 and 1.53 times that with the zero-point term and 2 ns a column here;
 // the expansion moves 1.5 bytes per code at 7.1 TB/s (part of it in L2) and is one more launch.  Fitted to both kernels
-// at 1046 sizes (M 129..8192, N 264..24576, K 256..12288, with and without zero points): the choice costs 0.34 % on
-// average against the faster of the two, and what is expanded is slower by 5 % at most (16.4 | 14.9 us in another run of the
-// smallest size below, with zero points).  Around the line (expanded | in-kernel):
-// [256, 4096] x [6144, 4096] 28.5 | 27.2 us, with zero points 32.4 | 39.5; [256, 4096] x [24576, 4096] 67 | 71 and one row
-// more 101 | 74; [512, 4096] x [24576, 4096] 102 | 101, with zero points 123 | 152; [1000, 1024] x [1000, 1024] 14.7 | 12.9,
-// with zero points 15.7 | 15.2.
+// at 712 sizes (M 129..8192, N 264..24576, K 256..12288, with and without zero points): the choice costs 0.5 % on
+// average against the faster of the two.  Around the line (expanded, best width | in-kernel):
+// [256, 4096] x [6144, 4096] 27.5 | 28.1 us, with zero points 31.2 | 39.4; [256, 4096] x [24576, 4096] 65 | 70 and one row
+// more 92 | 74; [512, 4096] x [24576, 4096] 93 | 99, with zero points 114 | 152; [1000, 1024] x [1000, 1024] 14.8 | 13.1,
+// with zero points 14.8 | 15.9.
 static int choose_f8(long long M, long long N, int G, const DeviceInfo& dev, bool azp) {
   const int sms = dev.sm_count;
   if (g_force_bn != 0 || g_force_swap >= 0 || g_force_splits != 0 || g_cta_pairs >= 0 || g_epi_warps != 0 ||
@@ -106,7 +105,7 @@ static int choose_f8(long long M, long long N, int G, const DeviceInfo& dev, boo
   if (M <= 128 || (M + N) * (long long)G >= (1ll << 31) - 65536) return 0;
   int best_bn = 0;
   double best = 1e30, best_columns = 0;
-  const struct { int bn; double w; } cands[3] = {{256, 1.00}, {192, 1.02}, {128, 1.08}};
+  const struct { int bn; double w; } cands[3] = {{256, 1.00}, {192, 1.05}, {128, 1.07}};
   for (const auto& c : cands) {
     const long long tiles = ((M + 255) / 256) * ((N + c.bn - 1) / c.bn), units = sms / 2;
     const double columns = (double)((tiles + units - 1) / units) * c.bn;
@@ -114,7 +113,7 @@ static int choose_f8(long long M, long long N, int G, const DeviceInfo& dev, boo
   }
   double in_kernel = 0;
   choose_shape(M, N, sms, true, true, true, &in_kernel);
-  const double expanded_us = best * G * 0.00270 * (azp ? 1.24 : 1.0) + (azp ? best_columns * 0.002 : 0.0) + 2.7 +
+  const double expanded_us = best * G * 0.00240 * (azp ? 1.30 : 1.0) + (azp ? best_columns * 0.002 : 0.0) + 3.2 +
                              (double)(M + N) * G * (128 * 1.5 / 7.1e6);
   return expanded_us < in_kernel * G * 0.00378 * (azp ? 1.53 : 1.0) ? best_bn : 0;
 }
