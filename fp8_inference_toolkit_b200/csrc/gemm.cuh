@@ -106,6 +106,11 @@ int launch_w4a4_skinny(const uint8_t* x, const uint8_t* w, const float* sx, cons
                        long long M, long long N, int G, bool rowmajor, int epi_mode, int sm_count, unsigned int* status,
                        cudaStream_t st);
 
+// Weight-streaming form of the grouped MoE GEMM for few rows per expert (moe_skinny.cu): the same results bit for bit.
+bool moe_skinny_applicable(long long num_pairs, long long N, int G, long long num_experts);
+int launch_moe_skinny(const uint8_t* a, const float* sa, const uint8_t* b, const float* sb, const int32_t* offsets, void* out,
+                      long long P, long long N, int G, long long num_experts, cudaStream_t st);
+
 // Builds (or fetches from a small per-device cache) a tensor map over packed int4 data.
 // rowmajor: 2-D view [rows, row_bytes]; otherwise 3-D view [slabs, rows, 64].
 int get_tensor_map(int device, const void* base, bool rowmajor, long long rows, long long row_bytes_or_slabs,

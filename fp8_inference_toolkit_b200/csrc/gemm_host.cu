@@ -495,9 +495,16 @@ static int moe_grouped_gemm_impl(const uint8_t* a, const float* scale_a, const u
   DeviceGuard guard(device);
   I4TC_CUDA(guard.err);
 
+  // few rows per expert: stream the weights (unless a test pins the tile shape or the tile kernel).  Rows addressed through a table
+  // keep the tile kernel: its 16-byte stores suit another GPU's memory.
+  const int forced_bn = g_force_bn.load(), path = g_small_m_path.load();
+  if (forced_bn == 0 && (path == 0 || path == 2) && out != nullptr && moe_skinny_applicable(num_pairs, N, (int)num_groups, num_experts) &&
+      aligned_to(a, 16) && aligned_to(b, 16) && aligned_to(out, 4))
+    return launch_moe_skinny(a, scale_a, b, scale_b, expert_offsets, out, num_pairs, N, (int)num_groups, num_experts,
+                             static_cast<cudaStream_t>(stream));
+
   // 256-column tiles amortise the conversion of the activation tile better; narrow outputs fall
   // back to 128 columns.
-  const int forced_bn = g_force_bn.load();
   int bn = forced_bn ? forced_bn : ((N % 256 == 0) ? 256 : 128);
   GemmParams p;
   memset(&p, 0, sizeof(p));

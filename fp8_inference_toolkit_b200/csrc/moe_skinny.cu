@@ -1,0 +1,212 @@
+// Grouped W4A4 GEMM of a MoE layer with few rows per expert: weight streaming through register-fed tensor-core instructions.
+//
+// A decoding batch touches nearly every expert with a handful of rows, so the op is a stream of all experts' weights.  The tile
+// kernel multiplies 128-row tiles (97 % padding at four rows) behind a chain of per-group hand-overs.  Here a warp owns 16
+// weight rows of an expert and their whole K range; lane (g, t) holds 16 bytes of rows g and g + 8, which is an operand fragment once
+// its nibbles are spread, so the weights go from HBM to registers (512 contiguous bytes per load, DEPTH groups ahead) and
+// through nothing else.  The expert's rows wait in shared memory as int8, TOK at a time; an expert with more rows
+// goes over its weights again.  What hides the latency is the number of warps: no barrier, no shared-memory stage for the weights.
+//
+// One warp adds all K groups of its rows in ascending order with the tile kernel's operations (multiply by the row scale, fused
+// multiply-add by the column scale), so the results are the tile kernel's bit for bit.  Nibble arithmetic and fragment
+// layout as in skinny.cu.
+//
+// 128 experts of [1536, 2048] and [2048, 768] (321 MB of weights), top 8, both GEMMs, tile kernel -> this one: 64 tokens 189 -> 73 us
+// (4.4 TB/s), 192 tokens 190 -> 88, 400 tokens 191 -> 137.  Bound by instructions and latency (the nibbles' 24 logic
+// operations and four to sixteen products per warp and group), not by HBM: asking the L2 for a warp's whole K range beforehand
+// changed nothing at 64 tokens and cost 20 % at 192.  Weights through shared memory (cp.async.bulk, two warps a block, ten warps an SM): 123 us
+// at 64 tokens and 325 at 512.
+#include "gemm.cuh"
+#include "ptx.cuh"
+
+namespace i4tc {
+
+namespace {
+
+constexpr int kMoeWarps = 8;
+
+struct MoeSkinnyParams {
+  const uint8_t* a;       // [G, P, 64]
+  const float* sa;        // [G, P]
+  const uint8_t* b;       // [E, G, N, 64]
+  const float* sb;        // [E, G, N]
+  const int32_t* offsets; // [E + 1]
+  __nv_bfloat16* out;     // [P, N]
+  long long P;
+  int N, G;
+};
+
+__device__ __forceinline__ void mma_s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                       uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+__device__ __forceinline__ uint4 low_nibbles(const uint4& w) {
+  return make_uint4((w.x << 4) & 0xF0F0F0F0u, (w.y << 4) & 0xF0F0F0F0u, (w.z << 4) & 0xF0F0F0F0u, (w.w << 4) & 0xF0F0F0F0u);
+}
+__device__ __forceinline__ uint4 high_nibbles(const uint4& w) {
+  return make_uint4(w.x & 0xF0F0F0F0u, w.y & 0xF0F0F0F0u, w.z & 0xF0F0F0F0u, w.w & 0xF0F0F0F0u);
+}
+__device__ __forceinline__ uint4 load_stream(const uint8_t* p) {   // read once: past L1
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
+// Shared memory: even codes [group][TOK][64 B] | odd codes [group][TOK][64 B] | row scales [group][TOK]
+__host__ __device__ constexpr size_t moe_skinny_smem(int G, int tok) { return (size_t)G * tok * (128 + 4); }
+
+// NT: 8-row tiles of the expert's rows handled at once (TOK = 8 NT).  DEPTH: groups of weights in flight per warp.  BLOCKS: per SM.
+template <int NT, int DEPTH, int BLOCKS>
+__global__ void __launch_bounds__(kMoeWarps * 32, BLOCKS) moe_skinny_kernel(const MoeSkinnyParams p) {
+  constexpr int TOK = 8 * NT;
+  extern __shared__ __align__(128) uint8_t smem[];
+  const int e = blockIdx.y;
+  const int r0 = __ldg(p.offsets + e), rows = __ldg(p.offsets + e + 1) - r0;
+  if (rows <= 0) return;   // the whole block
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, t = lane & 3;
+  const int n0 = (blockIdx.x * kMoeWarps + warp) * 16;
+  const bool mine = n0 < p.N;   // a warp past the last rows only helps to stage
+  const int G = p.G;
+  uint8_t* lo_s = smem;
+  uint8_t* hi_s = smem + (size_t)G * TOK * 64;
+  float* sx_s = reinterpret_cast<float*>(smem + (size_t)G * TOK * 128);
+  const long long row = (long long)e * G * p.N + (mine ? n0 : 0) + g;   // weight row of group 0
+  const uint8_t* wsrc = p.b + row * 64 + t * 16;
+  const float* ssrc = p.sb + row;
+  const long long wstep = (long long)p.N * 64;
+
+  uint4 wa[DEPTH], wb[DEPTH];
+  float s0[DEPTH], s1[DEPTH];
+  const uint8_t* wat;
+  const float* sat;
+  auto fetch = [&](int d) {   // the groups in order
+    wa[d] = load_stream(wat);
+    wb[d] = load_stream(wat + 8 * 64);
+    s0[d] = __ldg(sat);
+    s1[d] = __ldg(sat + 8);
+    wat += wstep;
+    sat += p.N;
+  };
+  for (int first = 0; first < rows; first += TOK) {
+    wat = wsrc;
+    sat = ssrc;
+#pragma unroll
+    for (int d = 0; d < DEPTH; ++d)
+      if (d < G) fetch(d);
+    // ---- the next TOK rows of the expert (rows past its end: zero codes, zero scales) ----
+    const int n = min(TOK, rows - first);
+    if (first > 0) __syncthreads();   // the previous rows have been read
+    for (int i = threadIdx.x; i < G * TOK * 4; i += kMoeWarps * 32) {
+      const int j = i & 3, m = (i >> 2) % TOK, grp = (i >> 2) / TOK;
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (m < n) v = __ldg(reinterpret_cast<const uint4*>(p.a + ((long long)grp * p.P + r0 + first + m) * 64) + j);
+      *reinterpret_cast<uint4*>(lo_s + (size_t)i * 16) = low_nibbles(v);
+      *reinterpret_cast<uint4*>(hi_s + (size_t)i * 16) = high_nibbles(v);
+    }
+    for (int i = threadIdx.x; i < G * TOK; i += kMoeWarps * 32) {
+      const int m = i % TOK, grp = i / TOK;
+      sx_s[i] = m < n ? __ldg(p.sa + (long long)grp * p.P + r0 + first + m) * (1.0f / 256.0f) : 0.f;
+    }
+    __syncthreads();
+
+    float f[NT][4];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) f[nt][i] = 0.f;
+    for (int base = 0; base < G; base += DEPTH) {
+#pragma unroll
+      for (int d = 0; d < DEPTH; ++d) {
+        const int grp = base + d;
+        if (grp >= G) break;
+        const uint4 alo = low_nibbles(wa[d]), ahi = high_nibbles(wa[d]), blo = low_nibbles(wb[d]), bhi = high_nibbles(wb[d]);
+        const float sw0 = s0[d], sw1 = s1[d];
+        if (grp + DEPTH < G) fetch(d);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          const int at = (grp * TOK + 8 * nt + g) * 64 + t * 16;
+          const uint4 xlo = *reinterpret_cast<const uint4*>(lo_s + at), xhi = *reinterpret_cast<const uint4*>(hi_s + at);
+          const float2 sx = *reinterpret_cast<const float2*>(sx_s + grp * TOK + 8 * nt + 2 * t);
+          int c[4] = {0, 0, 0, 0};
+          mma_s8(c, alo.x, blo.x, ahi.x, bhi.x, xlo.x, xhi.x);
+          if (NT != 2) {   // two chains of two products (NT = 2 has no registers left for a second)
+            int c2[4] = {0, 0, 0, 0};
+            mma_s8(c2, alo.y, blo.y, ahi.y, bhi.y, xlo.y, xhi.y);
+            mma_s8(c, alo.z, blo.z, ahi.z, bhi.z, xlo.z, xhi.z);
+            mma_s8(c2, alo.w, blo.w, ahi.w, bhi.w, xlo.w, xhi.w);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) c[i] += c2[i];
+          } else {
+            mma_s8(c, alo.y, blo.y, ahi.y, bhi.y, xlo.y, xhi.y);
+            mma_s8(c, alo.z, blo.z, ahi.z, bhi.z, xlo.z, xhi.z);
+            mma_s8(c, alo.w, blo.w, ahi.w, bhi.w, xlo.w, xhi.w);
+          }
+          // (acc * scale_a[g, m]) * scale_b[g, n]; 2^-8 rides on the row's scale (exact)
+          f[nt][0] = fmaf(__int2float_rn(c[0]) * sx.x, sw0, f[nt][0]);
+          f[nt][1] = fmaf(__int2float_rn(c[1]) * sx.y, sw0, f[nt][1]);
+          f[nt][2] = fmaf(__int2float_rn(c[2]) * sx.x, sw1, f[nt][2]);
+          f[nt][3] = fmaf(__int2float_rn(c[3]) * sx.y, sw1, f[nt][3]);
+        }
+      }
+    }
+
+    // ---- lanes g and g ^ 1 swap a row each, so that a lane stores pairs of columns: n0 + (g & ~1) + {0, 1} (+ 8) ----
+    const bool odd = (g & 1) != 0;
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      const float o0 = __shfl_xor_sync(0xffffffffu, odd ? f[nt][0] : f[nt][1], 4);
+      const float o1 = __shfl_xor_sync(0xffffffffu, odd ? f[nt][2] : f[nt][3], 4);
+      const int m = 8 * nt + 2 * t + (odd ? 1 : 0);
+      if (m < n && mine) {
+        __nv_bfloat16* dst = p.out + (long long)(r0 + first + m) * p.N + n0 + (g & ~1);
+        const __nv_bfloat162 lo = odd ? __floats2bfloat162_rn(o0, f[nt][1]) : __floats2bfloat162_rn(f[nt][0], o0);
+        const __nv_bfloat162 hi = odd ? __floats2bfloat162_rn(o1, f[nt][3]) : __floats2bfloat162_rn(f[nt][2], o1);
+        *reinterpret_cast<__nv_bfloat162*>(dst) = lo;
+        *reinterpret_cast<__nv_bfloat162*>(dst + 8) = hi;
+      }
+    }
+  }
+}
+
+template <int NT, int DEPTH, int BLOCKS>
+int launch_nt(const MoeSkinnyParams& p, int num_experts, cudaStream_t st) {
+  const size_t smem = moe_skinny_smem(p.G, 8 * NT);
+  I4TC_CUDA(cudaFuncSetAttribute(moe_skinny_kernel<NT, DEPTH, BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int blocks = (p.N + 16 * kMoeWarps - 1) / (16 * kMoeWarps);
+  moe_skinny_kernel<NT, DEPTH, BLOCKS><<<dim3((unsigned)blocks, (unsigned)num_experts), kMoeWarps * 32, smem, st>>>(p);
+  I4TC_CUDA(cudaGetLastError());
+  return I4TC_OK;
+}
+
+}  // namespace
+
+// 8-row tiles handled at once: the rows an expert has on average, with room for most of their spread.  Beyond 26 rows an expert
+// the tile kernel takes over: it needs 190 us from 4 to 64 rows an expert, this kernel 137 at 25, and 195 with eight tiles at 44.
+static int nt_for(long long num_pairs, long long num_experts) {
+  return num_pairs <= 5 * num_experts ? 1 : num_pairs <= 12 * num_experts ? 2 : 4;
+}
+
+bool moe_skinny_applicable(long long num_pairs, long long N, int G, long long num_experts) {
+  return num_pairs <= 26 * num_experts && N % 16 == 0 && num_experts <= 65535 &&
+         moe_skinny_smem(G, 8 * nt_for(num_pairs, num_experts)) <= 110 * 1024;
+}
+
+int launch_moe_skinny(const uint8_t* a, const float* sa, const uint8_t* b, const float* sb, const int32_t* offsets, void* out,
+                      long long P, long long N, int G, long long num_experts, cudaStream_t st) {
+  MoeSkinnyParams p;
+  p.a = a; p.sa = sa; p.b = b; p.sb = sb; p.offsets = offsets;
+  p.out = static_cast<__nv_bfloat16*>(out);
+  p.P = P; p.N = (int)N; p.G = G;
+  switch (nt_for(P, num_experts)) {
+    case 1: return launch_nt<1, 2, 4>(p, (int)num_experts, st);
+    case 2: return launch_nt<2, 3, 3>(p, (int)num_experts, st);
+    default: return launch_nt<4, 2, 2>(p, (int)num_experts, st);
+  }
+}
+
+}  // namespace i4tc

@@ -1,0 +1,39 @@
+"""GPU: the weight-streaming form of the grouped MoE GEMM gives the tile kernel's bits at the edges of its row tiles (8, 16 and 32
+rows at once, experts without rows, experts that take several passes), of its blocks (N below, at and past 128 rows) and of its
+pipeline (fewer groups than it keeps in flight, odd counts)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("E,counts", [
+    (1, [1]), (4, [0, 5, 0, 8]), (16, [1, 9, 0, 17, 3]),              # 8 rows at once, up to three passes
+    (4, [16, 0, 33, 1]), (3, [12, 12, 12]),                            # 16 at once
+    (4, [32, 31, 40, 1]), (2, [0, 52]),                                # 32 at once, the most rows per expert it takes
+])
+@pytest.mark.parametrize("N,G", [(16, 1), (112, 2), (128, 3), (144, 16), (2048, 6)])
+def test_same_bits_as_the_tile_kernel(E, counts, N, G):
+    from fp8_inference_toolkit_b200 import moe, ops
+
+    counts = counts + [0] * (E - len(counts))
+    P = sum(counts)
+    assert 0 < P <= 26 * E
+    gen = torch.Generator(device="cuda").manual_seed(P + N + G)
+    a = torch.randint(0, 256, (G, P, 64), dtype=torch.uint8, device="cuda", generator=gen)
+    b = torch.randint(0, 256, (E, G, N, 64), dtype=torch.uint8, device="cuda", generator=gen)
+    sa = torch.rand(G, P, device="cuda", generator=gen) * 0.1 + 1e-3
+    sb = torch.rand(E, G, N, device="cuda", generator=gen) * 0.01 + 1e-4
+    off = torch.tensor([sum(counts[:e]) for e in range(E + 1)], dtype=torch.int32, device="cuda")
+    outs = []
+    for path in (3, 0):
+        ops.set_small_m_path(path)
+        try:
+            out = torch.full((P, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+            moe.moe_w4a4_grouped_gemm(a, sa, b, sb, off, out, N, G, E)
+        finally:
+            ops.set_small_m_path(0)
+        outs.append(out)
+    assert not outs[0].isnan().any()
+    assert torch.equal(outs[0], outs[1])
+    ops.check_status()
