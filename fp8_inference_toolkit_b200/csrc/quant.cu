@@ -158,10 +158,17 @@ __device__ __forceinline__ SnapRecip make_snap_recip(float absmax, float s) {
   if (s_above) q.r *= 1.0f - 7.62939453125e-06f;
   return q;
 }
+// Slices whose reciprocal is out of range divide (out of line: inlined, this and the other rare paths made the kernels larger
+// than the instruction cache, a third of their stalls).
+__device__ __noinline__ uint32_t pack8_div_bf16(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, float s) {
+  Vec8<__nv_bfloat16> x;
+  x.w[0] = w0; x.w[1] = w1; x.w[2] = w2; x.w[3] = w3;
+  return pack8_div(x, s);
+}
 // Eight codes of a bf16 slice whose absmax gave q; the same words as pack8_div(x, absmax / 7).
 __device__ __forceinline__ uint32_t pack8_snap(const Vec8<__nv_bfloat16>& x, const SnapRecip& q, bool zero) {
   if (zero) return 0u;
-  if (!q.fast) return pack8_div(x, __fdiv_rn(q.absmax, 7.0f));
+  if (!q.fast) return pack8_div_bf16(x.w[0], x.w[1], x.w[2], x.w[3], __fdiv_rn(q.absmax, 7.0f));
   constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
   const float2 r2 = make_float2(q.r, q.r), off = make_float2(40.f, 40.f), mg = make_float2(kMagic, kMagic);
   const float2 nmg = make_float2(-kMagic - 32.0f, -kMagic - 32.0f);
@@ -291,24 +298,67 @@ __device__ __forceinline__ float exp_reproducible(float t) {
   return __fmul_rn(p, __int_as_float(((int)n + 127) << 23));   // |n| <= 126: an exact power of two
 }
 
-// (g * sigmoid(g)) * u with sigmoid(g) = 1 / (1 + exp_reproducible(-g)): the definition of SwiGLU here.
-__device__ __forceinline__ float silu_mul_reproducible(float g, float u) {
+// (g * sigmoid(g)) * u with sigmoid(g) = 1 / (1 + exp_reproducible(-g)): the definition of SwiGLU here (out of line, it is rare).
+__device__ __noinline__ float silu_mul_reproducible(float g, float u) {
   const float sig = __fdiv_rn(1.0f, __fadd_rn(1.0f, exp_reproducible(-g)));
   return __fmul_rn(__fmul_rn(g, sig), u);
 }
 
-// silu(g) * u rounded to bf16 and widened again: the value the next quantiser sees, bit-identical to
-// bf16(silu_mul_reproducible(g, u)).  The fast evaluation (exp through the special-function unit, documented error
-// 2 + |1.173 x| ulp, and a correctly rounded reciprocal) is within ~17 ulp of that definition for |g| <= 8; it decides
-// the bf16 rounding unless the fp32 value lies within 32 ulp of a rounding boundary (one element in a thousand),
-// and only those elements and the rare |g| > 8 are evaluated by the definition itself.
-__device__ __forceinline__ float silu_mul_bf16(float g, float u) {
-  const float sig = __frcp_rn(1.0f + __expf(-g));
-  float y = __fmul_rn(__fmul_rn(g, sig), u);
-  const uint32_t low = __float_as_uint(y) & 0xFFFFu;
-  const bool near_boundary = (low - (0x8000u - 32u)) <= 64u;
-  if (near_boundary || !(fabsf(g) <= 8.0f)) y = silu_mul_reproducible(g, u);
-  return __bfloat162float(__float2bfloat16_rn(y));
+__device__ __forceinline__ float ex2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// bf16(silu(g) * u) of eight elements, bit-identical to bf16(silu_mul_reproducible(g, u)).
+// A fast evaluation decides unless its fp32 value lies within 32 ulp of a bf16 rounding boundary (one element in a thousand);
+// those elements are evaluated by the definition itself, and so is the whole vector when some |g| > 32 or is not a number.
+//   e**-g = 2**(g * hi) * (1 + g * lo), hi = -log2(e) cut to 16 bits (g has 8, so g * hi is exact), lo = ln 2 times the rest:
+//   within 2^-22 (the instruction's bound) + 2^-24 (the square of g * lo <= 1.6e-4 is below 2^-26);
+//   one reciprocal serves two elements, 1 / a = b * rcp(a b): a, b <= 1 + e**32.
+// With the roundings of the steps (3.5 x 2^-23), of the definition's (2 x 2^-23) and its exponential (2 x 2^-23) the two differ
+// by less than 11 x 2^-23 relative, 22 ulp.
+// Element by element with __expf, an IEEE reciprocal and a branch each: SwiGLU + quantise of [4096, 2 x 12288] 98 us; vectors with the rare paths inlined 79, with them out of line 58.
+__device__ __forceinline__ Vec8<__nv_bfloat16> silu_mul8(const Vec8<__nv_bfloat16>& gv, const Vec8<__nv_bfloat16>& uv) {
+  constexpr float kHi = -1.4426879882812500f;                 // -log2(e) to 16 bits
+  constexpr float kLo = -4.888495152e-06f;                    // (-log2(e) - kHi) * ln 2
+  const float2 hi2 = make_float2(kHi, kHi), lo2 = make_float2(kLo, kLo), one = make_float2(1.f, 1.f);
+  Vec8<__nv_bfloat16> out;
+  float2 y[4];
+  uint32_t nearest = 0xFFFFFFFFu;   // two 16-bit minima of (low half - first near value)
+  __nv_bfloat162 gmax = __habs2(*reinterpret_cast<const __nv_bfloat162*>(&gv.w[0]));
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 g = make_float2(gv.get(2 * i), gv.get(2 * i + 1)), u = make_float2(uv.get(2 * i), uv.get(2 * i + 1));
+    const float2 t = __fmul2_rn(g, hi2);
+    const float2 e0 = make_float2(ex2_approx(t.x), ex2_approx(t.y));
+    const float2 a = __fadd2_rn(__ffma2_rn(e0, __fmul2_rn(g, lo2), e0), one);
+    const float r = rcp_approx(a.x * a.y);
+    y[i] = __fmul2_rn(__fmul2_rn(g, make_float2(a.y * r, a.x * r)), u);
+    const uint32_t low = __byte_perm(__float_as_uint(y[i].x), __float_as_uint(y[i].y), 0x5410);
+    nearest = __viaddmin_u16x2(low, 0x80208020u, nearest);   // low - (0x8000 - 32)
+    const __nv_bfloat162 h = __floats2bfloat162_rn(y[i].x, y[i].y);
+    out.w[i] = *reinterpret_cast<const uint32_t*>(&h);
+    if (i > 0) gmax = __hmax2_nan(gmax, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&gv.w[i])));
+  }
+  const bool large = !(__low2float(gmax) <= 32.0f && __high2float(gmax) <= 32.0f);
+  if ((nearest & 0xFFFFu) <= 64u || (nearest >> 16) <= 64u || large) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const bool nx = large || (__float_as_uint(y[i].x) & 0xFFFFu) - (0x8000u - 32u) <= 64u;
+      const bool ny = large || (__float_as_uint(y[i].y) & 0xFFFFu) - (0x8000u - 32u) <= 64u;
+      if (nx) y[i].x = silu_mul_reproducible(gv.get(2 * i), uv.get(2 * i));
+      if (ny) y[i].y = silu_mul_reproducible(gv.get(2 * i + 1), uv.get(2 * i + 1));
+      const __nv_bfloat162 h = __floats2bfloat162_rn(y[i].x, y[i].y);
+      out.w[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+  }
+  return out;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -337,15 +387,12 @@ __device__ __forceinline__ void load_segment(Vec8<T> (&v)[kQVecs], const T* src,
   if (row_ok && k < K) {
 #pragma unroll
     for (int j = 0; j < kQVecs; ++j) {
-      if (MODE == 2) {
+      if constexpr (MODE == 2) {
         Vec8<T> g, u;
         g.load(src + k + 8 * j);
         u.load(src + K + k + 8 * j);
-        float f[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) f[i] = silu_mul_bf16(g.get(i), u.get(i));
-        v[j].set_all(f);
-      } else if (MODE == 3) {
+        v[j] = silu_mul8(g, u);
+      } else if constexpr (MODE == 3) {
         // RMSNorm in front of the quantiser: bf16(bf16(x * inv_rms) * weight), the roundings of an unfused
         // normalisation that works in fp32 and returns the input's type
         Vec8<T> xv, wv;
@@ -402,7 +449,7 @@ struct QuantOutMap {
 };
 
 template <typename T, int LPG, int MODE, bool GIVEN, bool OUTMAP = false>
-__global__ void __launch_bounds__(256) quant_grouped_kernel(
+__global__ void __launch_bounds__(256, MODE == 2 ? 3 : 1) quant_grouped_kernel(
     const T* __restrict__ x, int64_t rows, int K, int64_t ldx, const int32_t* __restrict__ row_index,
     int index_div, int64_t src_rows, const float* __restrict__ given_scale, uint8_t* __restrict__ packed,
     float* __restrict__ scale, int role, int segs_per_block, const T* __restrict__ aux, float eps,
