@@ -10,6 +10,7 @@
 // max(s, 1/(7*512)) for activations (int4_quant.cu:97,142) and s or 1.0 (all-zero slice) for
 // weights (int4_quant.cu:267).
 #include "common.cuh"
+#include <type_traits>
 
 namespace i4tc {
 
@@ -33,10 +34,6 @@ struct Vec8 {
     for (int i = 0; i < 8; ++i) v[i] = 0.f;
   }
   __device__ __forceinline__ float get(int i) const { return v[i]; }
-  __device__ __forceinline__ void set_all(const float (&f)[8]) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = f[i];
-  }
   __device__ __forceinline__ float absmax() const {
     float m = 0.f;
 #pragma unroll
@@ -55,13 +52,6 @@ struct Vec8<__nv_bfloat16> {
   __device__ __forceinline__ void zero() { w[0] = w[1] = w[2] = w[3] = 0u; }
   __device__ __forceinline__ float get(int i) const {
     return (i & 1) ? __uint_as_float(w[i >> 1] & 0xFFFF0000u) : __uint_as_float(w[i >> 1] << 16);
-  }
-  __device__ __forceinline__ void set_all(const float (&f)[8]) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
-      w[i] = *reinterpret_cast<const uint32_t*>(&h);
-    }
   }
   // |x| maxima of the two 16-bit halves, still packed (max and abs are exact in bf16)
   __device__ __forceinline__ __nv_bfloat162 absmax2() const {
@@ -650,11 +640,74 @@ __device__ __forceinline__ uint32_t pack8_asym(const Vec8<T>& x, const AsymGroup
   return (wl | wh) ^ 0x88888888u;   // u - 8 as a two's-complement nibble is u ^ 8
 }
 
-template <typename T, int LPG, bool ASYM>
+// x / f of one element (out of line: only elements out of the range below come here).
+__device__ __noinline__ float div_exact(float x, float f) { return __fdiv_rn(x, f); }
+
+// v[i] = RN(x[i] / f[i]) for eight 16-bit elements and factors.  An approximate quotient q0 = x * y (y ~ 1 / f within 2^-23) and its
+// remainder r = x - q0 * f, exact in one fused multiply-add, give q = RN(q0 + r * y) (Markstein's correction), which is
+// off x / f by less than 2^-45 relative before the rounding; a quotient of significands of at most 11 bits is no closer than
+// 2^-36 to the middle between two fp32 numbers, so q is the correctly rounded one.  Elements and factors whose quotient or remainder
+// could leave the normal range, zeros of the factor, infinities and NaN divide.
+// [1500, 4096] asymmetric: a division per element in quant_ext_kernel 17.1 us, in this kernel 17.2, corrected reciprocals 11.5.
+template <typename T>
+__device__ __forceinline__ void smooth_div8(const uint4& xu, const uint4& fu, float (&v)[8]) {
+  constexpr bool BF = std::is_same<T, __nv_bfloat16>::value;
+  // magnitudes as integers: bf16 |x| in {0} or [2^-40, 2^60], |f| in [2^-40, 2^40]; fp16 anything finite, |f| > 0
+  constexpr uint32_t kXLo = BF ? 0x2B80u : 1u, kXHi = BF ? 0x5D80u : 0x7BFFu, kFLo = BF ? 0x2B80u : 1u, kFHi = BF ? 0x5380u : 0x7BFFu;
+  const uint32_t xw[4] = {xu.x, xu.y, xu.z, xu.w}, fw[4] = {fu.x, fu.y, fu.z, fu.w};
+  uint32_t xlo = 0xFFFFFFFFu, xhi = 0u, flo = 0xFFFFFFFFu, fhi = 0u;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t xa = xw[i] & 0x7FFF7FFFu, fa = fw[i] & 0x7FFF7FFFu;
+    xlo = __viaddmin_u16x2(xa, 0xFFFFFFFFu, xlo);   // (a zero becomes the largest value)
+    xhi = __vmaxu2(xa, xhi);
+    flo = __vminu2(fa, flo);
+    fhi = __vmaxu2(fa, fhi);
+    float2 x, f;
+    if constexpr (BF) {
+      x = make_float2(__uint_as_float(xw[i] << 16), __uint_as_float(xw[i] & 0xFFFF0000u));
+      f = make_float2(__uint_as_float(fw[i] << 16), __uint_as_float(fw[i] & 0xFFFF0000u));
+    } else {
+      x = __half22float2(*reinterpret_cast<const __half2*>(&xw[i]));
+      f = __half22float2(*reinterpret_cast<const __half2*>(&fw[i]));
+    }
+    const float2 y = make_float2(rcp_approx(f.x), rcp_approx(f.y));
+    const float2 q0 = __fmul2_rn(x, y);
+    const float2 r = __ffma2_rn(make_float2(-q0.x, -q0.y), f, x);
+    const float2 q = __ffma2_rn(r, y, q0);
+    v[2 * i] = q.x;
+    v[2 * i + 1] = q.y;
+  }
+  const bool ok = (xlo & 0xFFFFu) + 1u >= kXLo && (xlo >> 16) + 1u >= kXLo &&
+                  (xhi & 0xFFFFu) <= kXHi && (xhi >> 16) <= kXHi && (flo & 0xFFFFu) >= kFLo && (flo >> 16) >= kFLo &&
+                  (fhi & 0xFFFFu) <= kFHi && (fhi >> 16) <= kFHi;
+  if (!ok) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float x, f;
+      const uint32_t xi = (xw[i / 2] >> (16 * (i & 1))) & 0xFFFFu, fi = (fw[i / 2] >> (16 * (i & 1))) & 0xFFFFu;
+      if constexpr (BF) {
+        x = __uint_as_float(xi << 16);
+        f = __uint_as_float(fi << 16);
+      } else {
+        x = __half2float(__ushort_as_half((unsigned short)xi));
+        f = __half2float(__ushort_as_half((unsigned short)fi));
+      }
+      v[i] = div_exact(x, f);
+    }
+  }
+}
+
+template <typename T>
+constexpr uint32_t kOnes = std::is_same<T, __nv_bfloat16>::value ? 0x3F803F80u : 0x3C003C00u;   // 1.0 twice
+
+// SMOOTH: every element is divided (IEEE, fp32) by its channel's factor first, and fp32 values are quantised.
+template <typename T, int LPG, bool ASYM, bool SMOOTH>
 __global__ void __launch_bounds__(256) quant_grouped_ext_kernel(const T* __restrict__ x, int64_t rows, int K,
-                                                                int64_t ldx, float clip, uint8_t* __restrict__ packed,
-                                                                float* __restrict__ scale,
+                                                                int64_t ldx, float clip, const T* __restrict__ smooth,
+                                                                uint8_t* __restrict__ packed, float* __restrict__ scale,
                                                                 float* __restrict__ azp_adj, int segs_per_block) {
+  using V = typename std::conditional<SMOOTH, float, T>::type;
   constexpr int GS = LPG * kQLane;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t r = (int64_t)blockIdx.x * kQRows + warp;
@@ -663,15 +716,29 @@ __global__ void __launch_bounds__(256) quant_grouped_ext_kernel(const T* __restr
   const int seg_begin = blockIdx.y * segs_per_block;
   const int seg_end = min(nseg, seg_begin + segs_per_block);
   const T* src = row_ok ? x + r * ldx : nullptr;
-  Vec8<T> cur[kQVecs], nxt[kQVecs];
-  load_segment<T, 0>(cur, src, seg_begin * kQSeg + lane * kQLane, K, row_ok);
+  using S = typename std::conditional<SMOOTH, __nv_bfloat16, T>::type;   // SMOOTH keeps 16-bit words, whatever they hold
+  Vec8<S> cur[kQVecs], nxt[kQVecs];
+  const S* ssrc = reinterpret_cast<const S*>(src);
+  load_segment<S, 0>(cur, ssrc, seg_begin * kQSeg + lane * kQLane, K, row_ok);
   for (int seg = seg_begin; seg < seg_end; ++seg) {
     const int k = seg * kQSeg + lane * kQLane;
-    if (seg + 1 < seg_end) load_segment<T, 0>(nxt, src, k + kQSeg, K, row_ok);
+    if (seg + 1 < seg_end) load_segment<S, 0>(nxt, ssrc, k + kQSeg, K, row_ok);
     const bool ok = row_ok && k < K;
     const int g = k / GS;
     float mn, mx;
-    minmax_of(cur, mn, mx);
+    Vec8<V> val[kQVecs];
+    if constexpr (SMOOTH) {
+#pragma unroll
+      for (int j = 0; j < kQVecs; ++j) {
+        uint4 f = make_uint4(kOnes<T>, kOnes<T>, kOnes<T>, kOnes<T>);   // (past the row's end: zeros over ones)
+        if (k < K) f = __ldg(reinterpret_cast<const uint4*>(smooth + k + 8 * j));
+        smooth_div8<T>(make_uint4(cur[j].w[0], cur[j].w[1], cur[j].w[2], cur[j].w[3]), f, val[j].v);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < kQVecs; ++j) val[j] = cur[j];
+    }
+    minmax_of(val, mn, mx);
 #pragma unroll
     for (int o = 1; o < LPG; o <<= 1) {
       mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
@@ -693,19 +760,19 @@ __global__ void __launch_bounds__(256) quant_grouped_ext_kernel(const T* __restr
         scale[(int64_t)g * rows + r] = q.s;
         azp_adj[(int64_t)g * rows + r] = 8.0f - q.azp;
       }
-      w.x = pack8_asym<T>(cur[0], q);
-      w.y = pack8_asym<T>(cur[1], q);
-      w.z = pack8_asym<T>(cur[2], q);
-      w.w = pack8_asym<T>(cur[3], q);
+      w.x = pack8_asym<V>(val[0], q);
+      w.y = pack8_asym<V>(val[1], q);
+      w.z = pack8_asym<V>(val[2], q);
+      w.w = pack8_asym<V>(val[3], q);
     } else {
       const float s = __fdiv_rn(thr, 7.0f);
       const bool zero = !(s > 0.0f);
       const Recip q = make_recip<false>(zero ? 1.0f : s);
       if (ok && (lane % LPG) == 0) scale[(int64_t)g * rows + r] = fmaxf(s, min_scale());
-      w.x = pack8<T, true>(cur[0], q, zero);
-      w.y = pack8<T, true>(cur[1], q, zero);
-      w.z = pack8<T, true>(cur[2], q, zero);
-      w.w = pack8<T, true>(cur[3], q, zero);
+      w.x = pack8<V, true>(val[0], q, zero);
+      w.y = pack8<V, true>(val[1], q, zero);
+      w.z = pack8<V, true>(val[2], q, zero);
+      w.w = pack8<V, true>(val[3], q, zero);
     }
     if (ok) *reinterpret_cast<uint4*>(packed + ((int64_t)g * rows + r) * (GS / 2) + (lane % LPG) * 16) = w;
 #pragma unroll
@@ -713,8 +780,8 @@ __global__ void __launch_bounds__(256) quant_grouped_ext_kernel(const T* __restr
   }
 }
 
-template <typename T, bool ASYM>
-static int launch_grouped_ext_t(const T* x, int64_t rows, int64_t K, int64_t ldx, int gs, float clip, uint8_t* packed,
+template <typename T, bool ASYM, bool SMOOTH = false>
+static int launch_grouped_ext_t(const T* x, int64_t rows, int64_t K, int64_t ldx, int gs, float clip, const T* smooth, uint8_t* packed,
                                 float* scale, float* azp_adj, cudaStream_t st) {
   const int64_t row_blocks = (rows + kQRows - 1) / kQRows;
   const int nseg = (int)((K + kQSeg - 1) / kQSeg);
@@ -723,33 +790,38 @@ static int launch_grouped_ext_t(const T* x, int64_t rows, int64_t K, int64_t ldx
   if (spb < 1) spb = 1;
   dim3 grid((unsigned)row_blocks, (unsigned)((nseg + spb - 1) / spb));
   I4TC_REQUIRE(grid.y <= 65535, I4TC_EINVAL, "K=%lld too large for the grouped quantiser", (long long)K);
+#define I4TC_LAUNCH_E(LPG) \
+  quant_grouped_ext_kernel<T, LPG, ASYM, SMOOTH><<<grid, 256, 0, st>>>(x, rows, (int)K, ldx, clip, smooth, packed, scale, azp_adj, spb)
   switch (gs) {
-    case 64: quant_grouped_ext_kernel<T, 2, ASYM><<<grid, 256, 0, st>>>(x, rows, (int)K, ldx, clip, packed, scale, azp_adj, spb); break;
-    case 128: quant_grouped_ext_kernel<T, 4, ASYM><<<grid, 256, 0, st>>>(x, rows, (int)K, ldx, clip, packed, scale, azp_adj, spb); break;
-    case 256: quant_grouped_ext_kernel<T, 8, ASYM><<<grid, 256, 0, st>>>(x, rows, (int)K, ldx, clip, packed, scale, azp_adj, spb); break;
+    case 64: I4TC_LAUNCH_E(2); break;
+    case 128: I4TC_LAUNCH_E(4); break;
+    case 256: I4TC_LAUNCH_E(8); break;
     default: return fail(I4TC_EUNSUPPORTED, "group_size=%d not supported (64, 128 or 256)", gs);
   }
+#undef I4TC_LAUNCH_E
   I4TC_CUDA(cudaGetLastError());
   return I4TC_OK;
 }
 
-// Whether the vectorised kernel can take this call: 16-byte aligned rows and outputs (it moves 128 bits per lane).
-bool grouped_ext_fast_ok(const void* x, int64_t ldx, const uint8_t* packed) {
-  return aligned_to(x, 16) && (ldx * 2) % 16 == 0 && aligned_to(packed, 16);
+// Whether the vectorised kernel can take this call: 16-byte aligned rows, smoothing factors and outputs (it moves 128 bits per lane).
+bool grouped_ext_fast_ok(const void* x, int64_t ldx, const void* smooth, const uint8_t* packed) {
+  return aligned_to(x, 16) && (ldx * 2) % 16 == 0 && aligned_to(smooth, 16) && aligned_to(packed, 16);
+}
+
+template <typename T>
+static int launch_grouped_ext_d(bool asym, const void* x, int64_t rows, int64_t K, int64_t ldx, int gs, float clip, const void* smooth,
+                                uint8_t* packed, float* scale, float* azp_adj, cudaStream_t st) {
+  const T* p = static_cast<const T*>(x);
+  const T* f = static_cast<const T*>(smooth);
+  if (!asym) return launch_grouped_ext_t<T, false>(p, rows, K, ldx, gs, clip, nullptr, packed, scale, azp_adj, st);
+  return f == nullptr ? launch_grouped_ext_t<T, true>(p, rows, K, ldx, gs, clip, nullptr, packed, scale, azp_adj, st)
+                      : launch_grouped_ext_t<T, true, true>(p, rows, K, ldx, gs, clip, f, packed, scale, azp_adj, st);
 }
 
 int launch_grouped_ext(bool asym, const void* x, int dtype, int64_t rows, int64_t K, int64_t ldx, int gs, float clip,
-                       uint8_t* packed, float* scale, float* azp_adj, cudaStream_t st) {
-  if (dtype == I4TC_BF16) {
-    const __nv_bfloat16* p = static_cast<const __nv_bfloat16*>(x);
-    return asym ? launch_grouped_ext_t<__nv_bfloat16, true>(p, rows, K, ldx, gs, clip, packed, scale, azp_adj, st)
-                : launch_grouped_ext_t<__nv_bfloat16, false>(p, rows, K, ldx, gs, clip, packed, scale, azp_adj, st);
-  }
-  if (dtype == I4TC_FP16) {
-    const __half* p = static_cast<const __half*>(x);
-    return asym ? launch_grouped_ext_t<__half, true>(p, rows, K, ldx, gs, clip, packed, scale, azp_adj, st)
-                : launch_grouped_ext_t<__half, false>(p, rows, K, ldx, gs, clip, packed, scale, azp_adj, st);
-  }
+                       const void* smooth, uint8_t* packed, float* scale, float* azp_adj, cudaStream_t st) {
+  if (dtype == I4TC_BF16) return launch_grouped_ext_d<__nv_bfloat16>(asym, x, rows, K, ldx, gs, clip, smooth, packed, scale, azp_adj, st);
+  if (dtype == I4TC_FP16) return launch_grouped_ext_d<__half>(asym, x, rows, K, ldx, gs, clip, smooth, packed, scale, azp_adj, st);
   return fail(I4TC_EUNSUPPORTED, "input must be bf16 or fp16 (dtype %d)", dtype);
 }
 

@@ -1,7 +1,7 @@
 // Clipped, asymmetric and smoothed per-group activation quantisers, the per-group sums of weight codes, and
 // the zero-point pass that finishes a per-group linear whose activations were quantised asymmetrically.
 //
-// Quantisers: a warp works on four (row, K-group) slices at a time, all 32 lanes on each; a lane keeps its
+// Quantisers (for rows, factors or outputs that the 128-bit kernels of quant.cu cannot take): a warp works on four (row, K-group) slices at a time, all 32 lanes on each; a lane keeps its
 // gs/32 consecutive elements of every slice in registers between the reductions (warp shuffles) and the quantise
 // step, so the input is read once; per slice the warp writes gs/2 contiguous bytes.  The reference launches one 256-thread block per slice and reads it two or
 // three times (int4_native_tc/csrc/int4_quant.cu:857-903, 1189-1259, 1324-1430).
@@ -219,10 +219,10 @@ int launch_ext(const void* x, int dtype, int64_t rows, int64_t K, int64_t ldx, i
   DeviceGuard guard(device);
   I4TC_CUDA(guard.err);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // without a smoothing vector the 128-bit kernel does the same arithmetic at a fraction of the instructions
-  if (smooth == nullptr && K % 32 == 0 && (dtype == I4TC_BF16 || dtype == I4TC_FP16) &&
-      grouped_ext_fast_ok(x, ldx, packed))
-    return launch_grouped_ext(ASYM, x, dtype, rows, K, ldx, (int)group_size, (float)clip_ratio, packed, scale, azp_adj,
+  // the 128-bit kernel does the same arithmetic at a fraction of the instructions
+  if ((smooth == nullptr || ASYM) && K % 32 == 0 && (dtype == I4TC_BF16 || dtype == I4TC_FP16) &&
+      grouped_ext_fast_ok(x, ldx, smooth, packed))
+    return launch_grouped_ext(ASYM, x, dtype, rows, K, ldx, (int)group_size, (float)clip_ratio, smooth, packed, scale, azp_adj,
                               st);
   if (dtype == I4TC_BF16)
     return launch_ext_t<__nv_bfloat16, ASYM>(static_cast<const __nv_bfloat16*>(x), rows, K, ldx, (int)group_size,
