@@ -69,45 +69,87 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_kernel(const __nv_bfloat
   }
 }
 
-// Heads [0, q_heads) with wq and [q_heads, q_heads + k_heads) with wk of every token of qkv (row stride ld, heads of 128):
-// normalise, then rotate halves by the token's position (token % seq), in place.  A warp takes a head, a lane four
-// consecutive elements; the other half of the rotation is 16 lanes away.  Every bf16 rounding of the separate ops is
-// kept, so results differ from theirs by the order of the sum of squares only.
-__global__ void __launch_bounds__(256) qk_norm_rope_kernel(__nv_bfloat16* __restrict__ qkv, long long tokens, long long ld, int q_heads,
-                                                          int heads, int seq, const __nv_bfloat16* __restrict__ wq,
-                                                          const __nv_bfloat16* __restrict__ wk,
-                                                          const __nv_bfloat16* __restrict__ cos_t,
-                                                          const __nv_bfloat16* __restrict__ sin_t, float eps) {
-  const int lane = threadIdx.x & 31;
-  const long long item = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (item >= tokens * heads) return;   // whole warps
-  const long long tok = item / heads;
-  const int head = (int)(item - tok * heads);
-  uint2* at = reinterpret_cast<uint2*>(qkv + tok * ld + head * 128) + lane;
-  const uint2 u = *at;
-  const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y);
-  float s = a.x * a.x;
-  s = fmaf(a.y, a.y, s); s = fmaf(b.x, b.x, s); s = fmaf(b.y, b.y, s);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  const float r = rsqrtf(s * (1.0f / 128.0f) + eps);
-  const uint2 gw = __ldg(reinterpret_cast<const uint2*>(head < q_heads ? wq : wk) + lane);
-  const float2 g0 = unpack_bf16x2(gw.x), g1 = unpack_bf16x2(gw.y);
-  const float x[4] = {bf16_round(bf16_round(a.x * r) * g0.x), bf16_round(bf16_round(a.y * r) * g0.y),
-                      bf16_round(bf16_round(b.x * r) * g1.x), bf16_round(bf16_round(b.y * r) * g1.y)};
-  const long long row = (tok % seq) * 16 + (lane & 15);   // tables [seq, 64]: 16 uint2 a row
-  const uint2 cu = __ldg(reinterpret_cast<const uint2*>(cos_t) + row), su = __ldg(reinterpret_cast<const uint2*>(sin_t) + row);
-  const float2 c0 = unpack_bf16x2(cu.x), c1 = unpack_bf16x2(cu.y), s0 = unpack_bf16x2(su.x), s1 = unpack_bf16x2(su.y);
-  const float c[4] = {c0.x, c0.y, c1.x, c1.y}, sn[4] = {s0.x, s0.y, s1.x, s1.y};
-  const bool low = lane < 16;
-  float o[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float y = __shfl_xor_sync(0xffffffffu, x[i], 16);
-    const float p = bf16_round(x[i] * c[i]), q = bf16_round(y * sn[i]);
-    o[i] = low ? p - q : p + q;   // x1 c - x2 s | x2 c + x1 s
+// Heads [0, q_heads) with wq and [q_heads, heads) with wk of every token of qkv (row stride ld, heads of 128):
+// normalise, then rotate halves by the token's position (token % seq), in place.  A block takes a token and a warp two heads at a
+// time, a lane eight consecutive elements of one; the other half of the rotation is 8 lanes away.  Tables and weights stay in
+// registers over the heads.  Every bf16 rounding of the separate ops is kept, so results differ from theirs by the order of the sum of
+// squares only (four-element chains, then partners 64, 32, 16, 8 and 4 elements away).
+// A warp per head with 8-byte accesses, an index division per head and single conversions was bound by the special-function unit:
+// [4096, 40 heads] 38.6 us -> 14.5 (5.8 TB/s of the one read and one write).
+constexpr int kRopeWarps = 4;
+
+// Eight bf16 as one 16-byte access, or as two of 8 where an operand is aligned to no more.
+template <bool A16>
+__device__ __forceinline__ uint4 load_oct(const __nv_bfloat16* p) {
+  if constexpr (A16) return *reinterpret_cast<const uint4*>(p);
+  const uint2 a = *reinterpret_cast<const uint2*>(p), b = *reinterpret_cast<const uint2*>(p + 4);
+  return make_uint4(a.x, a.y, b.x, b.y);
+}
+template <bool A16>
+__device__ __forceinline__ void store_oct(__nv_bfloat16* p, const uint4& v) {
+  if constexpr (A16) {
+    *reinterpret_cast<uint4*>(p) = v;
+  } else {
+    *reinterpret_cast<uint2*>(p) = make_uint2(v.x, v.y);
+    *reinterpret_cast<uint2*>(p + 4) = make_uint2(v.z, v.w);
   }
-  *at = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
+}
+
+template <bool A16>
+__global__ void __launch_bounds__(kRopeWarps * 32) qk_norm_rope_kernel(__nv_bfloat16* __restrict__ qkv, long long ld, int q_heads,
+                                                                       int heads, int seq, const __nv_bfloat16* __restrict__ wq,
+                                                                       const __nv_bfloat16* __restrict__ wk,
+                                                                       const __nv_bfloat16* __restrict__ cos_t,
+                                                                       const __nv_bfloat16* __restrict__ sin_t, float eps) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l = lane & 15;
+  const unsigned tok = blockIdx.x;
+  __nv_bfloat16* at = qkv + (long long)tok * ld + l * 8;
+  const long long row = (long long)(tok % (unsigned)seq) * 64 + (l & 7) * 8;   // tables [seq, 64]
+  const uint4 cu = load_oct<A16>(cos_t + row), su = load_oct<A16>(sin_t + row);
+  const uint4 gq = load_oct<A16>(wq + l * 8), gk = load_oct<A16>(wk + l * 8);
+  const uint32_t c[4] = {cu.x, cu.y, cu.z, cu.w}, sn[4] = {su.x, su.y, su.z, su.w};
+  auto b2 = [](uint32_t u) { return *reinterpret_cast<const __nv_bfloat162*>(&u); };
+  int h = warp * 2 + (lane >> 4);
+  uint4 cur = make_uint4(0u, 0u, 0u, 0u);
+  if (h < heads) cur = load_oct<A16>(at + (long long)h * 128);
+  for (int h0 = warp * 2; h0 < heads; h0 += kRopeWarps * 2, h += kRopeWarps * 2) {   // the same trips for both halves of the warp
+    uint4 nxt = make_uint4(0u, 0u, 0u, 0u);
+    if (h + kRopeWarps * 2 < heads) nxt = load_oct<A16>(at + (long long)(h + kRopeWarps * 2) * 128);
+    const uint32_t u[4] = {cur.x, cur.y, cur.z, cur.w};
+    float2 f[4];
+    float s[2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) f[i] = unpack_bf16x2(u[i]);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      s[i] = f[2 * i].x * f[2 * i].x;
+      s[i] = fmaf(f[2 * i].y, f[2 * i].y, s[i]);
+      s[i] = fmaf(f[2 * i + 1].x, f[2 * i + 1].x, s[i]);
+      s[i] = fmaf(f[2 * i + 1].y, f[2 * i + 1].y, s[i]);
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
+      s[1] += __shfl_xor_sync(0xffffffffu, s[1], o);
+    }
+    const float r = rsqrtf((s[0] + s[1]) * (1.0f / 128.0f) + eps);
+    const bool q = h < q_heads;
+    const uint32_t gw[4] = {q ? gq.x : gk.x, q ? gq.y : gk.y, q ? gq.z : gk.z, q ? gq.w : gk.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      // (products of two bf16 are exact in fp32 and a sum of two is never closer to a bf16 tie than fp32 resolves: the packed operations
+      // round like fp32 ones rounded to bf16)
+      const __nv_bfloat162 x = __hmul2_rn(__floats2bfloat162_rn(f[i].x * r, f[i].y * r), b2(gw[i]));
+      const uint32_t mine = *reinterpret_cast<const uint32_t*>(&x);
+      const uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 8);
+      const __nv_bfloat162 p = __hmul2_rn(x, b2(c[i])), t = __hmul2_rn(b2(other), b2(sn[i]));
+      const __nv_bfloat162 y = l < 8 ? __hsub2_rn(p, t) : __hadd2_rn(p, t);   // x1 c - x2 s | x2 c + x1 s
+      o[i] = *reinterpret_cast<const uint32_t*>(&y);
+    }
+    if (h < heads) store_oct<A16>(at + (long long)h * 128, make_uint4(o[0], o[1], o[2], o[3]));
+    cur = nxt;
+  }
 }
 
 }  // namespace i4tc
@@ -143,8 +185,10 @@ extern "C" int i4tc_qk_norm_rope(void* qkv, int64_t tokens, int64_t ld, int64_t 
                    aligned_to(cos_table, 8) && aligned_to(sin_table, 8), I4TC_EALIGN, "operands must be 8-byte aligned");
   DeviceGuard guard(device);
   I4TC_CUDA(guard.err);
-  qk_norm_rope_kernel<<<(unsigned)((tokens * heads + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<__nv_bfloat16*>(qkv), tokens, ld, (int)q_heads, (int)heads, (int)seq, static_cast<const __nv_bfloat16*>(q_weight),
+  const bool a16 = aligned_to(qkv, 16) && ld % 8 == 0 && aligned_to(q_weight, 16) && aligned_to(k_weight, 16) &&
+                   aligned_to(cos_table, 16) && aligned_to(sin_table, 16);
+  (a16 ? qk_norm_rope_kernel<true> : qk_norm_rope_kernel<false>)<<<(unsigned)tokens, kRopeWarps * 32, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<__nv_bfloat16*>(qkv), ld, (int)q_heads, (int)heads, (int)seq, static_cast<const __nv_bfloat16*>(q_weight),
       static_cast<const __nv_bfloat16*>(k_weight), static_cast<const __nv_bfloat16*>(cos_table),
       static_cast<const __nv_bfloat16*>(sin_table), eps);
   I4TC_CUDA(cudaGetLastError());
