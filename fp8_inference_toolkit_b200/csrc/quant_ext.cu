@@ -311,6 +311,117 @@ __global__ void __launch_bounds__(256) quant_int8_rowwise_kernel(const T* __rest
   }
 }
 
+// The same with the row in registers (K a multiple of 8, at most 8 x 2048), for 16-bit inputs: one pass over memory and no division per
+// element.  y = x * r with r = 127 / absmax within 1.8e-7 lies within 4e-5 of RN(x / s), so unless it is within 1e-4 of a half the
+// nearest integer is the code; vectors with another element (two in ten thousand, and exact halves) divide.  Two passes with a division per element:
+// [512, 12288] 11.2 us -> 6.6.
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float c;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(c) : "f"(a), "f"(b));
+  return c;
+}
+template <typename T>
+__device__ __forceinline__ float2 widen_pair(uint32_t w) {
+  float2 f;
+  widen2<T>(w, f.x, f.y);
+  return f;
+}
+template <typename T>
+__device__ __forceinline__ float absmax_words(const uint4& u, float m) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 f = widen_pair<T>(w[i]);
+    m = fmaxf(m, fmaxf(fabsf(f.x), fabsf(f.y)));
+  }
+  return m;
+}
+
+// Eight codes by division (out of line: it is rare and long).
+template <typename T>
+__device__ __noinline__ uint2 int8_codes_exact(uint4 u, float s, bool zero) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+  uint32_t b[2] = {0u, 0u};
+  if (!zero) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = widen_pair<T>(w[i]);
+      const int lo = (int)fminf(fmaxf(rintf(__fdiv_rn(f.x, s)), -128.0f), 127.0f), hi = (int)fminf(fmaxf(rintf(__fdiv_rn(f.y, s)), -128.0f), 127.0f);
+      b[i >> 1] |= (((uint32_t)lo & 0xFFu) | (((uint32_t)hi & 0xFFu) << 8)) << (16 * (i & 1));
+    }
+  }
+  return make_uint2(b[0], b[1]);
+}
+
+template <typename T, int NCH>
+__global__ void __launch_bounds__(256) quant_int8_row_kernel(const T* __restrict__ x, int K, int64_t ldx, int8_t* __restrict__ q,
+                                                             float* __restrict__ scale) {
+  __shared__ float s_max[8];
+  const int64_t r = blockIdx.x;
+  const T* src = x + r * ldx;
+  int8_t* dst = q + r * (int64_t)K;
+  const int t = threadIdx.x;
+  uint4 u[NCH];
+  float m = 0.f;
+#pragma unroll
+  for (int c = 0; c < NCH; ++c) {
+    const int k = c * 2048 + t * 8;
+    u[c] = k < K ? __ldg(reinterpret_cast<const uint4*>(src + k)) : make_uint4(0u, 0u, 0u, 0u);
+  }
+#pragma unroll
+  for (int c = 0; c < NCH; ++c) m = absmax_words<T>(u[c], m);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((t & 31) == 0) s_max[t >> 5] = m;
+  __syncthreads();
+  m = s_max[0];
+#pragma unroll
+  for (int i = 1; i < 8; ++i) m = fmaxf(m, s_max[i]);
+  const float s = __fdiv_rn(m, 127.0f);
+  if (t == 0) scale[r] = fmaxf(s, 1.0f / (127.0f * 512.0f));
+  float rc;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rc) : "f"(m));
+  rc *= 127.0f;
+  const bool fast = rc > 7.8886090522e-31f && rc < 1.2676506002e30f;   // 2^-100 .. 2^100
+  constexpr float kMagic = 12582912.0f;   // 1.5 * 2^23
+  const float2 r2 = make_float2(rc, rc), mg = make_float2(kMagic, kMagic), nmg = make_float2(-kMagic, -kMagic);
+#pragma unroll
+  for (int c = 0; c < NCH; ++c) {
+    const int k = c * 2048 + t * 8;
+    if (k >= K) continue;
+    const uint32_t w[4] = {u[c].x, u[c].y, u[c].z, u[c].w};
+    uint32_t b[4];   // two's complement in the low bytes of 1.5 * 2^23 + code
+    float worst = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = widen_pair<T>(w[i]);
+      const float2 v = __ffma2_rn(f, r2, mg), n = __fadd2_rn(v, nmg);
+      const float2 d = __ffma2_rn(f, r2, make_float2(-n.x, -n.y));
+      worst = max_nan(worst, max_nan(fabsf(d.x), fabsf(d.y)));   // (an element that is not a number goes the long way)
+      b[i] = __byte_perm(__float_as_uint(v.x), __float_as_uint(v.y), 0x0040);
+    }
+    uint2 codes = make_uint2(__byte_perm(b[0], b[1], 0x5410), __byte_perm(b[2], b[3], 0x5410));
+    if (!fast || !(worst <= 0.5f - 1e-4f)) codes = int8_codes_exact<T>(u[c], s, m == 0.f);
+    *reinterpret_cast<uint2*>(dst + k) = codes;
+  }
+}
+
+template <typename T>
+int launch_int8_rows(const T* x, int64_t rows, int64_t K, int64_t ldx, int8_t* q, float* scale, cudaStream_t st) {
+  const unsigned grid = (unsigned)rows;
+  if (K % 8 == 0 && K <= 16384 && aligned_to(x, 16) && (ldx * 2) % 16 == 0 && aligned_to(q, 8)) {
+    if (K <= 2048) quant_int8_row_kernel<T, 1><<<grid, 256, 0, st>>>(x, (int)K, ldx, q, scale);
+    else if (K <= 4096) quant_int8_row_kernel<T, 2><<<grid, 256, 0, st>>>(x, (int)K, ldx, q, scale);
+    else if (K <= 8192) quant_int8_row_kernel<T, 4><<<grid, 256, 0, st>>>(x, (int)K, ldx, q, scale);
+    else if (K <= 12288) quant_int8_row_kernel<T, 6><<<grid, 256, 0, st>>>(x, (int)K, ldx, q, scale);
+    else quant_int8_row_kernel<T, 8><<<grid, 256, 0, st>>>(x, (int)K, ldx, q, scale);
+  } else {
+    quant_int8_rowwise_kernel<T><<<grid, 256, 0, st>>>(x, (int)K, ldx, q, scale);
+  }
+  I4TC_CUDA(cudaGetLastError());
+  return I4TC_OK;
+}
+
 }  // namespace i4tc
 
 using namespace i4tc;
@@ -324,12 +435,8 @@ extern "C" int i4tc_quant_rowwise_int8(const void* x, int dtype, int64_t rows, i
   I4TC_CUDA(guard.err);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   switch (dtype) {
-    case I4TC_BF16:
-      quant_int8_rowwise_kernel<__nv_bfloat16><<<(unsigned)rows, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), (int)K, ldx, q, scale);
-      break;
-    case I4TC_FP16:
-      quant_int8_rowwise_kernel<__half><<<(unsigned)rows, 256, 0, st>>>(static_cast<const __half*>(x), (int)K, ldx, q, scale);
-      break;
+    case I4TC_BF16: return launch_int8_rows(static_cast<const __nv_bfloat16*>(x), rows, K, ldx, q, scale, st);
+    case I4TC_FP16: return launch_int8_rows(static_cast<const __half*>(x), rows, K, ldx, q, scale, st);
     case I4TC_FP32:
       quant_int8_rowwise_kernel<float><<<(unsigned)rows, 256, 0, st>>>(static_cast<const float*>(x), (int)K, ldx, q, scale);
       break;
