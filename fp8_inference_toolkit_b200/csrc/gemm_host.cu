@@ -35,8 +35,11 @@ struct Shape {
 // weights); otherwise the candidate with the fewest cost-weighted waves wins.  Weights = measured time per output
 // column relative to 256-wide pair tiles at M = 8192 (per-group | per-channel epilogue): 192-wide pair tiles 1.10 | 1.30,
 // 256-wide single tiles 1.05 | 1.20, 128-wide single tiles 1.25 | 1.45.
+// int8 operands (i8_groups = their K groups, else 0): 192-wide pair tiles 1.10, 256-wide single 1.20, 128-wide single 1.60, pairs from 129
+// rows on, and 1.5 us more for a launch of pairs at 1.3 ns per column and group; over 110 sizes the choice costs 0.7 % against the
+// fastest of the four, with the per-channel weights it was 3.6 %.
 static Shape choose_shape(long long M, long long N, int sms, bool allow_swap, bool group_mode, bool pairs_allowed,
-                          double* cost_out = nullptr) {
+                          double* cost_out = nullptr, int i8_groups = 0) {
   Shape s;
   s.pair = false;
   s.swap = allow_swap && M <= 64;
@@ -65,18 +68,20 @@ static Shape choose_shape(long long M, long long N, int sms, bool allow_swap, bo
     s.bn = N >= 16384 ? 256 : 128;
     return s;
   }
-  struct Cand { int bn; bool pair; double w_group, w_channel; };
-  const Cand cands[4] = {{256, true, 1.00, 1.00}, {192, true, 1.10, 1.30}, {256, false, 1.05, 1.20}, {128, false, 1.25, 1.45}};
+  struct Cand { int bn; bool pair; double w_group, w_channel, w_i8; };
+  const Cand cands[4] = {{256, true, 1.00, 1.00, 1.00}, {192, true, 1.10, 1.30, 1.10}, {256, false, 1.05, 1.20, 1.20},
+                         {128, false, 1.25, 1.45, 1.60}};
   double best = 1e30;
   s.bn = 256;
   for (const Cand& c : cands) {
-    if (c.pair && (!pairs_allowed || M < 512 || sms < 2 || force_pairs == 0)) continue;
+    if (c.pair && (!pairs_allowed || (M < 512 && i8_groups == 0) || sms < 2 || force_pairs == 0)) continue;
     if (!c.pair && force_pairs == 1 && pairs_allowed) continue;
     const long long rows = c.pair ? (M + 255) / 256 : (M + 127) / 128;
     const long long units = c.pair ? sms / 2 : sms;
     const long long tiles = rows * ((N + c.bn - 1) / c.bn);
     const long long waves = (tiles + units - 1) / units;
-    const double cost = (double)waves * c.bn * (group_mode ? c.w_group : c.w_channel);
+    double cost = (double)waves * c.bn * (i8_groups ? c.w_i8 : group_mode ? c.w_group : c.w_channel);
+    if (i8_groups && c.pair) cost += 1.5 / (0.0013 * i8_groups);
     if (cost < best) {
       best = cost;
       s.bn = c.bn;
@@ -188,7 +193,7 @@ static int run_dense(const DenseArgs& d, int device, void* stream) {
 
   const bool group_mode = d.epi_mode == EPI_GROUP || d.epi_mode == EPI_GROUP_INT32;
   const bool pairs_allowed = (d.epi_mode == EPI_CHANNEL || d.epi_mode == EPI_GROUP) && info->pairs.load();
-  Shape sh = choose_shape(d.M, d.N, info->sm_count, true, group_mode, pairs_allowed);
+  Shape sh = choose_shape(d.M, d.N, info->sm_count, true, group_mode, pairs_allowed, nullptr, d.i8_operands ? d.G : 0);
   I4TC_REQUIRE(sh.bn != 192 || sh.pair, I4TC_EINVAL, "192-wide tiles need a dense problem with scaled outputs (SM pairs)");
   GemmParams p;
   memset(&p, 0, sizeof(p));

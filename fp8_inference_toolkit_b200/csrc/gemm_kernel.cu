@@ -75,6 +75,12 @@ struct Cfg {
   static constexpr int PK_Q = QR * kPackedRow;
   static constexpr int I8_P = kBM * kI8Row;                            // 16 KB
   static constexpr int I8_Q = QR * kI8Row;
+  // int8 operands need no packed stages: their ring takes that room too (4 to 7 stages instead of 2 to 4).  A tile's K loop was
+  // the latency of the copies over the depth of the ring: [512, 12288] x [4096, 12288] 41.7 -> 35.0 us at 128 columns, 84 -> 48 at 256;
+  // [1000, 4096] x [6144, 4096] on pairs of 192 31.5 -> 25.3; [8192, 4096] x [6144, 4096] 138 -> 126.  (Committing
+  // every second group instead, in a ring of four, 41.7 -> 50.9: the stages come back two at a time.)
+  static constexpr int NI8 = (NI * (I8_P + I8_Q) + NP * (PK_P + PK_Q)) / (I8_P + I8_Q);
+  static constexpr int NPB = NP > NI8 ? NP : NI8;                      // "tile landed" barriers
   static constexpr int COLS_PER_WARP = BN / (EW / 4);                  // epilogue columns per warp
   static constexpr int TMEM_COLS = (NT * BN > 256) ? 512 : 256;        // allocation: a power of two >= 32
   // shared memory layout (offsets from a 1024-byte aligned base)
@@ -86,7 +92,7 @@ struct Cfg {
   static constexpr int SCALE_STAGE = (kBM + BN) * 4;                  // bytes
   static constexpr int SQ_BYTES = (kNS * SCALE_STAGE > EW * COLS_PER_WARP * 4) ? kNS * SCALE_STAGE : EW * COLS_PER_WARP * 4;
   static constexpr int OFF_BAR = OFF_SQ + SQ_BYTES;
-  static constexpr int NUM_BARS = 2 * NP + 2 * NI + 2 * NT + 3 * kNS;
+  static constexpr int NUM_BARS = NPB + NP + 2 * NI8 + 2 * NT + 3 * kNS;
   static constexpr int OFF_MISC = OFF_BAR + NUM_BARS * 8;              // tmem ptr, abort flag
   static constexpr int SMEM_BYTES = OFF_MISC + 16 + 1024;              // + alignment slack
 };
@@ -581,10 +587,10 @@ w4a4_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ C
 
   const uint32_t bar0 = sbase + C::OFF_BAR;
   const uint32_t bar_pk_full = bar0;
-  const uint32_t bar_pk_empty = bar_pk_full + C::NP * 8;
+  const uint32_t bar_pk_empty = bar_pk_full + C::NPB * 8;
   const uint32_t bar_i8_full = bar_pk_empty + C::NP * 8;
-  const uint32_t bar_i8_empty = bar_i8_full + C::NI * 8;
-  const uint32_t bar_tm_full = bar_i8_empty + C::NI * 8;
+  const uint32_t bar_i8_empty = bar_i8_full + C::NI8 * 8;
+  const uint32_t bar_tm_full = bar_i8_empty + C::NI8 * 8;
   const uint32_t bar_tm_empty = bar_tm_full + C::NT * 8;
   const uint32_t bar_sc_full = bar_tm_empty + C::NT * 8;
   const uint32_t bar_sc_empty = bar_sc_full + kNS * 8;
@@ -596,8 +602,9 @@ w4a4_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ C
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + C::OFF_MISC + 8);
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < C::NP; ++i) { mbar_init(bar_pk_full + i * 8, 1); mbar_init(bar_pk_empty + i * 8, kConvWarps); }
-    for (int i = 0; i < C::NI; ++i) { mbar_init(bar_i8_full + i * 8, kConvWarps * CG); mbar_init(bar_i8_empty + i * 8, 1); }
+    for (int i = 0; i < C::NPB; ++i) mbar_init(bar_pk_full + i * 8, 1);
+    for (int i = 0; i < C::NP; ++i) mbar_init(bar_pk_empty + i * 8, kConvWarps);
+    for (int i = 0; i < C::NI8; ++i) { mbar_init(bar_i8_full + i * 8, kConvWarps * CG); mbar_init(bar_i8_empty + i * 8, 1); }
     for (int i = 0; i < C::NT; ++i) { mbar_init(bar_tm_full + i * 8, 1); mbar_init(bar_tm_empty + i * 8, EW * CG); }
     for (int i = 0; i < kNS; ++i) {
       mbar_init(bar_sc_full + i * 8, 32); mbar_init(bar_sc_empty + i * 8, EW); mbar_init(bar_sc_peer + i * 8, 1);
@@ -635,7 +642,7 @@ w4a4_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ C
       // free again when the MMAs that read it have completed
       while (ok && sched.template next<BN>(p, ti)) {
         for (int g = ti.g0; g < ti.g1; ++g, ++it) {
-          const uint32_t s = it % C::NI, ph = (it / C::NI) & 1u;
+          const uint32_t s = it % C::NI8, ph = (it / C::NI8) & 1u;
           ok = wait_bar(bar_i8_empty + s * 8, ph ^ 1u, abort_flag);
           if (!ok) break;
           if (lane == 0) {
@@ -672,7 +679,7 @@ w4a4_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ C
     }
     if (!ok) {
       // aborting: wait (bounded) for copies that may still be in flight into this CTA's shared memory
-      const uint32_t depth = p.i8_operands ? (uint32_t)C::NI : (uint32_t)C::NP;
+      const uint32_t depth = p.i8_operands ? (uint32_t)C::NI8 : (uint32_t)C::NP;
       const uint32_t n = it < depth ? it : depth;
       for (uint32_t j = it - n; j < it; ++j) {
         const uint64_t t0 = globaltimer_ns();
@@ -692,14 +699,14 @@ w4a4_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ C
     const uint32_t sc_ring = (p.zp != nullptr) ? kNS / 2 : kNS;   // scale stages in the ring (see epilogue_group)
     SchedT<CG> sched;
     TileInfo ti;
-    uint32_t it = 0, flush = 0;
+    const uint32_t ring = p.i8_operands ? (uint32_t)C::NI8 : (uint32_t)C::NI;
+    uint32_t s = 0, ph = 0, flush = 0;   // stage of the group and its phase
     bool ok = true;
     while (ok && sched.template next<BN>(p, ti)) {
-      for (int g = ti.g0; g < ti.g1; ++g, ++it) {
+      for (int g = ti.g0; g < ti.g1; ++g) {
         const bool first = per_group_flush || g == ti.g0;
         const bool last = per_group_flush || g == ti.g1 - 1;
         const uint32_t buf = flush % C::NT;
-        const uint32_t s = it % C::NI, ph = (it / C::NI) & 1u;
         const uint32_t b_tm = bar_tm_empty + buf * 8, p_tm = ((flush / C::NT) & 1u) ^ 1u;
         // Per-group scales: this thread also waits for the group's scale stage (in a CTA pair: both CTAs' stages), so
         // that "group done" vouches for the scales and the epilogue warps -- the busy ones in that mode -- wait once.
@@ -750,6 +757,7 @@ w4a4_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ C
           }
         }
         if (last) ++flush;
+        if (++s == ring) { s = 0; ph ^= 1u; }
       }
     }
     } else if (!leader && CG == 2 && p.epi_mode == EPI_GROUP) {
@@ -823,7 +831,7 @@ w4a4_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ C
       // nothing to convert: these warps only pass "tile landed" on to the MMA thread (in a CTA pair: the leader's)
       while (ok && sched.template next<BN>(p, ti)) {
         for (int g = ti.g0; g < ti.g1; ++g, ++it) {
-          const uint32_t si = it % C::NI, phi = (it / C::NI) & 1u;
+          const uint32_t si = it % C::NI8, phi = (it / C::NI8) & 1u;
           ok = wait_bar(bar_pk_full + si * 8, phi, abort_flag);
           if (!ok) break;
           if (lane == 0) arrive_bar<CG>(arr_i8_full + si * 8);
