@@ -86,6 +86,42 @@ bool grouped_ext_fast_ok(const void* x, int64_t ldx, const void* smooth, const u
 int launch_grouped_ext(bool asym, const void* x, int dtype, int64_t rows, int64_t K, int64_t ldx, int gs, float clip,
                        const void* smooth, uint8_t* packed, float* scale, float* azp_adj, cudaStream_t st);
 
+// ---- overlap of a kernel's start with the end of the one before it (programmatic dependent launch) --------------
+// A kernel launched with `overlap` may start while its predecessor in the stream still runs, once every block of that has called
+// pdl_trigger() or ended; pdl_wait() returns when the predecessor has completed and its writes are visible (at once in a
+// kernel that was launched without).  Rules here: only i4tc_linear overlaps, and only behind a quantiser that it launched
+// itself without -- so everything earlier in the stream, the weights among it, is complete; every thread waits before it reads what the
+// predecessor wrote and before it writes what anybody else reads; every block waits before it ends; and a kernel in the middle of a
+// chain triggers after its own wait, so that whatever starts next finds everything but this kernel's results complete.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The wait with the pointers passed through it, so that no load from them can be placed before.
+template <typename T>
+__device__ __forceinline__ const T* pdl_wait(const T* p) {
+  asm volatile("griddepcontrol.wait;" : "+l"(p)::"memory");
+  return p;
+}
+
+__device__ __forceinline__ void pdl_wait(const uint8_t*& a, const float*& b) {
+  asm volatile("griddepcontrol.wait;" : "+l"(a), "+l"(b)::"memory");
+}
+
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_kernel(bool overlap, void (*kernel)(KArgs...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
+                                 const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
 // ---- device helpers ------------------------------------------------------------
 __device__ __forceinline__ float to_f32(__nv_bfloat16 v) { return __bfloat162float(v); }
 __device__ __forceinline__ float to_f32(__half v) { return __half2float(v); }

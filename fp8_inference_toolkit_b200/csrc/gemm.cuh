@@ -58,13 +58,14 @@ struct GemmParams {
   int groups_per_split;
   float* split_ws;
   long long ws_stride;
+  int overlap;   // host: launch so that the kernel may start before its predecessor, the quantiser, has ended
 };
 
 // out[i] = bf16(sum_s ws[s * stride + i]), s ascending.
-int launch_split_reduce(const float* ws, long long stride, int splits, long long n, void* out, cudaStream_t st);
+int launch_split_reduce(const float* ws, long long stride, int splits, long long n, void* out, bool overlap, cudaStream_t st);
 // out[m, n] = cast((sum_s ws[s * stride + m * N + n] * sb[n]) * sa[m]): the ranges hold exact integer sums.
 int launch_split_reduce_scaled(const float* ws, long long stride, int splits, long long M, long long N, const float* sa,
-                               const float* sb, void* out, int out_dtype, cudaStream_t st);
+                               const float* sb, void* out, int out_dtype, bool overlap, cudaStream_t st);
 
 // What became of a launch of CTA pairs (clusters of two) that did not succeed.
 struct PairLaunch {
@@ -97,14 +98,14 @@ int launch_w4a4_group_f8(const GemmParams& p, const uint8_t* a, const uint8_t* b
 // x / w are the packed operands in either layout (rowmajor: [rows, G * 64]; else [G, rows, 64]).
 bool gemv_applicable(long long M, long long N, long long K, int epi_mode);
 int launch_w4a4_gemv(const uint8_t* x, const uint8_t* w, const float* sx, const float* sw, void* out, int out_dtype,
-                     long long M, long long N, int G, bool rowmajor, int epi_mode, int sm_count, cudaStream_t st);
+                     long long M, long long N, int G, bool rowmajor, int epi_mode, int sm_count, bool overlap, cudaStream_t st);
 
 // Register-fed tensor-core weight-streaming kernel for M <= 32 tokens (same operands and outputs as the kernel above;
 // `status` is the device status word that a bounded wait flags).
 bool skinny_applicable(long long M, long long N, long long K, int epi_mode, bool rowmajor, int sm_count);
 int launch_w4a4_skinny(const uint8_t* x, const uint8_t* w, const float* sx, const float* sw, void* out, int out_dtype,
                        long long M, long long N, int G, bool rowmajor, int epi_mode, int sm_count, unsigned int* status,
-                       cudaStream_t st);
+                       bool overlap, cudaStream_t st);
 
 // Weight-streaming form of the grouped MoE GEMM for few rows per expert (moe_skinny.cu): the same results bit for bit.
 bool moe_skinny_applicable(long long num_pairs, long long N, int G, long long num_experts);

@@ -90,6 +90,7 @@ w4a4_group_f8_kernel(const __grid_constant__ GemmParams p, const __grid_constant
     prefetch_tensormap(&tmQ);
   }
   if (warp == 1) { tmem_alloc_cg2(smem_u32(tmem_slot), 512); tmem_relinquish_cg2(); }
+  pdl_wait();   // the expanded operands, the scales and the output
   tc_fence_before_sync();
   cluster_sync();   // the peer's barriers are initialised before anything arrives on them
   tc_fence_after_sync();
@@ -337,27 +338,33 @@ __device__ __forceinline__ void expand_word(uint32_t w, uint32_t& lo, uint32_t& 
   hi = codes_to_e4m3(m >> 16, nhi);
 }
 
+// Chunk c (16 packed bytes) of a packed [G, rows, 64 B] operand -> 32 bytes of its e4m3 form [G, pitch, 128 B].
+__device__ __forceinline__ void expand_chunk(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, long long c, int rows, int pitch,
+                                             bool permute) {
+  const long long slot = c >> 2;
+  const int g = (int)(slot / pitch), r = (int)(slot - (long long)g * pitch), j = (int)c & 3;
+  uint4 w = make_uint4(0, 0, 0, 0);
+  if (r < rows) w = __ldg(reinterpret_cast<const uint4*>(src + ((long long)g * rows + r) * 64 + j * 16));
+  uint4 x, y;
+  expand_word(w.x, x.x, x.y); expand_word(w.y, x.z, x.w);
+  expand_word(w.z, y.x, y.y); expand_word(w.w, y.z, y.w);
+  uint4* at = reinterpret_cast<uint4*>(dst + ((long long)g * pitch + (permute ? qperm(r) : r)) * 128 + j * 32);
+  at[0] = x;
+  at[1] = y;
+}
+
 // Packed [G, rows, 64 B] of both operands -> e4m3 [G, pitch, 128 B], pitch = rows rounded up to 32 (Q rows of a 32-row
 // block in the order qperm; the rows that fill up a block are zero).  A thread expands 16 packed bytes.
 __global__ void __launch_bounds__(256) expand_e4m3_kernel(const uint8_t* __restrict__ a, const uint8_t* __restrict__ b,
                                                           int M, int m_pitch, int N, int n_pitch, int G,
                                                           uint8_t* __restrict__ ea, uint8_t* __restrict__ eb) {
-  const long long ca = (long long)G * m_pitch * 4, cb = (long long)G * n_pitch * 4;
-  for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < ca + cb; i += (long long)gridDim.x * 256) {
-    const bool second = i >= ca;
-    const long long c = second ? i - ca : i;
-    const int pitch = second ? n_pitch : m_pitch, rows = second ? N : M;
-    const long long slot = c >> 2;
-    const int g = (int)(slot / pitch), r = (int)(slot - (long long)g * pitch), j = (int)c & 3;
-    uint4 w = make_uint4(0, 0, 0, 0);
-    if (r < rows) w = __ldg(reinterpret_cast<const uint4*>((second ? b : a) + ((long long)g * rows + r) * 64 + j * 16));
-    uint4 x, y;
-    expand_word(w.x, x.x, x.y); expand_word(w.y, x.z, x.w);
-    expand_word(w.z, y.x, y.y); expand_word(w.w, y.z, y.w);
-    uint4* dst = reinterpret_cast<uint4*>((second ? eb : ea) + ((long long)g * pitch + (second ? qperm(r) : r)) * 128 + j * 32);
-    dst[0] = x;
-    dst[1] = y;
-  }
+  // the weights first: they are there while the quantiser still works on the activations
+  const long long ca = (long long)G * m_pitch * 4, cb = (long long)G * n_pitch * 4, step = (long long)gridDim.x * 256;
+  long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  for (; i < cb; i += step) expand_chunk(b, eb, i, N, n_pitch, true);
+  a = pdl_wait(a);
+  pdl_trigger();
+  for (; i < ca + cb; i += step) expand_chunk(a, ea, i - cb, M, m_pitch, false);
 }
 
 template <int BN, bool AZP>
@@ -371,13 +378,15 @@ static int launch_f8(const GemmParams& p, const CUtensorMap& tmP, const CUtensor
   cfg.blockDim = dim3(C::THREADS, 1, 1);
   cfg.dynamicSmemBytes = C::SMEM_BYTES;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = p.overlap ? 2 : 1;
   return launch_pairs(cfg, pl, w4a4_group_f8_kernel<BN, AZP>, p, tmP, tmQ, p_pitch, q_pitch);
 }
 
@@ -396,8 +405,8 @@ int launch_w4a4_group_f8(const GemmParams& p, const uint8_t* a, const uint8_t* b
   if (int rc = get_tensor_map_i8(device, eb, (long long)n_pitch * p.G, 128, bn / 2, &tmQ)) return rc;
   const long long chunks = (long long)(m_pitch + n_pitch) * p.G * 4;
   const long long blocks = (chunks + 255) / 256, cap = (long long)sm_count * 8 * 4;
-  expand_e4m3_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(a, b, M, m_pitch, N, n_pitch, p.G, ea, eb);
-  I4TC_CUDA(cudaGetLastError());
+  I4TC_CUDA(launch_kernel(p.overlap != 0, expand_e4m3_kernel, dim3((unsigned)(blocks < cap ? blocks : cap)), 256, 0, st, a, b, M, m_pitch,
+                          N, n_pitch, p.G, ea, eb));
   const long long tiles = (long long)p.num_p_tiles * p.num_q_tiles;
   const int grid = 2 * (int)(tiles < sm_count / 2 ? tiles : sm_count / 2);
   const bool azp = p.zp != nullptr;

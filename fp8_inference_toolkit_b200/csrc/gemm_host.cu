@@ -140,6 +140,7 @@ struct DenseArgs {
   const float* w_col_sum = nullptr;
   uint8_t* scratch = nullptr;   // room for the expanded operands (per-group mode)
   long long scratch_bytes = 0;
+  bool overlap = false;       // a and its scales come from a quantiser launched just before: start under its end (see pdl_wait)
   bool i8_operands = false;   // a and b are int8 [rows, K] (W4A8): no conversion, accumulator unit 1
 };
 
@@ -162,10 +163,10 @@ static int run_dense(const DenseArgs& d, int device, void* stream) {
     // one or two tokens: dp4a on the CUDA cores does not waste tensor-core columns; from three on the tensor cores win
     if (skinny_ok && (path == 2 || !gemv_ok || d.M > 2))
       return launch_w4a4_skinny(d.a, d.b, d.sa, d.sb, d.out, d.out_dtype, d.M, d.N, d.G, d.rowmajor, d.epi_mode,
-                                info->sm_count, info->status, static_cast<cudaStream_t>(stream));
+                                info->sm_count, info->status, d.overlap, static_cast<cudaStream_t>(stream));
     if (gemv_ok)
       return launch_w4a4_gemv(d.a, d.b, d.sa, d.sb, d.out, d.out_dtype, d.M, d.N, d.G, d.rowmajor, d.epi_mode,
-                              info->sm_count, static_cast<cudaStream_t>(stream));
+                              info->sm_count, d.overlap, static_cast<cudaStream_t>(stream));
   }
 
   if (d.scratch != nullptr && d.epi_mode == EPI_GROUP) {
@@ -183,6 +184,7 @@ static int run_dense(const DenseArgs& d, int device, void* stream) {
       p.num_q_tiles = (int)((d.N + bn - 1) / bn);
       p.splits = 1; p.groups_per_split = d.G;
       p.status = info->status;
+      p.overlap = d.overlap;
       PairLaunch pl;
       const int rc = launch_w4a4_group_f8(p, d.a, d.b, d.scratch, bn, device, info->sm_count, static_cast<cudaStream_t>(stream), &pl);
       if (!pl.failed) return rc;
@@ -207,6 +209,7 @@ static int run_dense(const DenseArgs& d, int device, void* stream) {
   p.ldc = d.N;
   p.out_gstride = d.M * d.N;
   p.status = info->status;
+  p.overlap = d.overlap;
   p.p_rowmajor = p.q_rowmajor = d.rowmajor ? 1 : 0;
   const bool per_group_scales = d.epi_mode == EPI_GROUP;
   const uint8_t *pbase, *qbase;
@@ -295,9 +298,9 @@ static int run_dense(const DenseArgs& d, int device, void* stream) {
   if (int rc = launch_w4a4_gemm(p, tmP, tmQ, sh.bn, grid, false, epi_warps_for(d.epi_mode), static_cast<cudaStream_t>(stream))) return rc;
   if (p.splits > 1) {
     if (d.epi_mode == EPI_CHANNEL)
-      return launch_split_reduce_scaled(p.split_ws, p.ws_stride, p.splits, d.M, d.N, d.sa, d.sb, d.out, d.out_dtype,
+      return launch_split_reduce_scaled(p.split_ws, p.ws_stride, p.splits, d.M, d.N, d.sa, d.sb, d.out, d.out_dtype, d.overlap,
                                         static_cast<cudaStream_t>(stream));
-    return launch_split_reduce(p.split_ws, p.ws_stride, p.splits, d.M * d.N, d.out, static_cast<cudaStream_t>(stream));
+    return launch_split_reduce(p.split_ws, p.ws_stride, p.splits, d.M * d.N, d.out, d.overlap, static_cast<cudaStream_t>(stream));
   }
   return I4TC_OK;
 }
@@ -356,9 +359,8 @@ extern "C" int i4tc_gemm_int32(const uint8_t* a, const uint8_t* b, int32_t* c, i
   return run_dense(d, device, stream);
 }
 
-extern "C" int i4tc_gemm_scaled(const uint8_t* a, const uint8_t* b, const float* scale_a, const float* scale_b,
-                                void* out, int out_dtype, int64_t M, int64_t N, int64_t K, int device,
-                                void* stream) {
+static int gemm_scaled_impl(const uint8_t* a, const uint8_t* b, const float* scale_a, const float* scale_b, void* out,
+                            int out_dtype, int64_t M, int64_t N, int64_t K, bool overlap, int device, void* stream) {
   I4TC_REQUIRE(K > 0 && K % 64 == 0, I4TC_EINVAL, "K must be a positive multiple of 64");
   I4TC_REQUIRE(K <= 65536, I4TC_EINVAL, "K must not exceed 65536");
   I4TC_REQUIRE(out_dtype == I4TC_BF16 || out_dtype == I4TC_FP16, I4TC_EUNSUPPORTED, "out must be bf16 or fp16");
@@ -366,7 +368,14 @@ extern "C" int i4tc_gemm_scaled(const uint8_t* a, const uint8_t* b, const float*
   if (rc) return rc < 0 ? rc : I4TC_OK;
   I4TC_REQUIRE(scale_a && scale_b, I4TC_EINVAL, "null scale pointer");
   DenseArgs d{a, b, scale_a, scale_b, out, out_dtype, M, N, (int)((K + 127) / 128), true, K, EPI_CHANNEL};
+  d.overlap = overlap;
   return run_dense(d, device, stream);
+}
+
+extern "C" int i4tc_gemm_scaled(const uint8_t* a, const uint8_t* b, const float* scale_a, const float* scale_b,
+                                void* out, int out_dtype, int64_t M, int64_t N, int64_t K, int device,
+                                void* stream) {
+  return gemm_scaled_impl(a, b, scale_a, scale_b, out, out_dtype, M, N, K, false, device, stream);
 }
 
 extern "C" int i4tc_gemm_w4a8_scaled(const int8_t* a, const int8_t* b, const float* scale_a, const float* scale_b,
@@ -422,10 +431,10 @@ extern "C" int64_t i4tc_gemm_grouped_scratch_bytes(int64_t M, int64_t N, int64_t
   return i4tc_gemm_grouped_expanded_width(M, N, num_groups, azp, device) != 0 ? group_f8_scratch_bytes(M, N, (int)num_groups) : 0;
 }
 
-extern "C" int i4tc_gemm_grouped_scratch(const uint8_t* a, const uint8_t* b, const float* scale_a, const float* scale_b,
-                                         const float* azp_adj, const float* w_col_sum, void* out, int64_t M, int64_t N,
-                                         int64_t group_size, int64_t num_groups, void* scratch, int64_t scratch_bytes,
-                                         int device, void* stream) {
+static int gemm_grouped_scratch_impl(const uint8_t* a, const uint8_t* b, const float* scale_a, const float* scale_b,
+                                     const float* azp_adj, const float* w_col_sum, void* out, int64_t M, int64_t N,
+                                     int64_t group_size, int64_t num_groups, void* scratch, int64_t scratch_bytes,
+                                     bool overlap, int device, void* stream) {
   I4TC_REQUIRE(group_size == 128, I4TC_EUNSUPPORTED, "fused grouped GEMM only supports group_size=128");
   I4TC_REQUIRE(num_groups > 0 && num_groups <= 512, I4TC_EINVAL, "num_groups must be in [1, 512]");
   int rc = check_dense_common(a, b, out, M, N);
@@ -437,7 +446,16 @@ extern "C" int i4tc_gemm_grouped_scratch(const uint8_t* a, const uint8_t* b, con
   d.w_col_sum = w_col_sum;
   d.scratch = static_cast<uint8_t*>(scratch);
   d.scratch_bytes = scratch != nullptr ? scratch_bytes : 0;
+  d.overlap = overlap;
   return run_dense(d, device, stream);
+}
+
+extern "C" int i4tc_gemm_grouped_scratch(const uint8_t* a, const uint8_t* b, const float* scale_a, const float* scale_b,
+                                         const float* azp_adj, const float* w_col_sum, void* out, int64_t M, int64_t N,
+                                         int64_t group_size, int64_t num_groups, void* scratch, int64_t scratch_bytes,
+                                         int device, void* stream) {
+  return gemm_grouped_scratch_impl(a, b, scale_a, scale_b, azp_adj, w_col_sum, out, M, N, group_size, num_groups, scratch,
+                                   scratch_bytes, false, device, stream);
 }
 
 extern "C" int i4tc_linear(const void* x, int dtype, int64_t M, int64_t K, int64_t ldx, const uint8_t* w, const float* w_scale,
@@ -445,11 +463,11 @@ extern "C" int i4tc_linear(const void* x, int dtype, int64_t M, int64_t K, int64
                            int64_t scratch_bytes, int device, void* stream) {
   if (per_channel) {
     if (int rc = i4tc_quant_rowwise(x, dtype, M, K, ldx, x_packed, x_scale, I4TC_ROLE_ACTIVATION, device, stream)) return rc;
-    return i4tc_gemm_scaled(x_packed, w, x_scale, w_scale, out, I4TC_BF16, M, N, K, device, stream);
+    return gemm_scaled_impl(x_packed, w, x_scale, w_scale, out, I4TC_BF16, M, N, K, true, device, stream);
   }
   if (int rc = i4tc_quant_grouped(x, dtype, M, K, ldx, 128, x_packed, x_scale, I4TC_ROLE_ACTIVATION, device, stream)) return rc;
-  return i4tc_gemm_grouped_scratch(x_packed, w, x_scale, w_scale, nullptr, nullptr, out, M, N, 128, K / 128, scratch,
-                                   scratch_bytes, device, stream);
+  return gemm_grouped_scratch_impl(x_packed, w, x_scale, w_scale, nullptr, nullptr, out, M, N, 128, K / 128, scratch,
+                                   scratch_bytes, true, device, stream);
 }
 
 extern "C" int i4tc_gemm_grouped_int32(const uint8_t* a, const uint8_t* b, int32_t* out, int64_t M, int64_t N,

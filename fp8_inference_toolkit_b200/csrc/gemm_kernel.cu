@@ -618,6 +618,8 @@ w4a4_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ C
     if (CG == 2) { tmem_alloc_cg2(smem_u32(tmem_slot), C::TMEM_COLS); tmem_relinquish_cg2(); }
     else { tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS); tmem_relinquish(); }
   }
+  pdl_wait();   // nothing of the operands, the scales or the output is touched before
+  pdl_trigger();
   tc_fence_before_sync();
   if (CG == 2) cluster_sync();   // the peer's barriers are initialised before anything arrives on them
   else __syncthreads();
@@ -920,20 +922,22 @@ static int launch_bn(const GemmParams& p, const CUtensorMap& tmP, const CUtensor
     configured[dev] = true;
   }
   if (CG == 1) {
-    w4a4_gemm_kernel<BN, CG, EW><<<grid, C::THREADS, C::SMEM_BYTES, st>>>(p, tmP, tmQ);
+    I4TC_CUDA(launch_kernel(p.overlap != 0, w4a4_gemm_kernel<BN, CG, EW>, dim3((unsigned)grid), C::THREADS, C::SMEM_BYTES, st, p, tmP, tmQ));
   } else {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid, 1, 1);
     cfg.blockDim = dim3(C::THREADS, 1, 1);
     cfg.dynamicSmemBytes = C::SMEM_BYTES;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = CG;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = p.overlap ? 2 : 1;
     return launch_pairs(cfg, pl, w4a4_gemm_kernel<BN, CG, EW>, p, tmP, tmQ);
   }
   I4TC_CUDA(cudaGetLastError());
@@ -942,6 +946,7 @@ static int launch_bn(const GemmParams& p, const CUtensorMap& tmP, const CUtensor
 
 __global__ void __launch_bounds__(256) split_reduce_kernel(const float* __restrict__ ws, long long stride, int splits,
                                                           long long n, __nv_bfloat16* __restrict__ out) {
+  ws = pdl_wait(ws);
   const long long i = ((long long)blockIdx.x * 256 + threadIdx.x) * 4;
   // 16-byte loads need every range to start on a 16-byte boundary, the 8-byte store an 8-byte aligned output
   const bool vec = ((stride & 3) == 0) && ((reinterpret_cast<uintptr_t>(ws) & 15) == 0) &&
@@ -970,6 +975,7 @@ template <typename OutT>
 __global__ void __launch_bounds__(256) split_reduce_scaled_kernel(const float* __restrict__ ws, long long stride, int splits,
                                                                  long long M, long long N, const float* __restrict__ sa,
                                                                  const float* __restrict__ sb, OutT* __restrict__ out) {
+  ws = pdl_wait(ws);   // (the scales are older than the sums)
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i >= M * N) return;
   float acc = ws[i];
@@ -979,21 +985,20 @@ __global__ void __launch_bounds__(256) split_reduce_scaled_kernel(const float* _
 }
 
 int launch_split_reduce_scaled(const float* ws, long long stride, int splits, long long M, long long N, const float* sa,
-                               const float* sb, void* out, int out_dtype, cudaStream_t st) {
-  const long long blocks = (M * N + 255) / 256;
+                               const float* sb, void* out, int out_dtype, bool overlap, cudaStream_t st) {
+  const dim3 blocks((unsigned)((M * N + 255) / 256));
   if (out_dtype == I4TC_FP16)
-    split_reduce_scaled_kernel<__half><<<(unsigned)blocks, 256, 0, st>>>(ws, stride, splits, M, N, sa, sb, static_cast<__half*>(out));
+    I4TC_CUDA(launch_kernel(overlap, split_reduce_scaled_kernel<__half>, blocks, 256, 0, st, ws, stride, splits, M, N, sa, sb,
+                            static_cast<__half*>(out)));
   else
-    split_reduce_scaled_kernel<__nv_bfloat16><<<(unsigned)blocks, 256, 0, st>>>(ws, stride, splits, M, N, sa, sb,
-                                                                                static_cast<__nv_bfloat16*>(out));
-  I4TC_CUDA(cudaGetLastError());
+    I4TC_CUDA(launch_kernel(overlap, split_reduce_scaled_kernel<__nv_bfloat16>, blocks, 256, 0, st, ws, stride, splits, M, N, sa, sb,
+                            static_cast<__nv_bfloat16*>(out)));
   return I4TC_OK;
 }
 
-int launch_split_reduce(const float* ws, long long stride, int splits, long long n, void* out, cudaStream_t st) {
-  const long long blocks = (n + 1023) / 1024;
-  split_reduce_kernel<<<(unsigned)blocks, 256, 0, st>>>(ws, stride, splits, n, static_cast<__nv_bfloat16*>(out));
-  I4TC_CUDA(cudaGetLastError());
+int launch_split_reduce(const float* ws, long long stride, int splits, long long n, void* out, bool overlap, cudaStream_t st) {
+  I4TC_CUDA(launch_kernel(overlap, split_reduce_kernel, dim3((unsigned)((n + 1023) / 1024)), 256, 0, st, ws, stride, splits, n,
+                          static_cast<__nv_bfloat16*>(out)));
   return I4TC_OK;
 }
 

@@ -62,11 +62,14 @@ __global__ void __launch_bounds__(512) w4a4_gemv_kernel(const GemvParams p) {
     for (int j = 0; j < 4; ++j) wv[j] = __ldg(src + j);
   }
 
+  const uint8_t* x = p.x;
+  const float* sx = p.sx;
+  pdl_wait(x, sx);
   // ---- stage the tokens: packed 16-byte chunk -> 16 bytes of even codes, 16 bytes of odd codes ----
   for (int i = threadIdx.x; i < p.G * MT * 4; i += blockDim.x) {
     const int j = i & 3, m = (i >> 2) % MT, g = (i >> 2) / MT;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (m < p.M) v = __ldg(reinterpret_cast<const uint4*>(p.x + (long long)m * p.x_row + (long long)g * p.x_grp) + j);
+    if (m < p.M) v = __ldg(reinterpret_cast<const uint4*>(x + (long long)m * p.x_row + (long long)g * p.x_grp) + j);
     uint32_t lo[4], hi[4];
     expand8(v, lo, hi);
     uint4* dst = reinterpret_cast<uint4*>(act + ((size_t)(g * MT + m) * 128 + j * 32));
@@ -76,7 +79,7 @@ __global__ void __launch_bounds__(512) w4a4_gemv_kernel(const GemvParams p) {
   if (PER_GROUP) {
     for (int i = threadIdx.x; i < p.G * MT; i += blockDim.x) {
       const int m = i % MT, g = i / MT;
-      sx_s[i] = (m < p.M) ? __ldg(p.sx + (long long)g * p.M + m) * (1.0f / 256.0f) : 0.f;
+      sx_s[i] = (m < p.M) ? __ldg(sx + (long long)g * p.M + m) * (1.0f / 256.0f) : 0.f;
     }
   }
   __syncthreads();
@@ -158,7 +161,7 @@ __global__ void __launch_bounds__(512) w4a4_gemv_kernel(const GemvParams p) {
       }
       // reference order: (acc * scale_b[n]) * scale_a[m]
       const float sb = n_ok ? __ldg(p.sw + n) : 0.f;
-      v = (__int2float_rn(s) * (sb * (1.0f / 256.0f))) * __ldg(p.sx + m);
+      v = (__int2float_rn(s) * (sb * (1.0f / 256.0f))) * __ldg(sx + m);
     }
     if (n_ok) {
       if (p.out_fp16) static_cast<__half*>(p.out)[(long long)m * p.N + n] = __float2half_rn(v);
@@ -168,7 +171,7 @@ __global__ void __launch_bounds__(512) w4a4_gemv_kernel(const GemvParams p) {
 }
 
 template <int MT, bool PER_GROUP>
-int launch_mt(const GemvParams& p, int warps, size_t smem, cudaStream_t st) {
+int launch_mt(const GemvParams& p, int warps, size_t smem, bool overlap, cudaStream_t st) {
   static bool configured[64] = {false};
   int dev = 0;
   I4TC_CUDA(cudaGetDevice(&dev));
@@ -177,8 +180,7 @@ int launch_mt(const GemvParams& p, int warps, size_t smem, cudaStream_t st) {
     configured[dev] = true;
   }
   const int grid = (p.N + kRows - 1) / kRows;
-  w4a4_gemv_kernel<MT, PER_GROUP><<<grid, warps * 32, smem, st>>>(p);
-  I4TC_CUDA(cudaGetLastError());
+  I4TC_CUDA(launch_kernel(overlap, w4a4_gemv_kernel<MT, PER_GROUP>, dim3((unsigned)grid), (unsigned)warps * 32, smem, st, p));
   return I4TC_OK;
 }
 
@@ -195,7 +197,7 @@ bool gemv_applicable(long long M, long long N, long long K, int epi_mode) {
 }
 
 int launch_w4a4_gemv(const uint8_t* x, const uint8_t* w, const float* sx, const float* sw, void* out, int out_dtype,
-                     long long M, long long N, int G, bool rowmajor, int epi_mode, int sm_count, cudaStream_t st) {
+                     long long M, long long N, int G, bool rowmajor, int epi_mode, int sm_count, bool overlap, cudaStream_t st) {
   GemvParams p;
   p.x = x; p.w = w; p.sx = sx; p.sw = sw; p.out = out;
   p.M = (int)M; p.N = (int)N; p.G = G;
@@ -216,7 +218,7 @@ int launch_w4a4_gemv(const uint8_t* x, const uint8_t* w, const float* sx, const 
   const size_t smem = (size_t)G * mt * 128 + (pg ? (size_t)G * mt * 4 : 0) + (size_t)warps * mt * kRows * 4;
 #define I4TC_GEMV_CASE(MT_)                                                        \
   case MT_:                                                                        \
-    return pg ? launch_mt<MT_, true>(p, warps, smem, st) : launch_mt<MT_, false>(p, warps, smem, st);
+    return pg ? launch_mt<MT_, true>(p, warps, smem, overlap, st) : launch_mt<MT_, false>(p, warps, smem, overlap, st);
   switch (mt) {
     I4TC_GEMV_CASE(1)
     I4TC_GEMV_CASE(2)

@@ -452,6 +452,7 @@ __global__ void __launch_bounds__(quant_rows<MODE>() * 32, MODE == 3 ? 8 : MODE 
     float* __restrict__ scale, int role, int segs_per_block, const T* __restrict__ aux, float eps,
     QuantOutMap out = QuantOutMap{nullptr, nullptr, 0, 0, 0, 0, nullptr, 1, 0, 0}) {
   constexpr int GS = LPG * kQLane;
+  if (MODE == 0) pdl_trigger();   // (the GEMM behind it may start)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t r = (int64_t)blockIdx.x * quant_rows<MODE>() + warp;
   bool row_ok = r < rows;
@@ -835,6 +836,7 @@ __global__ void __launch_bounds__(256) quant_rowwise_kernel(const T* __restrict_
                                                             uint8_t* __restrict__ packed,
                                                             float* __restrict__ scale, int role) {
   __shared__ float s_max[8];
+  pdl_trigger();
   const int64_t r = blockIdx.x;
   const T* src = x + r * ldx;
   const int t = threadIdx.x;

@@ -140,10 +140,7 @@ __global__ void __launch_bounds__(skinny_warps(MTILES) * 32) w4a4_skinny_kernel(
       mbar_arrive_expect_tx(bar, tx);
       // the block's rows (and all tokens) of one group are contiguous
       bulk_load(dst, p.w + (long long)grp * p.w_grp + (long long)n0 * 64, CHUNK, bar);
-      if (STAGE) {
-        bulk_load(dst + CHUNK, p.x + (long long)grp * p.x_grp, (uint32_t)p.M * 64u, bar);
-        if (PER_GROUP) bulk_load(dst + CHUNK + TOK * 64, p.sw + (long long)grp * p.N + n0, ROWS * 4, bar);
-      }
+      if (STAGE && PER_GROUP) bulk_load(dst + CHUNK + TOK * 64, p.sw + (long long)grp * p.N + n0, ROWS * 4, bar);
     }
   } else if (gw > 0) {
     // everything of this warp on its first barrier: one copy per weight row (and per staged token)
@@ -151,10 +148,16 @@ __global__ void __launch_bounds__(skinny_warps(MTILES) * 32) w4a4_skinny_kernel(
     __syncwarp();
     for (int r = lane; r < ROWS; r += 32)
       bulk_load(smem_u32(wsm) + r * rs, p.w + (long long)(n0 + r) * p.w_row + (long long)g0 * 64, (uint32_t)gw * 64u, bars);
-    if (STAGE) {
-      for (int m = lane; m < p.M; m += 32)
-        bulk_load(smem_u32(wsm) + tok_off + m * rs, p.x + (long long)m * p.x_row + (long long)g0 * 64, (uint32_t)gw * 64u, bars);
-    }
+  }
+  // the weights are on their way; the tokens may still be at the quantiser
+  const uint8_t* x = p.x;
+  const float* sx = p.sx;
+  pdl_wait(x, sx);
+  if (STAGE && !rm) {
+    if (lane < gw) bulk_load(smem_u32(wsm) + lane * ITEM + CHUNK, x + (long long)(g0 + lane) * p.x_grp, (uint32_t)p.M * 64u, bars + lane * 8u);
+  } else if (STAGE && gw > 0) {
+    for (int m = lane; m < p.M; m += 32)
+      bulk_load(smem_u32(wsm) + tok_off + m * rs, x + (long long)m * p.x_row + (long long)g0 * 64, (uint32_t)gw * 64u, bars);
   }
   if (STAGE) {
     // padding tokens: zero codes; token scales with the 2^-8 folded in
@@ -173,7 +176,7 @@ __global__ void __launch_bounds__(skinny_warps(MTILES) * 32) w4a4_skinny_kernel(
     if (PER_GROUP) {
       for (int i = lane; i < gw * TOK; i += 32) {
         const int gi = i / TOK, m = i - gi * TOK;
-        sx_s[i] = m < p.M ? __ldg(p.sx + (long long)(g0 + gi) * p.M + m) * (1.0f / 256.0f) : 0.f;
+        sx_s[i] = m < p.M ? __ldg(sx + (long long)(g0 + gi) * p.M + m) * (1.0f / 256.0f) : 0.f;
       }
     }
     __syncwarp();
@@ -187,11 +190,11 @@ __global__ void __launch_bounds__(skinny_warps(MTILES) * 32) w4a4_skinny_kernel(
     for (int nt = 0; nt < NT; ++nt) {
       const int tok = 8 * nt + g;
       xb[nt] = make_uint4(0u, 0u, 0u, 0u);
-      if (tok < p.M) xb[nt] = __ldg(reinterpret_cast<const uint4*>(p.x + (long long)tok * p.x_row + (long long)grp * p.x_grp) + t);
+      if (tok < p.M) xb[nt] = __ldg(reinterpret_cast<const uint4*>(x + (long long)tok * p.x_row + (long long)grp * p.x_grp) + t);
       if (PER_GROUP) {
         const int t0 = 8 * nt + 2 * t;
-        sxs[nt][0] = t0 < p.M ? __ldg(p.sx + (long long)grp * p.M + t0) * (1.0f / 256.0f) : 0.f;
-        sxs[nt][1] = t0 + 1 < p.M ? __ldg(p.sx + (long long)grp * p.M + t0 + 1) * (1.0f / 256.0f) : 0.f;
+        sxs[nt][0] = t0 < p.M ? __ldg(sx + (long long)grp * p.M + t0) * (1.0f / 256.0f) : 0.f;
+        sxs[nt][1] = t0 + 1 < p.M ? __ldg(sx + (long long)grp * p.M + t0 + 1) * (1.0f / 256.0f) : 0.f;
       }
     }
     if (PER_GROUP) {
@@ -309,7 +312,7 @@ __global__ void __launch_bounds__(skinny_warps(MTILES) * 32) w4a4_skinny_kernel(
 #pragma unroll
       for (int w2 = 1; w2 < nwarps; ++w2) s += (int)red[(size_t)w2 * TOK * ROWS];
       // reference order: (acc * scale_b[n]) * scale_a[m]
-      v = (__int2float_rn(s) * (__ldg(p.sw + n0 + row) * (1.0f / 256.0f))) * __ldg(p.sx + tok);
+      v = (__int2float_rn(s) * (__ldg(p.sw + n0 + row) * (1.0f / 256.0f))) * __ldg(sx + tok);
     }
     const long long idx = (long long)tok * p.N + n0 + row;
     if (p.out_fp16) static_cast<__half*>(p.out)[idx] = __float2half_rn(v);
@@ -329,7 +332,7 @@ size_t skinny_smem(int warps, int rows, int nt, int gper, bool per_group, bool s
 }
 
 template <int MTILES, int NT, bool PER_GROUP, bool STAGE>
-int launch_one(const SkinnyParams& p, size_t smem, cudaStream_t st) {
+int launch_one(const SkinnyParams& p, size_t smem, bool overlap, cudaStream_t st) {
   static bool configured[64] = {false};
   int dev = 0;
   I4TC_CUDA(cudaGetDevice(&dev));
@@ -338,21 +341,21 @@ int launch_one(const SkinnyParams& p, size_t smem, cudaStream_t st) {
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     configured[dev] = true;
   }
-  w4a4_skinny_kernel<MTILES, NT, PER_GROUP, STAGE><<<p.N / (16 * MTILES), skinny_warps(MTILES) * 32, smem, st>>>(p);
-  I4TC_CUDA(cudaGetLastError());
+  I4TC_CUDA(launch_kernel(overlap, w4a4_skinny_kernel<MTILES, NT, PER_GROUP, STAGE>, dim3((unsigned)(p.N / (16 * MTILES))),
+                          (unsigned)skinny_warps(MTILES) * 32, smem, st, p));
   return I4TC_OK;
 }
 
 template <int MTILES, bool PER_GROUP, bool STAGE>
-int launch_nt(const SkinnyParams& p, int nt, size_t smem, cudaStream_t st) {
+int launch_nt(const SkinnyParams& p, int nt, size_t smem, bool overlap, cudaStream_t st) {
   switch (nt) {
-    case 1: return launch_one<MTILES, 1, PER_GROUP, STAGE>(p, smem, st);
-    case 2: return launch_one<MTILES, 2, PER_GROUP, STAGE>(p, smem, st);
+    case 1: return launch_one<MTILES, 1, PER_GROUP, STAGE>(p, smem, overlap, st);
+    case 2: return launch_one<MTILES, 2, PER_GROUP, STAGE>(p, smem, overlap, st);
     default: break;
   }
   if constexpr (MTILES == 1) {   // 32-row tiles exist for up to 16 tokens only
-    if (nt == 3) return launch_one<MTILES, 3, PER_GROUP, STAGE>(p, smem, st);
-    if (nt == 4) return launch_one<MTILES, 4, PER_GROUP, STAGE>(p, smem, st);
+    if (nt == 3) return launch_one<MTILES, 3, PER_GROUP, STAGE>(p, smem, overlap, st);
+    if (nt == 4) return launch_one<MTILES, 4, PER_GROUP, STAGE>(p, smem, overlap, st);
   }
   return fail(I4TC_EINVAL, "unsupported token count");
 }
@@ -405,7 +408,7 @@ bool skinny_applicable(long long M, long long N, long long K, int epi_mode, bool
 
 int launch_w4a4_skinny(const uint8_t* x, const uint8_t* w, const float* sx, const float* sw, void* out, int out_dtype,
                        long long M, long long N, int G, bool rowmajor, int epi_mode, int sm_count, unsigned int* status,
-                       cudaStream_t st) {
+                       bool overlap, cudaStream_t st) {
   SkinnyParams p;
   p.x = x; p.w = w; p.sx = sx; p.sw = sw; p.out = out;
   p.M = (int)M; p.N = (int)N; p.G = G;
@@ -430,7 +433,7 @@ int launch_w4a4_skinny(const uint8_t* x, const uint8_t* w, const float* sx, cons
     pl.smem = skinny_smem(pl.warps, pl.rows, nt, pl.gper, pg, false, rowmajor);
   }
 #define I4TC_SKINNY_CASE(MT_, PG_, ST_) \
-  if (pl.rows == 16 * MT_ && pg == PG_ && pl.stage == ST_) return launch_nt<MT_, PG_, ST_>(p, nt, pl.smem, st);
+  if (pl.rows == 16 * MT_ && pg == PG_ && pl.stage == ST_) return launch_nt<MT_, PG_, ST_>(p, nt, pl.smem, overlap, st);
   I4TC_SKINNY_CASE(1, true, true)
   I4TC_SKINNY_CASE(1, true, false)
   I4TC_SKINNY_CASE(1, false, true)
