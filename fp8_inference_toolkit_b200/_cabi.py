@@ -49,6 +49,7 @@ SIGNATURES = {
     "i4tc_gemm_grouped_scratch_bytes": (_l, [_l, _l, _l, _i, _i]),
     "i4tc_gemm_grouped_scratch": (_i, [_p, _p, _p, _p, _p, _p, _p, _l, _l, _l, _l, _p, _l, _i, _p]),
     "i4tc_linear": (_i, [_p, _i, _l, _l, _l, _p, _p, _i, _p, _p, _p, _l, _p, _l, _i, _p]),
+    "i4tc_linear_asymmetric": (_i, [_p, _i, _l, _l, _l, _d, _p, _p, _p, _p, _p, _p, _p, _p, _l, _p, _l, _i, _p]),
     "i4tc_gemm_grouped_int32": (_i, [_p, _p, _p, _l, _l, _l, _i, _p]),
     "i4tc_moe_sort_scratch_bytes": (_l, [_l, _l]),
     "i4tc_moe_sort": (_i, [_p, _l, _l, _p, _p, _p, _p, _l, _i, _p]),

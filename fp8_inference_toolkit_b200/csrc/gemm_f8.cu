@@ -386,7 +386,7 @@ static int launch_f8(const GemmParams& p, const CUtensorMap& tmP, const CUtensor
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = p.overlap ? 2 : 1;
+  cfg.numAttrs = 2;   // (behind the expansion, whoever called)
   return launch_pairs(cfg, pl, w4a4_group_f8_kernel<BN, AZP>, p, tmP, tmQ, p_pitch, q_pitch);
 }
 

@@ -298,9 +298,9 @@ static int run_dense(const DenseArgs& d, int device, void* stream) {
   if (int rc = launch_w4a4_gemm(p, tmP, tmQ, sh.bn, grid, false, epi_warps_for(d.epi_mode), static_cast<cudaStream_t>(stream))) return rc;
   if (p.splits > 1) {
     if (d.epi_mode == EPI_CHANNEL)
-      return launch_split_reduce_scaled(p.split_ws, p.ws_stride, p.splits, d.M, d.N, d.sa, d.sb, d.out, d.out_dtype, d.overlap,
+      return launch_split_reduce_scaled(p.split_ws, p.ws_stride, p.splits, d.M, d.N, d.sa, d.sb, d.out, d.out_dtype, true,
                                         static_cast<cudaStream_t>(stream));
-    return launch_split_reduce(p.split_ws, p.ws_stride, p.splits, d.M * d.N, d.out, d.overlap, static_cast<cudaStream_t>(stream));
+    return launch_split_reduce(p.split_ws, p.ws_stride, p.splits, d.M * d.N, d.out, true, static_cast<cudaStream_t>(stream));
   }
   return I4TC_OK;
 }
@@ -468,6 +468,17 @@ extern "C" int i4tc_linear(const void* x, int dtype, int64_t M, int64_t K, int64
   if (int rc = i4tc_quant_grouped(x, dtype, M, K, ldx, 128, x_packed, x_scale, I4TC_ROLE_ACTIVATION, device, stream)) return rc;
   return gemm_grouped_scratch_impl(x_packed, w, x_scale, w_scale, nullptr, nullptr, out, M, N, 128, K / 128, scratch,
                                    scratch_bytes, true, device, stream);
+}
+
+extern "C" int i4tc_linear_asymmetric(const void* x, int dtype, int64_t M, int64_t K, int64_t ldx, double clip_ratio,
+                                      const void* smooth_scale, const uint8_t* w, const float* w_scale, const float* w_col_sum,
+                                      uint8_t* x_packed, float* x_scale, float* x_azp, void* out, int64_t N, void* scratch,
+                                      int64_t scratch_bytes, int device, void* stream) {
+  if (int rc = i4tc_quant_asymmetric_grouped(x, dtype, M, K, ldx, 128, clip_ratio, smooth_scale, x_packed, x_scale, x_azp, device, stream))
+    return rc;
+  I4TC_REQUIRE(M == 0 || N == 0 || (x_azp && w_col_sum), I4TC_EINVAL, "null x_azp or w_col_sum");
+  return gemm_grouped_scratch_impl(x_packed, w, x_scale, w_scale, x_azp, w_col_sum, out, M, N, 128, K / 128, scratch, scratch_bytes,
+                                   true, device, stream);
 }
 
 extern "C" int i4tc_gemm_grouped_int32(const uint8_t* a, const uint8_t* b, int32_t* out, int64_t M, int64_t N,

@@ -708,6 +708,7 @@ __global__ void __launch_bounds__(256) quant_grouped_ext_kernel(const T* __restr
                                                                 int64_t ldx, float clip, const T* __restrict__ smooth,
                                                                 uint8_t* __restrict__ packed, float* __restrict__ scale,
                                                                 float* __restrict__ azp_adj, int segs_per_block) {
+  pdl_trigger();
   using V = typename std::conditional<SMOOTH, float, T>::type;
   constexpr int GS = LPG * kQLane;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

@@ -82,6 +82,7 @@ __global__ void __launch_bounds__(256) quant_ext_kernel(const T* __restrict__ x,
                                                         bool vec_s, uint8_t* __restrict__ packed,
                                                         float* __restrict__ scale, float* __restrict__ azp_adj) {
   constexpr int GS = EPL * 32;
+  pdl_trigger();
   constexpr int U = kSlicesPerWarp;
   const int lane = threadIdx.x & 31;
   const unsigned items = rows * G;   // < 2^31, checked by the host

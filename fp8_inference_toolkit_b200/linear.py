@@ -114,12 +114,9 @@ class W4A4Int4TCLinearMethod:
         if self.per_channel:
             out = ops.linear(x2d, layer.weight_int4, layer.weight_scale, N, True)
         elif self.asymmetric:
-            out = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
             sm = getattr(layer, "smooth_scale", None)
-            xp, xs, azp = ops.dynamic_int4_quant_asymmetric_clipped_grouped(
-                x2d, GROUP_SIZE, self.clip_ratio, None if sm is None else sm.to(x2d.dtype))
-            ops.cutlass_int4_fused_grouped_gemm_azp(xp, layer.weight_int4, xs, layer.weight_scale, out, azp,
-                                                    layer.w_col_sum, M, N, GROUP_SIZE, K // GROUP_SIZE)
+            out = ops.linear_asymmetric(x2d, layer.weight_int4, layer.weight_scale, layer.w_col_sum, N, self.clip_ratio,
+                                        None if sm is None else sm.to(x2d.dtype))
         else:
             sm = getattr(layer, "smooth_scale", None)
             if sm is not None:

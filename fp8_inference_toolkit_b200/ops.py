@@ -392,6 +392,43 @@ def linear(x: torch.Tensor, w_packed: torch.Tensor, w_scale: torch.Tensor, N: in
     return out
 
 
+def linear_asymmetric(x: torch.Tensor, w_packed: torch.Tensor, w_scale: torch.Tensor, w_col_sum: torch.Tensor, N: int,
+                      clip_ratio: float, smooth_scale: torch.Tensor | None = None) -> torch.Tensor:
+    """``dynamic_int4_quant_asymmetric_clipped_grouped`` + ``cutlass_int4_fused_grouped_gemm_azp`` in one library call and one
+    buffer, as ``linear`` does for symmetric codes.  bf16 [M,N]."""
+    x, M, K, G = _ext_input(x, 128, "dynamic_int4_quant_asymmetric_clipped_grouped")
+    _require(0.0 < clip_ratio <= 1.0, "clip_ratio must be in (0, 1]")
+    sm_ptr = None
+    if smooth_scale is not None:
+        _require(smooth_scale.is_cuda and smooth_scale.dtype == x.dtype, "smooth_scale must match the input's dtype")
+        _require(smooth_scale.numel() == K, "smooth_scale must be [K]")
+        _same_device(x, smooth_scale)
+        smooth_scale = smooth_scale.contiguous()
+        sm_ptr = smooth_scale.data_ptr()
+    _packed(w_packed, "b_packed")
+    _require(w_packed.numel() == N * (K // 2), "b_packed must be [G, N, 64]")
+    _f32(w_scale, "scale_b", G * N)
+    _f32(w_col_sum, "w_col_sum", G * N)
+    _same_device(x, w_packed, w_scale, w_col_sum)
+    dev = _dev(x)
+    out = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
+    codes, values = _pad256(M * (K // 2)), _pad256(G * M * 4)
+    base_bytes = codes + 2 * values
+    extra = lib.i4tc_gemm_grouped_scratch_bytes(M, N, G, 1, dev) if M > 128 else 0
+    if extra:
+        try:
+            buf = torch.empty(base_bytes + extra, dtype=torch.uint8, device=x.device)
+        except torch.cuda.OutOfMemoryError:
+            extra = 0
+    if not extra:
+        buf = torch.empty(base_bytes, dtype=torch.uint8, device=x.device)
+    at = buf.data_ptr()
+    check(lib.i4tc_linear_asymmetric(x.data_ptr(), _DTYPES[x.dtype], M, K, x.stride(0), float(clip_ratio), sm_ptr, w_packed.data_ptr(),
+                                     w_scale.data_ptr(), w_col_sum.data_ptr(), at, at + codes, at + codes + values, out.data_ptr(),
+                                     N, at + base_bytes if extra else None, extra, dev, _stream(x)), "linear_asymmetric")
+    return out
+
+
 def cutlass_int4_fused_grouped_gemm(a_packed, b_packed, scale_a, scale_b, out, M: int, N: int,
                                     group_size: int, num_groups: int) -> None:
     """Per-group-128 fused linear into the caller's bf16 ``out`` [M,N].

@@ -222,6 +222,13 @@ int i4tc_linear(const void* x, int dtype, int64_t M, int64_t K, int64_t ldx, con
                 int per_channel, uint8_t* x_packed, float* x_scale, void* out, int64_t N, void* scratch,
                 int64_t scratch_bytes, int device, void* stream);
 
+/* The linear with asymmetric activation codes in one call: x [M, K] (bf16 or fp16) through i4tc_quant_asymmetric_grouped (groups
+ * of 128) into x_packed / x_scale / x_azp, then i4tc_gemm_grouped_scratch with w_col_sum into bf16 out [M, N]. */
+int i4tc_linear_asymmetric(const void* x, int dtype, int64_t M, int64_t K, int64_t ldx, double clip_ratio,
+                           const void* smooth_scale, const uint8_t* w, const float* w_scale, const float* w_col_sum,
+                           uint8_t* x_packed, float* x_scale, float* x_azp, void* out, int64_t N, void* scratch,
+                           int64_t scratch_bytes, int device, void* stream);
+
 /* int32 partial sums of every group, out [G, M, N]: the integer accumulators that the fused
  * kernel drains.  No reference op exposes them; used to check the integer path bit for bit. */
 int i4tc_gemm_grouped_int32(const uint8_t* a, const uint8_t* b, int32_t* out, int64_t M,

@@ -75,3 +75,27 @@ def test_in_a_graph(M, K, N, per_channel):
         z = _separate(x, lin, per_channel)[:, :1].expand(M, K).contiguous()
         assert torch.equal(y, _separate(z, lin, per_channel))
     ops.check_status()
+
+
+@pytest.mark.parametrize("smooth", [False, True])
+@pytest.mark.parametrize("M,K,N", [(1, 1024, 96), (40, 2048, 1000), (300, 4096, 4096), (1000, 2048, 3001)])
+def test_asymmetric_back_to_back(M, K, N, smooth):
+    from fp8_inference_toolkit_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    w = (torch.randn(N, K, device="cuda", generator=gen) * 0.02).to(torch.bfloat16)
+    wp, ws = ops.static_int4_weight_quant_grouped(w, 128)
+    cs = ops.int4_weight_group_sums(wp)
+    sm = (torch.rand(K, device="cuda", generator=gen) + 0.5).to(torch.bfloat16) if smooth else None
+    xs = [(torch.randn(M, K, device="cuda", generator=gen) + 0.75 * i).to(torch.bfloat16) for i in range(4)]
+    want = []
+    for x in xs:
+        out = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+        p, s, z = ops.dynamic_int4_quant_asymmetric_clipped_grouped(x, 128, 0.95, sm)
+        ops.cutlass_int4_fused_grouped_gemm_azp(p, wp, s, ws, out, z, cs, M, N, 128, K // 128)
+        want.append(out)
+    torch.cuda.synchronize()
+    got = [ops.linear_asymmetric(xs[i % 4], wp, ws, cs, N, 0.95, sm) for i in range(20)]
+    for i, out in enumerate(got):
+        assert torch.equal(out, want[i % 4])
+    ops.check_status()
