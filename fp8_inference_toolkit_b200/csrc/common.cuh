@@ -90,7 +90,7 @@ int launch_grouped_ext(bool asym, const void* x, int dtype, int64_t rows, int64_
 // A kernel launched with `overlap` may start while its predecessor in the stream still runs, once every block of that has called
 // pdl_trigger() or ended; pdl_wait() returns when the predecessor has completed and its writes are visible (at once in a
 // kernel that was launched without).  Rules here: a kernel that reads or writes memory before its wait is overlapped by
-// i4tc_linear(_asymmetric) only, behind a quantiser that it launched itself without -- so everything earlier in the stream, the weights among it, is
+// i4tc_linear(_asymmetric) only (the others wait first and may overlap anything), behind a quantiser that it launched itself without -- so everything earlier in the stream, the weights among it, is
 // complete; every thread waits before it reads what the
 // predecessor wrote and before it writes what anybody else reads; every block waits before it ends; and a kernel in the middle of a
 // chain triggers after its own wait, so that whatever starts next finds everything but this kernel's results complete.
@@ -103,6 +103,10 @@ __device__ __forceinline__ const T* pdl_wait(const T* p) {
   return p;
 }
 
+template <typename T>
+__device__ __forceinline__ void pdl_fresh(T*& p) {   // after pdl_wait(): loads from p stay behind it
+  asm volatile("" : "+l"(p)::"memory");
+}
 __device__ __forceinline__ void pdl_wait(const uint8_t*& a, const float*& b) {
   asm volatile("griddepcontrol.wait;" : "+l"(a), "+l"(b)::"memory");
 }

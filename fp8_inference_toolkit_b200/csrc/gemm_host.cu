@@ -557,6 +557,7 @@ static int moe_grouped_gemm_impl(const uint8_t* a, const float* scale_a, const u
   p.out_rows = reinterpret_cast<const unsigned long long*>(out_rows);
   p.ldc = N;
   p.num_q_tiles = (int)((N + bn - 1) / bn);
+  p.overlap = 1;   // (the tile kernel waits before it touches anything)
   p.expert_offsets = expert_offsets;
   p.num_experts = (int)num_experts;
   p.splits = 1;

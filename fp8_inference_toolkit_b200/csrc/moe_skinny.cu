@@ -65,7 +65,13 @@ __global__ void __launch_bounds__(kMoeWarps * 32, BLOCKS) moe_skinny_kernel(cons
   constexpr int TOK = 8 * NT;
   extern __shared__ __align__(128) uint8_t smem[];
   const int e = blockIdx.y;
-  const int r0 = __ldg(p.offsets + e), rows = __ldg(p.offsets + e + 1) - r0;
+  const int32_t* offsets = p.offsets;
+  const uint8_t *pa = p.a, *pb = p.b;
+  const float *psa = p.sa, *psb = p.sb;
+  pdl_wait();
+  pdl_fresh(offsets); pdl_fresh(pa); pdl_fresh(pb); pdl_fresh(psa); pdl_fresh(psb);
+  pdl_trigger();
+  const int r0 = __ldg(offsets + e), rows = __ldg(offsets + e + 1) - r0;
   if (rows <= 0) return;   // the whole block
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
@@ -76,8 +82,8 @@ __global__ void __launch_bounds__(kMoeWarps * 32, BLOCKS) moe_skinny_kernel(cons
   uint8_t* hi_s = smem + (size_t)G * TOK * 64;
   float* sx_s = reinterpret_cast<float*>(smem + (size_t)G * TOK * 128);
   const long long row = (long long)e * G * p.N + (mine ? n0 : 0) + g;   // weight row of group 0
-  const uint8_t* wsrc = p.b + row * 64 + t * 16;
-  const float* ssrc = p.sb + row;
+  const uint8_t* wsrc = pb + row * 64 + t * 16;
+  const float* ssrc = psb + row;
   const long long wstep = (long long)p.N * 64;
 
   uint4 wa[DEPTH], wb[DEPTH];
@@ -104,13 +110,13 @@ __global__ void __launch_bounds__(kMoeWarps * 32, BLOCKS) moe_skinny_kernel(cons
     for (int i = threadIdx.x; i < G * TOK * 4; i += kMoeWarps * 32) {
       const int j = i & 3, m = (i >> 2) % TOK, grp = (i >> 2) / TOK;
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (m < n) v = __ldg(reinterpret_cast<const uint4*>(p.a + ((long long)grp * p.P + r0 + first + m) * 64) + j);
+      if (m < n) v = __ldg(reinterpret_cast<const uint4*>(pa + ((long long)grp * p.P + r0 + first + m) * 64) + j);
       *reinterpret_cast<uint4*>(lo_s + (size_t)i * 16) = low_nibbles(v);
       *reinterpret_cast<uint4*>(hi_s + (size_t)i * 16) = high_nibbles(v);
     }
     for (int i = threadIdx.x; i < G * TOK; i += kMoeWarps * 32) {
       const int m = i % TOK, grp = i / TOK;
-      sx_s[i] = m < n ? __ldg(p.sa + (long long)grp * p.P + r0 + first + m) * (1.0f / 256.0f) : 0.f;
+      sx_s[i] = m < n ? __ldg(psa + (long long)grp * p.P + r0 + first + m) * (1.0f / 256.0f) : 0.f;
     }
     __syncthreads();
 
@@ -178,8 +184,8 @@ int launch_nt(const MoeSkinnyParams& p, int num_experts, cudaStream_t st) {
   const size_t smem = moe_skinny_smem(p.G, 8 * NT);
   I4TC_CUDA(cudaFuncSetAttribute(moe_skinny_kernel<NT, DEPTH, BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int blocks = (p.N + 16 * kMoeWarps - 1) / (16 * kMoeWarps);
-  moe_skinny_kernel<NT, DEPTH, BLOCKS><<<dim3((unsigned)blocks, (unsigned)num_experts), kMoeWarps * 32, smem, st>>>(p);
-  I4TC_CUDA(cudaGetLastError());
+  I4TC_CUDA(launch_kernel(true, moe_skinny_kernel<NT, DEPTH, BLOCKS>, dim3((unsigned)blocks, (unsigned)num_experts), kMoeWarps * 32, smem,
+                          st, p));
   return I4TC_OK;
 }
 

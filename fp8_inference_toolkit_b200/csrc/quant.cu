@@ -453,6 +453,10 @@ __global__ void __launch_bounds__(quant_rows<MODE>() * 32, MODE == 3 ? 8 : MODE 
     QuantOutMap out = QuantOutMap{nullptr, nullptr, 0, 0, 0, 0, nullptr, 1, 0, 0}) {
   constexpr int GS = LPG * kQLane;
   if (MODE == 0) pdl_trigger();   // (the GEMM behind it may start)
+  if (MODE == 2) {   // launched so that it starts under the end of the GEMM in front of it
+    x = pdl_wait(x);
+    pdl_trigger();
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t r = (int64_t)blockIdx.x * quant_rows<MODE>() + warp;
   bool row_ok = r < rows;
@@ -548,6 +552,41 @@ __global__ void __launch_bounds__(quant_rows<MODE>() * 32, MODE == 3 ? 8 : MODE 
     }
 #pragma unroll
     for (int j = 0; j < kQVecs; ++j) cur[j] = nxt[j];
+  }
+}
+
+// Tokens quantised once and written to every row that wants them: token t's codes and scales go to rows inv[t * top_k + j] of the
+// group-major [G, R, 64] / [G, R] destination (none for a negative index).  The layout of the kernel above, group size 128.
+// As a quantiser and a copy of its packed rows [4096 tokens, 2048] x 8 took 6.4 + 13.8 us and two launches; here 11.4.
+__global__ void __launch_bounds__(256) quant_fanout_kernel(const __nv_bfloat16* x, int64_t rows, int K, int64_t ldx,
+                                                           const int32_t* inv, int top_k, int64_t R,
+                                                           uint8_t* __restrict__ packed, float* __restrict__ scale) {
+  pdl_wait();
+  pdl_fresh(x);
+  pdl_fresh(inv);
+  pdl_trigger();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t r = (int64_t)blockIdx.x * kQRows + warp;
+  if (r >= rows) return;   // the whole warp
+  const int k = blockIdx.y * kQSeg + lane * kQLane;
+  Vec8<__nv_bfloat16> v[kQVecs];
+  load_segment<__nv_bfloat16, 0>(v, x + r * ldx, k, K, true);
+  float absmax = absmax_of(v);
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1) absmax = fmaxf(absmax, __shfl_xor_sync(0xffffffffu, absmax, o));
+  const float s = __fdiv_rn(absmax, 7.0f);
+  const AbsmaxCodes<__nv_bfloat16> codes(absmax, s);
+  const uint4 w = make_uint4(codes.word(v[0]), codes.word(v[1]), codes.word(v[2]), codes.word(v[3]));
+  const float sc = scale_out(absmax, s, I4TC_ROLE_ACTIVATION);
+  const int64_t g = k / 128;
+  for (int j0 = 0; j0 < top_k; j0 += 32) {
+    const int mine = j0 + lane < top_k ? __ldg(inv + r * top_k + j0 + lane) : -1;
+    for (int j = 0; j < min(32, top_k - j0); ++j) {
+      const int64_t pos = __shfl_sync(0xffffffffu, mine, j);
+      if (pos < 0 || k >= K) continue;
+      *reinterpret_cast<uint4*>(packed + (g * R + pos) * 64 + (lane & 3) * 16) = w;
+      if ((lane & 3) == 0) scale[g * R + pos] = sc;
+    }
   }
 }
 
@@ -968,9 +1007,9 @@ static int launch_grouped_t(const T* x, int64_t rows, int64_t K, int64_t ldx, in
   dim3 grid((unsigned)row_blocks, (unsigned)((nseg + spb - 1) / spb));
   I4TC_REQUIRE(grid.y <= 65535, I4TC_EINVAL, "K=%lld too large for the grouped quantiser", (long long)K);
 #define I4TC_LAUNCH_G(LPG)                                                                             \
-  quant_grouped_kernel<T, LPG, MODE, GIVEN><<<grid, quant_rows<MODE>() * 32, 0, st>>>(x, rows, (int)K, ldx, row_index,     \
-                                                                   index_div, src_rows, given, packed, scale, role, spb, \
-                                                                   static_cast<const T*>(aux), eps)
+  I4TC_CUDA(launch_kernel(MODE == 2, quant_grouped_kernel<T, LPG, MODE, GIVEN>, grid, quant_rows<MODE>() * 32, 0, st, x, rows, (int)K, \
+                          ldx, row_index, index_div, src_rows, given, packed, scale, role, spb, static_cast<const T*>(aux), eps,     \
+                          QuantOutMap{nullptr, nullptr, 0, 0, 0, 0, nullptr, 1, 0, 0}))
   switch (gs) {
     case 32: I4TC_LAUNCH_G(1); break;
     case 64: I4TC_LAUNCH_G(2); break;
@@ -1129,6 +1168,23 @@ extern "C" int i4tc_moe_gather_quant(const void* x, int dtype, int64_t num_token
   I4TC_REQUIRE(sorted_pairs || num_pairs == 0, I4TC_EINVAL, "null sorted_pairs");
   return launch_grouped<1, false>(x, dtype, num_pairs, K, ldx, 128, sorted_pairs, (int)top_k, nullptr, packed,
                                   scale, I4TC_ROLE_ACTIVATION, device, stream, nullptr, 0.f, num_tokens);
+}
+
+extern "C" int i4tc_moe_quant_fanout(const void* x, int64_t num_tokens, int64_t K, int64_t ldx, const int32_t* inv_pairs,
+                                     int64_t top_k, int64_t num_rows, uint8_t* packed, float* scale, int device, void* stream) {
+  I4TC_REQUIRE(top_k > 0 && top_k < (1 << 20) && num_tokens >= 0 && num_tokens * top_k < (1ll << 31), I4TC_EINVAL, "bad sizes");
+  I4TC_REQUIRE(K > 0 && K % 128 == 0 && K < (1ll << 31) && num_rows >= 0, I4TC_EINVAL, "K must be a positive multiple of 128");
+  if (num_tokens == 0 || num_rows == 0) return I4TC_OK;
+  I4TC_REQUIRE(x && inv_pairs && packed && scale, I4TC_EINVAL, "null pointer");
+  if (int rc = check_vec_input(x, I4TC_BF16, ldx, "moe_quant_fanout")) return rc;
+  I4TC_REQUIRE(aligned_to(packed, 16), I4TC_EALIGN, "packed output must be 16-byte aligned");
+  DeviceGuard guard(device);
+  I4TC_CUDA(guard.err);
+  const dim3 grid((unsigned)((num_tokens + kQRows - 1) / kQRows), (unsigned)((K + kQSeg - 1) / kQSeg));
+  I4TC_REQUIRE(grid.y <= 65535, I4TC_EINVAL, "K=%lld too large", (long long)K);
+  I4TC_CUDA(launch_kernel(true, quant_fanout_kernel, grid, 256, 0, static_cast<cudaStream_t>(stream),
+                          static_cast<const __nv_bfloat16*>(x), num_tokens, (int)K, ldx, inv_pairs, (int)top_k, num_rows, packed, scale));
+  return I4TC_OK;
 }
 
 extern "C" int i4tc_moe_ep_dispatch_quant(const void* x, int64_t num_tokens, int64_t K, int64_t ldx,

@@ -82,6 +82,22 @@ def moe_quant_gather(x: torch.Tensor, sorted_pairs: torch.Tensor, top_k: int):
     return packed, scale
 
 
+def moe_quant_fanout(x: torch.Tensor, inv_pairs: torch.Tensor, top_k: int):
+    """The result of ``moe_quant_gather`` from the other side of the permutation: every token is quantised once and its packed row
+    written to the rows ``inv_pairs[t * top_k + j]`` in the same kernel (left-out pairs, index -1, write nothing)."""
+    _require(x.is_cuda and x.dim() == 2 and x.is_contiguous() and x.dtype == torch.bfloat16,
+             "x must be a contiguous 2D bfloat16 CUDA tensor")
+    T, K = x.shape
+    _require(K % 128 == 0, "hidden size must be a multiple of 128")
+    P = inv_pairs.numel()
+    _require(P == T * top_k, "inv_pairs must hold top_k rows per token")
+    packed = torch.empty((K // 128, P, 64), dtype=torch.uint8, device=x.device)
+    scale = torch.empty((K // 128, P), dtype=torch.float32, device=x.device)
+    check(lib.i4tc_moe_quant_fanout(x.data_ptr(), T, K, x.stride(0), inv_pairs.data_ptr(), top_k, P, packed.data_ptr(),
+                                    scale.data_ptr(), _dev(x), _stream(x)), "moe_quant_fanout")
+    return packed, scale
+
+
 def moe_w4a4_grouped_gemm(a_packed, scale_a, b_packed, scale_b, expert_offsets, out, N: int, num_groups: int,
                           num_experts: int) -> None:
     """out[r,:] = linear_grouped(a[:, r, :], W_e) for rows r of expert e (bf16 [P,N], caller-allocated).
@@ -189,7 +205,7 @@ def moe_experts_forward(x_rows_packed, x_rows_scale, expert_offsets, w: MoEWeigh
 def moe_layer(x: torch.Tensor, expert_ids: torch.Tensor, expert_w: torch.Tensor, w: MoEWeights) -> torch.Tensor:
     """Single-GPU MoE layer.  ``x`` bf16 [T,H]; ``expert_ids`` i32 [T,k]; ``expert_w`` f32 [T,k] -> bf16 [T,H]."""
     T, top_k = expert_ids.shape
-    sorted_pairs, inv_pairs, offsets = moe_sort_tokens(expert_ids, w.num_experts)
-    ap, asc = moe_quant_gather(x, sorted_pairs, top_k)
+    _, inv_pairs, offsets = moe_sort_tokens(expert_ids, w.num_experts)
+    ap, asc = moe_quant_fanout(x, inv_pairs, top_k)
     y = moe_experts_forward(ap, asc, offsets, w)
     return moe_combine(y, inv_pairs, expert_w.contiguous(), T, top_k)

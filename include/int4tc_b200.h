@@ -278,6 +278,11 @@ int i4tc_moe_gather_quant(const void* x, int dtype, int64_t num_tokens, int64_t 
                           const int32_t* sorted_pairs, int64_t num_pairs, int64_t top_k,
                           uint8_t* packed, float* scale, int device, void* stream);
 
+/* Every token of bf16 x quantised once (gs=128, activation role) and written to rows inv_pairs[t * top_k + j], j < top_k, of
+ * packed [K/128, num_rows, 64] / scale [K/128, num_rows]; a negative index writes nothing. */
+int i4tc_moe_quant_fanout(const void* x, int64_t num_tokens, int64_t K, int64_t ldx, const int32_t* inv_pairs, int64_t top_k,
+                          int64_t num_rows, uint8_t* packed, float* scale, int device, void* stream);
+
 /* The same result from rows that were quantised once per token (i4tc_quant_grouped over x, group size 128:
  * tok_packed [G, T, 64], tok_scale [G, T]) -- the quantiser works on whole rows, so quantising a token once and
  * copying its 68 bytes per group to every (token, slot) pair gives the codes and scales of quantising after the

@@ -1,0 +1,43 @@
+"""GPU: quantising each token straight into its expert-sorted rows gives the rows of quantise-then-copy; the one-chunk sort; and
+layers one after the other, whose kernels start under the end of their predecessors, on inputs that change every call."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("T,K,top_k", [(1, 128, 1), (7, 384, 3), (65, 1152, 8), (130, 2048, 40)])
+def test_same_rows_as_the_copy(T, K, top_k):
+    from fp8_inference_toolkit_b200 import moe, ops
+
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, K, device="cuda", generator=gen).to(torch.bfloat16)
+    ids = torch.randint(-1, 9, (T, top_k), device="cuda", generator=gen).to(torch.int32)     # -1 and 8: left out
+    sp, inv, off = moe.moe_sort_tokens(ids, 8)
+    n = int(off[-1])
+    p, s = moe.moe_quant_gather(x, sp, top_k)
+    p2, s2 = moe.moe_quant_fanout(x, inv, top_k)
+    assert torch.equal(p[:, :n], p2[:, :n]) and torch.equal(s[:, :n], s2[:, :n])
+    ops.check_status()
+
+
+@pytest.mark.parametrize("T", [3, 64, 300, 700])
+def test_layers_back_to_back(T):
+    """300 and 700 tokens: the register-fed and the tile kernel."""
+    from fp8_inference_toolkit_b200 import moe, ops
+
+    E, H, I, k = 16, 512, 256, 2
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    w = moe.MoEWeights.quantize((torch.randn(E, 2 * I, H, device="cuda", generator=gen) * 0.02).to(torch.bfloat16),
+                                (torch.randn(E, H, I, device="cuda", generator=gen) * 0.02).to(torch.bfloat16))
+    xs = [torch.randn(T, H, device="cuda", generator=gen).mul_(2.0 ** i).to(torch.bfloat16) for i in range(4)]
+    routes = [moe.moe_route(torch.randn(T, E, device="cuda", generator=gen), k) for _ in range(4)]
+    want = []
+    for x, (ids, wt) in zip(xs, routes):
+        want.append(moe.moe_layer(x, ids, wt, w))
+        torch.cuda.synchronize()
+    got = [moe.moe_layer(xs[i % 4], *routes[i % 4], w) for i in range(24)]
+    for i, out in enumerate(got):
+        assert torch.equal(out, want[i % 4])
+    ops.check_status()
