@@ -87,13 +87,14 @@ int launch_grouped_ext(bool asym, const void* x, int dtype, int64_t rows, int64_
                        const void* smooth, uint8_t* packed, float* scale, float* azp_adj, cudaStream_t st);
 
 // ---- overlap of a kernel's start with the end of the one before it (programmatic dependent launch) --------------
-// A kernel launched with `overlap` may start while its predecessor in the stream still runs, once every block of that has called
-// pdl_trigger() or ended; pdl_wait() returns when the predecessor has completed and its writes are visible (at once in a
-// kernel that was launched without).  Rules here: a kernel that reads or writes memory before its wait is overlapped by
-// i4tc_linear(_asymmetric) only (the others wait first and may overlap anything), behind a quantiser that it launched itself without -- so everything earlier in the stream, the weights among it, is
-// complete; every thread waits before it reads what the
-// predecessor wrote and before it writes what anybody else reads; every block waits before it ends; and a kernel in the middle of a
-// chain triggers after its own wait, so that whatever starts next finds everything but this kernel's results complete.
+// A kernel launched with `overlap` may start while its predecessor in the stream still runs, once every block of that has
+// called pdl_trigger() or ended; pdl_wait() returns when the predecessor has completed and its writes are visible (at
+// once in a kernel that was launched without).  Rules here: every thread waits before it reads what the predecessor
+// wrote and before it writes what anybody else reads; every block waits before it ends; a kernel in the middle of a chain triggers after
+// its own wait, so that whatever starts next finds everything but this kernel's results complete.  A kernel that waits
+// before it touches memory at all may overlap anything; one that reads weights first is overlapped by i4tc_linear(_asymmetric)
+// only, behind a quantiser that it launched itself without -- so everything earlier in the stream, the weights among it, is
+// complete.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // The wait with the pointers passed through it, so that no load from them can be placed before.

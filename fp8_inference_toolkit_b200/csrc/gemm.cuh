@@ -58,7 +58,7 @@ struct GemmParams {
   int groups_per_split;
   float* split_ws;
   long long ws_stride;
-  int overlap;   // host: launch so that the kernel may start before its predecessor, the quantiser, has ended
+  int weights_early;   // host, expanded path: the kernel in front is the quantiser of the activations, so the weights may be read before the wait
 };
 
 // out[i] = bf16(sum_s ws[s * stride + i]), s ascending.

@@ -355,10 +355,14 @@ __device__ __forceinline__ void expand_chunk(const uint8_t* __restrict__ src, ui
 
 // Packed [G, rows, 64 B] of both operands -> e4m3 [G, pitch, 128 B], pitch = rows rounded up to 32 (Q rows of a 32-row
 // block in the order qperm; the rows that fill up a block are zero).  A thread expands 16 packed bytes.
-__global__ void __launch_bounds__(256) expand_e4m3_kernel(const uint8_t* __restrict__ a, const uint8_t* __restrict__ b,
-                                                          int M, int m_pitch, int N, int n_pitch, int G,
+__global__ void __launch_bounds__(256) expand_e4m3_kernel(const uint8_t* a, const uint8_t* b,
+                                                          int M, int m_pitch, int N, int n_pitch, int G, int weights_early,
                                                           uint8_t* __restrict__ ea, uint8_t* __restrict__ eb) {
-  // the weights first: they are there while the quantiser still works on the activations
+  if (!weights_early) {   // behind a kernel that may have written the weights
+    pdl_wait();
+    pdl_fresh(b);
+  }
+  // the weights first: with weights_early they are there while the quantiser still works on the activations
   const long long ca = (long long)G * m_pitch * 4, cb = (long long)G * n_pitch * 4, step = (long long)gridDim.x * 256;
   long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   for (; i < cb; i += step) expand_chunk(b, eb, i, N, n_pitch, true);
@@ -405,8 +409,8 @@ int launch_w4a4_group_f8(const GemmParams& p, const uint8_t* a, const uint8_t* b
   if (int rc = get_tensor_map_i8(device, eb, (long long)n_pitch * p.G, 128, bn / 2, &tmQ)) return rc;
   const long long chunks = (long long)(m_pitch + n_pitch) * p.G * 4;
   const long long blocks = (chunks + 255) / 256, cap = (long long)sm_count * 8 * 4;
-  I4TC_CUDA(launch_kernel(p.overlap != 0, expand_e4m3_kernel, dim3((unsigned)(blocks < cap ? blocks : cap)), 256, 0, st, a, b, M, m_pitch,
-                          N, n_pitch, p.G, ea, eb));
+  I4TC_CUDA(launch_kernel(true, expand_e4m3_kernel, dim3((unsigned)(blocks < cap ? blocks : cap)), 256, 0, st, a, b, M, m_pitch,
+                          N, n_pitch, p.G, p.weights_early, ea, eb));
   const long long tiles = (long long)p.num_p_tiles * p.num_q_tiles;
   const int grid = 2 * (int)(tiles < sm_count / 2 ? tiles : sm_count / 2);
   const bool azp = p.zp != nullptr;

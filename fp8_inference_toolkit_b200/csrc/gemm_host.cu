@@ -184,7 +184,7 @@ static int run_dense(const DenseArgs& d, int device, void* stream) {
       p.num_q_tiles = (int)((d.N + bn - 1) / bn);
       p.splits = 1; p.groups_per_split = d.G;
       p.status = info->status;
-      p.overlap = d.overlap;
+      p.weights_early = d.overlap;
       PairLaunch pl;
       const int rc = launch_w4a4_group_f8(p, d.a, d.b, d.scratch, bn, device, info->sm_count, static_cast<cudaStream_t>(stream), &pl);
       if (!pl.failed) return rc;
@@ -209,7 +209,6 @@ static int run_dense(const DenseArgs& d, int device, void* stream) {
   p.ldc = d.N;
   p.out_gstride = d.M * d.N;
   p.status = info->status;
-  p.overlap = d.overlap;
   p.p_rowmajor = p.q_rowmajor = d.rowmajor ? 1 : 0;
   const bool per_group_scales = d.epi_mode == EPI_GROUP;
   const uint8_t *pbase, *qbase;
@@ -557,7 +556,6 @@ static int moe_grouped_gemm_impl(const uint8_t* a, const float* scale_a, const u
   p.out_rows = reinterpret_cast<const unsigned long long*>(out_rows);
   p.ldc = N;
   p.num_q_tiles = (int)((N + bn - 1) / bn);
-  p.overlap = 1;   // (the tile kernel waits before it touches anything)
   p.expert_offsets = expert_offsets;
   p.num_experts = (int)num_experts;
   p.splits = 1;

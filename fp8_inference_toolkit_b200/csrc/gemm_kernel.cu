@@ -200,8 +200,11 @@ __device__ __forceinline__ uint4 quad_transpose(const uint32_t (&x)[4], int lq) 
 // "slabs" of 16 rows x 32 columns with tcgen05.ld.16x256b.x4: lane (lr = lane / 4, lq = lane % 4) then holds
 // rows {lr, lr + 8} of the slab and column pairs 8 * kk + 2 * lq + {0, 1}, kk = 0..3.  Over the two slabs of
 // a 32-column chunk a thread therefore owns 4 rows (8 * a + lr, a = 0..3) and, per row, adjacent column
-// pairs: the pair is the unit of the packed f32x2 arithmetic and of the scale reads (one 8-byte shared
-// load per pair, the same address in the 8 lanes that share lq).
+// pairs: the pair is the unit of the packed f32x2 arithmetic.  Where the Q rows are in the order qperm, two pairs are
+// four consecutive columns and their scales one 16-byte shared load, the same address in the 8 lanes that share lq.
+// A step drains both slabs of its columns on that one read: the shared memory is what the operand reads of the tensor core
+// keep busy (MoE of 4096 tokens 266 + 162 -> 258 + 154 us, [100, 12288] x [4096, 12288] 27.6 -> 25.6 against slab by
+// slab with 8-byte reads).
 //
 // Scales.  Two otherwise idle warps copy the kBM row scales and BN column scales of each K group from
 // global to shared memory (4-byte cp.async, kNS stages ahead, completion signalled on an mbarrier), so the
@@ -238,10 +241,8 @@ __device__ __forceinline__ void epilogue_group(const GemmParams& p, uint8_t* sme
 #pragma unroll
     for (int i = 0; i < CW / 2; ++i) f[i] = make_float2(0.f, 0.f);
     bool ok = true;
-    // Columns per step, of both slabs: a 32-column chunk, or half of one where registers are short.  (Slab by slab, with 8-byte reads
-    // of the column scales for each, a warp of 128 columns read shared memory 64 times per group: 4096 tokens x top 8 on
-    // 128 experts 266 + 162 us -> 258 + 154, [100, 12288] x [4096, 12288] 27.6 -> 25.6.  Letting warps whose rows lie past the tile skip
-    // the arithmetic in a loop of their own: +-0 to +6 %.)
+    // Columns per step, of both slabs: a 32-column chunk, or half of one where registers are short.  (Letting warps whose
+    // rows lie past the tile skip the arithmetic in a loop of their own: +-0 to +6 %.)
     constexpr int STEP = (CW > 64 || EW > 8) ? 16 : 32;
     bool pre = false;      // group `flush` was seen complete under the previous group's arithmetic
     for (int g = ti.g0; g < ti.g1; ++g) {
@@ -915,7 +916,7 @@ static int launch_bn(const GemmParams& p, const CUtensorMap& tmP, const CUtensor
     configured[dev] = true;
   }
   if (CG == 1) {
-    I4TC_CUDA(launch_kernel(p.overlap != 0, w4a4_gemm_kernel<BN, CG, EW>, dim3((unsigned)grid), C::THREADS, C::SMEM_BYTES, st, p, tmP, tmQ));
+    I4TC_CUDA(launch_kernel(true, w4a4_gemm_kernel<BN, CG, EW>, dim3((unsigned)grid), C::THREADS, C::SMEM_BYTES, st, p, tmP, tmQ));
   } else {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid, 1, 1);
@@ -930,7 +931,7 @@ static int launch_bn(const GemmParams& p, const CUtensorMap& tmP, const CUtensor
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = p.overlap ? 2 : 1;
+    cfg.numAttrs = 2;
     return launch_pairs(cfg, pl, w4a4_gemm_kernel<BN, CG, EW>, p, tmP, tmQ);
   }
   I4TC_CUDA(cudaGetLastError());

@@ -21,10 +21,12 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
 constexpr int kNormThreads = 256, kNormVecs = 8;   // a row of up to 256 * 8 * 8 = 16384 elements stays in registers
 
 // out = bf16(bf16(x * rsqrt(mean(x^2) + eps)) * w), one block per row.
-__global__ void __launch_bounds__(kNormThreads) rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, int K, long long ldx,
-                                                               const __nv_bfloat16* __restrict__ w, float eps,
+__global__ void __launch_bounds__(kNormThreads) rmsnorm_kernel(const __nv_bfloat16* x, int K, long long ldx,
+                                                               const __nv_bfloat16* w, float eps,
                                                                __nv_bfloat16* __restrict__ out) {
   __shared__ float part[kNormThreads / 32];
+  x = pdl_wait(x);
+  pdl_fresh(w);
   const uint4* src = reinterpret_cast<const uint4*>(x + (long long)blockIdx.x * ldx);
   const int nv = K / 8, t = threadIdx.x;
   uint4 v[kNormVecs];
@@ -96,11 +98,12 @@ __device__ __forceinline__ void store_oct(__nv_bfloat16* p, const uint4& v) {
 }
 
 template <bool A16>
-__global__ void __launch_bounds__(kRopeWarps * 32) qk_norm_rope_kernel(__nv_bfloat16* __restrict__ qkv, long long ld, int q_heads,
-                                                                       int heads, int seq, const __nv_bfloat16* __restrict__ wq,
-                                                                       const __nv_bfloat16* __restrict__ wk,
-                                                                       const __nv_bfloat16* __restrict__ cos_t,
-                                                                       const __nv_bfloat16* __restrict__ sin_t, float eps) {
+__global__ void __launch_bounds__(kRopeWarps * 32) qk_norm_rope_kernel(__nv_bfloat16* qkv, long long ld, int q_heads, int heads, int seq,
+                                                                       const __nv_bfloat16* wq, const __nv_bfloat16* wk,
+                                                                       const __nv_bfloat16* cos_t, const __nv_bfloat16* sin_t,
+                                                                       float eps) {
+  pdl_wait();
+  pdl_fresh(qkv); pdl_fresh(wq); pdl_fresh(wk); pdl_fresh(cos_t); pdl_fresh(sin_t);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l = lane & 15;
   const unsigned tok = blockIdx.x;
   __nv_bfloat16* at = qkv + (long long)tok * ld + l * 8;
@@ -166,10 +169,9 @@ extern "C" int i4tc_rmsnorm(const void* x, int64_t rows, int64_t K, int64_t ldx,
                "rows, weight and output must be 16-byte aligned");
   DeviceGuard guard(device);
   I4TC_CUDA(guard.err);
-  rmsnorm_kernel<<<(unsigned)rows, kNormThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), (int)K, ldx, static_cast<const __nv_bfloat16*>(weight), eps,
-      static_cast<__nv_bfloat16*>(out));
-  I4TC_CUDA(cudaGetLastError());
+  I4TC_CUDA(launch_kernel(true, rmsnorm_kernel, dim3((unsigned)rows), kNormThreads, 0, static_cast<cudaStream_t>(stream),
+                          static_cast<const __nv_bfloat16*>(x), (int)K, ldx, static_cast<const __nv_bfloat16*>(weight), eps,
+                          static_cast<__nv_bfloat16*>(out)));
   return I4TC_OK;
 }
 
@@ -187,10 +189,9 @@ extern "C" int i4tc_qk_norm_rope(void* qkv, int64_t tokens, int64_t ld, int64_t 
   I4TC_CUDA(guard.err);
   const bool a16 = aligned_to(qkv, 16) && ld % 8 == 0 && aligned_to(q_weight, 16) && aligned_to(k_weight, 16) &&
                    aligned_to(cos_table, 16) && aligned_to(sin_table, 16);
-  (a16 ? qk_norm_rope_kernel<true> : qk_norm_rope_kernel<false>)<<<(unsigned)tokens, kRopeWarps * 32, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<__nv_bfloat16*>(qkv), ld, (int)q_heads, (int)heads, (int)seq, static_cast<const __nv_bfloat16*>(q_weight),
-      static_cast<const __nv_bfloat16*>(k_weight), static_cast<const __nv_bfloat16*>(cos_table),
-      static_cast<const __nv_bfloat16*>(sin_table), eps);
-  I4TC_CUDA(cudaGetLastError());
+  I4TC_CUDA(launch_kernel(true, a16 ? qk_norm_rope_kernel<true> : qk_norm_rope_kernel<false>, dim3((unsigned)tokens), kRopeWarps * 32, 0,
+                          static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(qkv), ld, (int)q_heads, (int)heads, (int)seq,
+                          static_cast<const __nv_bfloat16*>(q_weight), static_cast<const __nv_bfloat16*>(k_weight),
+                          static_cast<const __nv_bfloat16*>(cos_table), static_cast<const __nv_bfloat16*>(sin_table), eps));
   return I4TC_OK;
 }

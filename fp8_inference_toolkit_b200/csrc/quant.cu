@@ -447,14 +447,15 @@ __host__ __device__ constexpr int quant_rows() { return MODE == 3 ? 4 : kQRows; 
 
 template <typename T, int LPG, int MODE, bool GIVEN, bool OUTMAP = false>
 __global__ void __launch_bounds__(quant_rows<MODE>() * 32, MODE == 3 ? 8 : MODE == 2 ? 3 : 1) quant_grouped_kernel(
-    const T* __restrict__ x, int64_t rows, int K, int64_t ldx, const int32_t* __restrict__ row_index,
-    int index_div, int64_t src_rows, const float* __restrict__ given_scale, uint8_t* __restrict__ packed,
-    float* __restrict__ scale, int role, int segs_per_block, const T* __restrict__ aux, float eps,
+    const T* __restrict__ x, int64_t rows, int K, int64_t ldx, const int32_t* row_index,
+    int index_div, int64_t src_rows, const float* given_scale, uint8_t* __restrict__ packed,
+    float* __restrict__ scale, int role, int segs_per_block, const T* aux, float eps,
     QuantOutMap out = QuantOutMap{nullptr, nullptr, 0, 0, 0, 0, nullptr, 1, 0, 0}) {
   constexpr int GS = LPG * kQLane;
   if (MODE == 0) pdl_trigger();   // (the GEMM behind it may start)
-  if (MODE == 2) {   // launched so that it starts under the end of the GEMM in front of it
+  if (MODE >= 2) {   // launched so that it starts under the end of the kernel in front of it
     x = pdl_wait(x);
+    pdl_fresh(aux); pdl_fresh(row_index); pdl_fresh(given_scale);
     pdl_trigger();
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1007,7 +1008,7 @@ static int launch_grouped_t(const T* x, int64_t rows, int64_t K, int64_t ldx, in
   dim3 grid((unsigned)row_blocks, (unsigned)((nseg + spb - 1) / spb));
   I4TC_REQUIRE(grid.y <= 65535, I4TC_EINVAL, "K=%lld too large for the grouped quantiser", (long long)K);
 #define I4TC_LAUNCH_G(LPG)                                                                             \
-  I4TC_CUDA(launch_kernel(MODE == 2, quant_grouped_kernel<T, LPG, MODE, GIVEN>, grid, quant_rows<MODE>() * 32, 0, st, x, rows, (int)K, \
+  I4TC_CUDA(launch_kernel(MODE >= 2, quant_grouped_kernel<T, LPG, MODE, GIVEN>, grid, quant_rows<MODE>() * 32, 0, st, x, rows, (int)K, \
                           ldx, row_index, index_div, src_rows, given, packed, scale, role, spb, static_cast<const T*>(aux), eps,     \
                           QuantOutMap{nullptr, nullptr, 0, 0, 0, 0, nullptr, 1, 0, 0}))
   switch (gs) {

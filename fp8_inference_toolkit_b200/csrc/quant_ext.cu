@@ -358,6 +358,7 @@ template <typename T, int NCH>
 __global__ void __launch_bounds__(256) quant_int8_row_kernel(const T* __restrict__ x, int K, int64_t ldx, int8_t* __restrict__ q,
                                                              float* __restrict__ scale) {
   __shared__ float s_max[8];
+  pdl_trigger();
   const int64_t r = blockIdx.x;
   const T* src = x + r * ldx;
   int8_t* dst = q + r * (int64_t)K;

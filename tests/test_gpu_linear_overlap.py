@@ -99,3 +99,37 @@ def test_asymmetric_back_to_back(M, K, N, smooth):
     for i, out in enumerate(got):
         assert torch.equal(out, want[i % 4])
     ops.check_status()
+
+
+@pytest.mark.parametrize("M,K,N", [(40, 2048, 1000), (100, 4096, 1024), (300, 4096, 4096), (1000, 2048, 3001)])
+def test_weights_written_in_front(M, K, N):
+    """The GEMM entry points start under the kernel in front of them as well, which may have written the weights."""
+    from fp8_inference_toolkit_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    x = torch.randn(M, K, device="cuda", generator=gen).to(torch.bfloat16)
+    ws = [(torch.randn(N, K, device="cuda", generator=gen) * 0.02).to(torch.bfloat16) for _ in range(3)]
+    xp, xs = ops.dynamic_int4_quant_grouped(x, 128)
+    x8, x8s = ops.dynamic_int8_quant(x)
+
+    def grouped(w):
+        out = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+        p, s = ops.static_int4_weight_quant_grouped(w, 128)
+        ops.cutlass_int4_fused_grouped_gemm(xp, p, xs, s, out, M, N, 128, K // 128)
+        return out
+
+    def int8(w):   # (the int8 rows of the weight stand for the unpacked codes)
+        out = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+        q, s = ops.dynamic_int8_quant(w)
+        ops.cutlass_w4a8_scaled_mm(x8, q, x8s, s, out, M, N, K)
+        return out
+
+    for run in (grouped, int8):
+        want = []
+        for w in ws:
+            want.append(run(w))
+            torch.cuda.synchronize()
+        got = [run(ws[i % 3]) for i in range(12)]   # the packed weights of a call take the memory of the ones before
+        for i, out in enumerate(got):
+            assert torch.equal(out, want[i % 3])
+    ops.check_status()
