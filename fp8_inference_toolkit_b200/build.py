@@ -16,7 +16,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(CSRC, "libint4tc_b200.so")
 SOURCES = ["runtime.cu", "quant.cu", "quant_ext.cu", "gemm_kernel.cu", "gemm_f8.cu", "gemm_host.cu", "gemv.cu", "skinny.cu", "moe_skinny.cu", "moe.cu", "model.cu"]
-HEADERS = ["common.cuh", "gemm.cuh", "gemm_dev.cuh", "ptx.cuh", os.path.join("..", "..", "include", "int4tc_b200.h")]
+HEADERS = ["common.cuh", "gemm.cuh", "gemm_dev.cuh", "quant_codes.cuh", "ptx.cuh", os.path.join("..", "..", "include", "int4tc_b200.h")]
 
 
 def _nvcc() -> str:

@@ -457,12 +457,38 @@ extern "C" int i4tc_gemm_grouped_scratch(const uint8_t* a, const uint8_t* b, con
                                    scratch_bytes, false, device, stream);
 }
 
+// One or two bf16 tokens against per-group scales, where the CUDA-core kernel is the one chosen (run_dense) and its 16-byte loads
+// suit: it quantises the tokens as well.  A second launch costs the host and the device more than every block's own pass over a few
+// thousand elements: [1, 4096] x [6144, 4096] 23.9 -> 20.3 us a call.  Everything else, refused calls among them, takes
+// the two kernels.  (An output that overlaps the activations does too: blocks here end at different times.)
+static bool linear_in_one_kernel(const void* x, int dtype, int64_t M, int64_t K, int64_t ldx, const uint8_t* w, const float* w_scale,
+                                 const uint8_t* x_packed, const float* x_scale, const void* out, int64_t N) {
+  if (dtype != I4TC_BF16 || M < 1 || M > 2 || K <= 0 || K % 128 != 0 || K / 128 > 512 || ldx < K || ldx % 8 != 0) return false;
+  if (N <= 0 || N >= (1ll << 31) - 256 || !gemv_applicable(M, N, K, EPI_GROUP)) return false;
+  if (!x || !w || !w_scale || !x_packed || !x_scale || !out) return false;
+  if (!aligned_to(x, 16) || !aligned_to(w, 16) || !aligned_to(x_packed, 16)) return false;
+  const int path = g_small_m_path.load();
+  if ((path != 0 && path != 1) || g_force_bn != 0 || g_force_swap >= 0 || g_force_splits != 0) return false;
+  const uintptr_t x0 = reinterpret_cast<uintptr_t>(x), o0 = reinterpret_cast<uintptr_t>(out);
+  return o0 >= x0 + (uintptr_t)(ldx * (M - 1) + K) * 2 || o0 + (uintptr_t)(M * N) * 2 <= x0;
+}
+
 extern "C" int i4tc_linear(const void* x, int dtype, int64_t M, int64_t K, int64_t ldx, const uint8_t* w, const float* w_scale,
                            int per_channel, uint8_t* x_packed, float* x_scale, void* out, int64_t N, void* scratch,
                            int64_t scratch_bytes, int device, void* stream) {
   if (per_channel) {
     if (int rc = i4tc_quant_rowwise(x, dtype, M, K, ldx, x_packed, x_scale, I4TC_ROLE_ACTIVATION, device, stream)) return rc;
     return gemm_scaled_impl(x_packed, w, x_scale, w_scale, out, I4TC_BF16, M, N, K, true, device, stream);
+  }
+  if (linear_in_one_kernel(x, dtype, M, K, ldx, w, w_scale, x_packed, x_scale, out, N)) {
+    const DeviceInfo* info;
+    if (int rc = device_info(device, &info)) return rc;
+    I4TC_REQUIRE(info->cc_major == 10, I4TC_EDEVICE, "device %d is sm_%d%d; this library needs sm_100", device, info->cc_major,
+                 info->cc_minor);
+    DeviceGuard guard(device);
+    I4TC_CUDA(guard.err);
+    return launch_w4a4_gemv_quant(x, ldx, x_packed, x_scale, w, w_scale, out, M, N, (int)(K / 128), info->sm_count,
+                                  static_cast<cudaStream_t>(stream));
   }
   if (int rc = i4tc_quant_grouped(x, dtype, M, K, ldx, 128, x_packed, x_scale, I4TC_ROLE_ACTIVATION, device, stream)) return rc;
   return gemm_grouped_scratch_impl(x_packed, w, x_scale, w_scale, nullptr, nullptr, out, M, N, 128, K / 128, scratch,

@@ -11,6 +11,7 @@
 // partial results are added in ascending range order through shared memory (int32 for per-channel
 // scales: exact; fp32 for per-group scales: a fixed order, so the result is deterministic).
 #include "gemm.cuh"
+#include "quant_codes.cuh"
 #include "ptx.cuh"
 
 namespace i4tc {
@@ -36,10 +37,44 @@ struct GemvParams {
   long long x_row, x_grp;   // byte strides of the activations: token, K group
   long long w_row, w_grp;   // byte strides of the weights: row, K group
   int out_fp16;
+  const __nv_bfloat16* xf;  // QX: the activations themselves, row stride ldx
+  long long ldx;
+  uint8_t* xq;              // QX: where their codes (strides as x) and scales go
+  float* sxq;
 };
 
+// QX: the tokens are quantised here.  Every block does all of it -- a few thousand elements, sixteen lanes to a group, against a
+// launch of its own for the quantiser -- and block 0 writes codes and scales out.  Only where M == MT.
+template <int MT>
+__device__ __forceinline__ void quantise_tokens(const GemvParams& p, const __nv_bfloat16* xf, uint8_t* act, float* sx_s) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5, l = lane & 15, n = p.G * MT;
+#pragma unroll 2
+  for (int i0 = warp * 2; i0 < n; i0 += nwarps * 2) {
+    const int i = i0 + (lane >> 4), m = i % MT, g = i / MT;
+    const bool ok = i < n;
+    Vec8<__nv_bfloat16> v;
+    if (ok) v.load(xf + (long long)m * p.ldx + g * 128 + l * 8);
+    else v.zero();
+    float absmax = v.absmax();
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) absmax = fmaxf(absmax, __shfl_xor_sync(0xffffffffu, absmax, o));
+    const float s = __fdiv_rn(absmax, 7.0f);
+    const uint32_t w = AbsmaxCodes<__nv_bfloat16>(absmax, s).word(v);
+    if (!ok) continue;
+    uint32_t* dst = reinterpret_cast<uint32_t*>(act + (size_t)i * 128 + (l >> 2) * 32) + (l & 3);
+    dst[0] = (w << 4) & 0xF0F0F0F0u;
+    dst[4] = w & 0xF0F0F0F0u;
+    const float sc = scale_out(absmax, s, I4TC_ROLE_ACTIVATION);
+    if (l == 0) sx_s[i] = sc * (1.0f / 256.0f);
+    if (blockIdx.x == 0) {
+      *reinterpret_cast<uint32_t*>(p.xq + (long long)m * p.x_row + (long long)g * p.x_grp + l * 4) = w;
+      if (l == 0) p.sxq[(long long)g * MT + m] = sc;
+    }
+  }
+}
+
 // MT: tokens handled (M <= MT).  PER_GROUP: fp32 scaling after every K group, else one int32 sum per row.
-template <int MT, bool PER_GROUP>
+template <int MT, bool PER_GROUP, bool QX = false>
 __global__ void __launch_bounds__(512) w4a4_gemv_kernel(const GemvParams p) {
   extern __shared__ __align__(16) uint8_t smem[];
   // layout: expanded activations [G][MT][128] | group scales of the tokens [G][MT] | partials [warps][MT][32]
@@ -53,8 +88,16 @@ __global__ void __launch_bounds__(512) w4a4_gemv_kernel(const GemvParams p) {
   const int gper = (p.G + nwarps - 1) / nwarps;
   const int g0 = min(p.G, warp * gper), g1 = min(p.G, g0 + gper);
 
+  const uint8_t* w = p.w;
+  const float* sw = p.sw;
+  const __nv_bfloat16* xf = p.xf;
+  if (QX) {   // (behind any kernel: nothing is read before the wait)
+    pdl_wait();
+    pdl_fresh(w); pdl_fresh(sw); pdl_fresh(xf);
+    pdl_trigger();
+  }
   // the first weight group is requested before the activations are staged
-  const uint8_t* wrow = p.w + (long long)(n_ok ? n : 0) * p.w_row;
+  const uint8_t* wrow = w + (long long)(n_ok ? n : 0) * p.w_row;
   uint4 wv[4];
   if (g0 < g1) {
     const uint4* src = reinterpret_cast<const uint4*>(wrow + (long long)g0 * p.w_grp);
@@ -64,9 +107,10 @@ __global__ void __launch_bounds__(512) w4a4_gemv_kernel(const GemvParams p) {
 
   const uint8_t* x = p.x;
   const float* sx = p.sx;
-  pdl_wait(x, sx);
+  if (QX) quantise_tokens<MT>(p, xf, act, sx_s);
+  else pdl_wait(x, sx);
   // ---- stage the tokens: packed 16-byte chunk -> 16 bytes of even codes, 16 bytes of odd codes ----
-  for (int i = threadIdx.x; i < p.G * MT * 4; i += blockDim.x) {
+  for (int i = threadIdx.x; !QX && i < p.G * MT * 4; i += blockDim.x) {
     const int j = i & 3, m = (i >> 2) % MT, g = (i >> 2) / MT;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     if (m < p.M) v = __ldg(reinterpret_cast<const uint4*>(x + (long long)m * p.x_row + (long long)g * p.x_grp) + j);
@@ -76,7 +120,7 @@ __global__ void __launch_bounds__(512) w4a4_gemv_kernel(const GemvParams p) {
     dst[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
     dst[1] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
   }
-  if (PER_GROUP) {
+  if (PER_GROUP && !QX) {
     for (int i = threadIdx.x; i < p.G * MT; i += blockDim.x) {
       const int m = i % MT, g = i / MT;
       sx_s[i] = (m < p.M) ? __ldg(sx + (long long)g * p.M + m) * (1.0f / 256.0f) : 0.f;
@@ -100,7 +144,7 @@ __global__ void __launch_bounds__(512) w4a4_gemv_kernel(const GemvParams p) {
     }
     float swv = 0.f;
     if (PER_GROUP) {
-      swv = n_ok ? __ldg(p.sw + (long long)g * p.N + n) : 0.f;
+      swv = n_ok ? __ldg(sw + (long long)g * p.N + n) : 0.f;
 #pragma unroll
       for (int m = 0; m < MT; ++m) acc[m] = 0;
     }
@@ -160,7 +204,7 @@ __global__ void __launch_bounds__(512) w4a4_gemv_kernel(const GemvParams p) {
         for (int mm = 0; mm < MT; ++mm) if (mm == m) s = acc[mm];
       }
       // reference order: (acc * scale_b[n]) * scale_a[m]
-      const float sb = n_ok ? __ldg(p.sw + n) : 0.f;
+      const float sb = n_ok ? __ldg(sw + n) : 0.f;
       v = (__int2float_rn(s) * (sb * (1.0f / 256.0f))) * __ldg(sx + m);
     }
     if (n_ok) {
@@ -170,17 +214,17 @@ __global__ void __launch_bounds__(512) w4a4_gemv_kernel(const GemvParams p) {
   }
 }
 
-template <int MT, bool PER_GROUP>
+template <int MT, bool PER_GROUP, bool QX = false>
 int launch_mt(const GemvParams& p, int warps, size_t smem, bool overlap, cudaStream_t st) {
   static bool configured[64] = {false};
   int dev = 0;
   I4TC_CUDA(cudaGetDevice(&dev));
   if (dev < 64 && !configured[dev]) {
-    I4TC_CUDA(cudaFuncSetAttribute(w4a4_gemv_kernel<MT, PER_GROUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    I4TC_CUDA(cudaFuncSetAttribute(w4a4_gemv_kernel<MT, PER_GROUP, QX>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     configured[dev] = true;
   }
   const int grid = (p.N + kRows - 1) / kRows;
-  I4TC_CUDA(launch_kernel(overlap, w4a4_gemv_kernel<MT, PER_GROUP>, dim3((unsigned)grid), (unsigned)warps * 32, smem, st, p));
+  I4TC_CUDA(launch_kernel(overlap, w4a4_gemv_kernel<MT, PER_GROUP, QX>, dim3((unsigned)grid), (unsigned)warps * 32, smem, st, p));
   return I4TC_OK;
 }
 
@@ -196,6 +240,27 @@ bool gemv_applicable(long long M, long long N, long long K, int epi_mode) {
   return need <= 200 * 1024;
 }
 
+static int gemv_warps(long long N, int G, int sm_count) {
+  // enough warps to keep the memory system busy: aim for >= 16 warps per SM over the whole grid
+  const long long blocks = (N + kRows - 1) / kRows;
+  int warps = (int)((16ll * sm_count + blocks - 1) / blocks);
+  warps = warps < 2 ? 2 : warps > 16 ? 16 : warps;
+  return warps > G ? G : warps;
+}
+
+int launch_w4a4_gemv_quant(const void* x, long long ldx, uint8_t* x_packed, float* x_scale, const uint8_t* w, const float* sw, void* out,
+                           long long M, long long N, int G, int sm_count, cudaStream_t st) {
+  GemvParams p;
+  p.x = nullptr; p.w = w; p.sx = nullptr; p.sw = sw; p.out = out;
+  p.M = (int)M; p.N = (int)N; p.G = G;
+  p.x_row = p.w_row = 64; p.x_grp = M * 64; p.w_grp = N * 64;
+  p.out_fp16 = 0;
+  p.xf = static_cast<const __nv_bfloat16*>(x); p.ldx = ldx; p.xq = x_packed; p.sxq = x_scale;
+  const int warps = gemv_warps(N, G, sm_count);
+  const size_t smem = (size_t)G * M * (128 + 4) + (size_t)warps * M * kRows * 4;
+  return M == 1 ? launch_mt<1, true, true>(p, warps, smem, true, st) : launch_mt<2, true, true>(p, warps, smem, true, st);
+}
+
 int launch_w4a4_gemv(const uint8_t* x, const uint8_t* w, const float* sx, const float* sw, void* out, int out_dtype,
                      long long M, long long N, int G, bool rowmajor, int epi_mode, int sm_count, bool overlap, cudaStream_t st) {
   GemvParams p;
@@ -207,13 +272,10 @@ int launch_w4a4_gemv(const uint8_t* x, const uint8_t* w, const float* sx, const 
     p.x_row = p.w_row = 64; p.x_grp = M * 64; p.w_grp = N * 64;
   }
   p.out_fp16 = out_dtype == I4TC_FP16;
+  p.xf = nullptr; p.ldx = 0; p.xq = nullptr; p.sxq = nullptr;
   I4TC_REQUIRE(aligned_to(x, 16) && aligned_to(w, 16), I4TC_EALIGN, "packed operands must be 16-byte aligned");
   const int mt = M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16;
-  // enough warps to keep the memory system busy: aim for >= 16 warps per SM over the whole grid
-  const long long blocks = (N + kRows - 1) / kRows;
-  int warps = (int)((16ll * sm_count + blocks - 1) / blocks);
-  warps = warps < 2 ? 2 : warps > 16 ? 16 : warps;
-  if (warps > G) warps = G;
+  const int warps = gemv_warps(N, G, sm_count);
   const bool pg = epi_mode == EPI_GROUP;
   const size_t smem = (size_t)G * mt * 128 + (pg ? (size_t)G * mt * 4 : 0) + (size_t)warps * mt * kRows * 4;
 #define I4TC_GEMV_CASE(MT_)                                                        \
