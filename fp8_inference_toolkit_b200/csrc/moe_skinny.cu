@@ -179,10 +179,21 @@ __global__ void __launch_bounds__(kMoeWarps * 32, BLOCKS) moe_skinny_kernel(cons
   }
 }
 
+constexpr size_t kMoeSkinnyMaxSmem = 110 * 1024;
+
 template <int NT, int DEPTH, int BLOCKS>
 int launch_nt(const MoeSkinnyParams& p, int num_experts, cudaStream_t st) {
+  // The limit belongs to the function, not to a launch, so it is the most that moe_skinny_applicable admits: with each call's own
+  // size, a thread with fewer groups could lower it between another thread's setting and its launch.
+  static bool configured[64] = {false};
+  int dev = 0;
+  I4TC_CUDA(cudaGetDevice(&dev));
+  if (dev >= 64 || !configured[dev]) {
+    I4TC_CUDA(cudaFuncSetAttribute(moe_skinny_kernel<NT, DEPTH, BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)kMoeSkinnyMaxSmem));
+    if (dev < 64) configured[dev] = true;
+  }
   const size_t smem = moe_skinny_smem(p.G, 8 * NT);
-  I4TC_CUDA(cudaFuncSetAttribute(moe_skinny_kernel<NT, DEPTH, BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int blocks = (p.N + 16 * kMoeWarps - 1) / (16 * kMoeWarps);
   I4TC_CUDA(launch_kernel(true, moe_skinny_kernel<NT, DEPTH, BLOCKS>, dim3((unsigned)blocks, (unsigned)num_experts), kMoeWarps * 32, smem,
                           st, p));
@@ -199,7 +210,7 @@ static int nt_for(long long num_pairs, long long num_experts) {
 
 bool moe_skinny_applicable(long long num_pairs, long long N, int G, long long num_experts) {
   return num_pairs <= 26 * num_experts && N % 16 == 0 && num_experts <= 65535 &&
-         moe_skinny_smem(G, 8 * nt_for(num_pairs, num_experts)) <= 110 * 1024;
+         moe_skinny_smem(G, 8 * nt_for(num_pairs, num_experts)) <= kMoeSkinnyMaxSmem;
 }
 
 int launch_moe_skinny(const uint8_t* a, const float* sa, const uint8_t* b, const float* sb, const int32_t* offsets, void* out,

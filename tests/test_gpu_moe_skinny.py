@@ -1,6 +1,8 @@
 """GPU: the weight-streaming form of the grouped MoE GEMM gives the tile kernel's bits at the edges of its row tiles (8, 16 and 32
 rows at once, experts without rows, experts that take several passes), of its blocks (N below, at and past 128 rows) and of its
-pipeline (fewer groups than it keeps in flight, odd counts)."""
+pipeline (fewer groups than it keeps in flight, odd counts), and from several threads."""
+import threading
+
 import pytest
 import torch
 
@@ -36,4 +38,39 @@ def test_same_bits_as_the_tile_kernel(E, counts, N, G):
         outs.append(out)
     assert not outs[0].isnan().any()
     assert torch.equal(outs[0], outs[1])
+    ops.check_status()
+
+
+def test_threads_with_other_group_counts():
+    """The kernel's shared-memory limit belongs to the function: a call with few groups must not lower it under a thread that is about
+    to launch with many (such a launch is refused)."""
+    from fp8_inference_toolkit_b200 import moe, ops
+
+    E, P, N = 4, 80, 128
+    off = torch.tensor([0, 20, 40, 60, 80], dtype=torch.int32, device="cuda")
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    jobs, codes = [], []
+    for G in (1, 24, 1, 24):     # 4 KB and 101 KB of shared memory at 32 rows at once
+        a = torch.randint(0, 256, (G, P, 64), dtype=torch.uint8, device="cuda", generator=gen)
+        b = torch.randint(0, 256, (E, G, N, 64), dtype=torch.uint8, device="cuda", generator=gen)
+        sa, sb = torch.rand(G, P, device="cuda", generator=gen), torch.rand(E, G, N, device="cuda", generator=gen)
+        want = torch.empty(P, N, dtype=torch.bfloat16, device="cuda")
+        moe.moe_w4a4_grouped_gemm(a, sa, b, sb, off, want, N, G, E)
+        out, stream = torch.empty_like(want), torch.cuda.Stream()
+        jobs.append((a, sa, b, sb, G, want, out, stream))
+    torch.cuda.synchronize()
+
+    def work(a, sa, b, sb, G, want, out, stream):   # nothing but library calls, which run beside each other
+        args = (a.data_ptr(), sa.data_ptr(), b.data_ptr(), sb.data_ptr(), off.data_ptr(), out.data_ptr(), P, N, G, E, 0, stream.cuda_stream)
+        codes.append({ops.lib.i4tc_moe_grouped_gemm(*args) for _ in range(20000)})
+
+    threads = [threading.Thread(target=work, args=j) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert codes == [{0}] * len(jobs)
+    for j in jobs:
+        assert torch.equal(j[6], j[5])
     ops.check_status()
