@@ -98,6 +98,7 @@ int launch_w4a4_group_f8(const GemmParams& p, const uint8_t* a, const uint8_t* b
 // x / w are the packed operands in either layout (rowmajor: [rows, G * 64]; else [G, rows, 64]).
 bool gemv_applicable(long long M, long long N, long long K, int epi_mode);
 // One or two bf16 tokens quantised inside the kernel (per group of 128; codes and scales are written too); bf16 out.
+bool gemv_quant_pays(long long M, long long N, int G, int sm_count);
 int launch_w4a4_gemv_quant(const void* x, long long ldx, uint8_t* x_packed, float* x_scale, const uint8_t* w, const float* sw, void* out,
                            long long M, long long N, int G, int sm_count, cudaStream_t st);
 int launch_w4a4_gemv(const uint8_t* x, const uint8_t* w, const float* sx, const float* sw, void* out, int out_dtype,

@@ -458,9 +458,9 @@ extern "C" int i4tc_gemm_grouped_scratch(const uint8_t* a, const uint8_t* b, con
 }
 
 // One or two bf16 tokens against per-group scales, where the CUDA-core kernel is the one chosen (run_dense) and its 16-byte loads
-// suit: it quantises the tokens as well.  A second launch costs the host and the device more than every block's own pass over a few
-// thousand elements: [1, 4096] x [6144, 4096] 23.9 -> 20.3 us a call.  Everything else, refused calls among them, takes
-// the two kernels.  (An output that overlaps the activations does too: blocks here end at different times.)
+// suit: it quantises the tokens as well, where that pays (gemv_quant_pays).  A second launch costs the host and the device more than
+// every block's own pass over a few thousand elements: [1, 4096] x [6144, 4096] 23.9 -> 20.3 us a call.  Everything else, refused calls
+// among them, takes the two kernels.  (An output that overlaps the activations does too: blocks here end at different times.)
 static bool linear_in_one_kernel(const void* x, int dtype, int64_t M, int64_t K, int64_t ldx, const uint8_t* w, const float* w_scale,
                                  const uint8_t* x_packed, const float* x_scale, const void* out, int64_t N) {
   if (dtype != I4TC_BF16 || M < 1 || M > 2 || K <= 0 || K % 128 != 0 || K / 128 > 512 || ldx < K || ldx % 8 != 0) return false;
@@ -485,10 +485,12 @@ extern "C" int i4tc_linear(const void* x, int dtype, int64_t M, int64_t K, int64
     if (int rc = device_info(device, &info)) return rc;
     I4TC_REQUIRE(info->cc_major == 10, I4TC_EDEVICE, "device %d is sm_%d%d; this library needs sm_100", device, info->cc_major,
                  info->cc_minor);
-    DeviceGuard guard(device);
-    I4TC_CUDA(guard.err);
-    return launch_w4a4_gemv_quant(x, ldx, x_packed, x_scale, w, w_scale, out, M, N, (int)(K / 128), info->sm_count,
-                                  static_cast<cudaStream_t>(stream));
+    if (gemv_quant_pays(M, N, (int)(K / 128), info->sm_count)) {
+      DeviceGuard guard(device);
+      I4TC_CUDA(guard.err);
+      return launch_w4a4_gemv_quant(x, ldx, x_packed, x_scale, w, w_scale, out, M, N, (int)(K / 128), info->sm_count,
+                                    static_cast<cudaStream_t>(stream));
+    }
   }
   if (int rc = i4tc_quant_grouped(x, dtype, M, K, ldx, 128, x_packed, x_scale, I4TC_ROLE_ACTIVATION, device, stream)) return rc;
   return gemm_grouped_scratch_impl(x_packed, w, x_scale, w_scale, nullptr, nullptr, out, M, N, 128, K / 128, scratch,

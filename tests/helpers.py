@@ -8,6 +8,26 @@ REL_TOL = 1e-2      # bf16 outputs: max relative error (reference bar, test_corr
 COS_TOL = 0.9999    # bf16 outputs: flat cosine (reference bar, test_v5_correctness.py:50)
 
 
+def launches(fn) -> int:
+    """Kernels that fn() launches, counted in a captured graph."""
+    from cuda.bindings import runtime as rt
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        fn()
+    side.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=side):
+        fn()
+    raw = rt.cudaGraph_t(graph.raw_cuda_graph())
+    err, _, count = rt.cudaGraphGetNodes(raw)
+    assert err == rt.cudaError_t.cudaSuccess
+    err, nodes, _ = rt.cudaGraphGetNodes(raw, count)
+    assert err == rt.cudaError_t.cudaSuccess
+    return sum(rt.cudaGraphNodeGetType(n)[1] == rt.cudaGraphNodeType.cudaGraphNodeTypeKernel for n in nodes)
+
+
 def dev_packed(codes: np.ndarray) -> torch.Tensor:
     return torch.from_numpy(O.pack_int4(codes)).cuda()
 

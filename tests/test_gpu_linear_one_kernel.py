@@ -59,3 +59,18 @@ def test_output_over_the_activations():
     ops.check(ops.lib.i4tc_linear(x.data_ptr(), ops._DTYPES[x.dtype], 1, K, K, wp.data_ptr(), ws.data_ptr(), 0, p.data_ptr(), s.data_ptr(),
                                   x.data_ptr(), N, None, 0, 0, torch.cuda.current_stream().cuda_stream), "linear")
     assert torch.equal(x, want)
+
+
+@pytest.mark.parametrize("M,K,N,want", [
+    (1, 4096, 6144, 1), (2, 4096, 6144, 1), (1, 1024, 65536, 1), (2, 12288, 4096, 1),     # little to quantise in a block and an SM
+    (1, 4096, 24576, 2), (2, 12288, 16000, 2), (2, 16384, 4096, 2), (1, 65408, 8192, 2),   # it would cost more than a launch
+])
+def test_where_it_pays(M, K, N, want):
+    from fp8_inference_toolkit_b200 import ops
+    from tests.helpers import launches
+
+    gen = torch.Generator(device="cuda").manual_seed(K)
+    wp = torch.randint(0, 256, (K // 128, N, 64), dtype=torch.uint8, device="cuda", generator=gen)
+    ws = torch.rand(K // 128, N, device="cuda", generator=gen)
+    x = torch.randn(M, K, device="cuda", generator=gen).to(torch.bfloat16)
+    assert launches(lambda: ops.linear(x, wp, ws, N, False)) == want
