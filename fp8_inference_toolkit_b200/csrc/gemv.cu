@@ -252,12 +252,12 @@ static int gemv_warps(long long N, int G, int sm_count) {
 // It costs a warp 0.5 us for every step of two groups, or 0.03 us for every step that an SM does over all of its blocks.
 // The lines are where it is no slower than the two kernels one after the other, without overlap ([M, K] x [N, K], captured, two | one): by
 // steps of a warp, [2, 12288] x [4096] 11.4 | 10.6 us at 6, [2, 16384] x [4096] 12.6 | 13.4 at 8, [2, 32768] x [1000] 20.5 | 24.2 at 16;
-// by those of an SM, [1, 1024] x [65536] 10.0 | 8.6 at 55, [1, 4096] x [24576] 13.9 | 15.2 at 83 (12.0 overlapped), [2, 12288] x [32768]
-// 51 | 71 at 664.
+// by those of an SM, [1, 4096] x [12288] 10.1 | 9.0 at 42, [1, 4096] x [16001] 11.8 | 12.8 at 54, [1, 4096] x [24576] 13.9 | 15.2 at 83
+// (12.0 overlapped), [2, 12288] x [32768] 51 | 71 at 664.
 bool gemv_quant_pays(long long M, long long N, int G, int sm_count) {
   const long long blocks = (N + kRows - 1) / kRows, steps = (G * M + 1) / 2;
   const int warps = gemv_warps(N, G, sm_count);
-  return steps <= 6 * warps && (blocks <= sm_count || blocks * steps <= 56ll * sm_count);
+  return steps <= 6 * warps && (blocks <= sm_count || blocks * steps <= 48ll * sm_count);
 }
 
 int launch_w4a4_gemv_quant(const void* x, long long ldx, uint8_t* x_packed, float* x_scale, const uint8_t* w, const float* sw, void* out,

@@ -62,8 +62,8 @@ def test_output_over_the_activations():
 
 
 @pytest.mark.parametrize("M,K,N,want", [
-    (1, 4096, 6144, 1), (2, 4096, 6144, 1), (1, 1024, 65536, 1), (2, 12288, 4096, 1),     # little to quantise in a block and an SM
-    (1, 4096, 24576, 2), (2, 12288, 16000, 2), (2, 16384, 4096, 2), (1, 65408, 8192, 2),   # it would cost more than a launch
+    (1, 4096, 6144, 1), (2, 4096, 6144, 1), (1, 4096, 12288, 1), (2, 12288, 4096, 1),     # little to quantise in a block and an SM
+    (1, 4096, 16001, 2), (1, 4096, 24576, 2), (2, 12288, 16000, 2), (2, 16384, 4096, 2), (1, 65408, 8192, 2),   # it would cost more than a launch
 ])
 def test_where_it_pays(M, K, N, want):
     from fp8_inference_toolkit_b200 import ops
