@@ -287,6 +287,10 @@ int launch_w4a4_gemv(const uint8_t* x, const uint8_t* w, const float* sx, const 
   p.xf = nullptr; p.ldx = 0; p.xq = nullptr; p.sxq = nullptr;
   I4TC_REQUIRE(aligned_to(x, 16) && aligned_to(w, 16), I4TC_EALIGN, "packed operands must be 16-byte aligned");
   const int mt = M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16;
+  // Blocks that start beside the quantiser's spread unevenly over the SMs.  For one or two tokens and many groups that costs more
+  // than the overlap gives ([1, 65408] x [8192, 65408] 67.9 us without, 80.4 with; flushed L2, [1, 32768] x [16000] 83 and 93,
+  // [2, 32768] x [4096] 33.8 and 37.9; but [1, 16384] x [16000] 32.1 and 29.6, [3, 32768] x [4097] 37.9 and 33.8).
+  if (M <= 2 && epi_mode == EPI_GROUP && G > 128) overlap = false;
   const int warps = gemv_warps(N, G, sm_count);
   const bool pg = epi_mode == EPI_GROUP;
   const size_t smem = (size_t)G * mt * 128 + (pg ? (size_t)G * mt * 4 : 0) + (size_t)warps * mt * kRows * 4;
