@@ -5,6 +5,7 @@
 // fp32 copies (norm: convert, square, mean, scale, convert back, weight; rotary: four products, two sums, a cat), 20-odd
 // launches per layer.
 #include "common.cuh"
+#include <type_traits>
 
 namespace i4tc {
 
@@ -72,8 +73,8 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_kernel(const __nv_bfloat
 }
 
 // Heads [0, q_heads) with wq and [q_heads, heads) with wk of every token of qkv (row stride ld, heads of 128):
-// normalise, then rotate halves by the token's position (token % seq), in place.  A block takes a token and a warp two heads at a
-// time, a lane eight consecutive elements of one; the other half of the rotation is 8 lanes away.  Tables and weights stay in
+// normalise, then rotate halves by the token's position (token % seq), in place.  A block takes a token (several, where a warp or two
+// hold all heads; few tokens are shared by several blocks) and a warp two heads at a time, a lane eight consecutive elements of one; the other half of the rotation is 8 lanes away.  Tables and weights stay in
 // registers over the heads.  Every bf16 rounding of the separate ops is kept, so results differ from theirs by the order of the sum of
 // squares only (four-element chains, then partners 64, 32, 16, 8 and 4 elements away).
 // A warp per head with 8-byte accesses, an index division per head and single conversions was bound by the special-function unit:
@@ -97,15 +98,20 @@ __device__ __forceinline__ void store_oct(__nv_bfloat16* p, const uint4& v) {
   }
 }
 
-template <bool A16>
-__global__ void __launch_bounds__(kRopeWarps * 32) qk_norm_rope_kernel(__nv_bfloat16* qkv, long long ld, int q_heads, int heads, int seq,
+// WPT: warps of a block that work on the same token.  SPLIT: the block rows of the grid share a token's heads.
+template <bool A16, int WPT, bool SPLIT>
+__global__ void __launch_bounds__(kRopeWarps * 32) qk_norm_rope_kernel(__nv_bfloat16* qkv, unsigned tokens, long long ld,
+                                                                       int q_heads, int heads, int seq,
                                                                        const __nv_bfloat16* wq, const __nv_bfloat16* wk,
                                                                        const __nv_bfloat16* cos_t, const __nv_bfloat16* sin_t,
                                                                        float eps) {
   pdl_wait();
   pdl_fresh(qkv); pdl_fresh(wq); pdl_fresh(wk); pdl_fresh(cos_t); pdl_fresh(sin_t);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l = lane & 15;
-  const unsigned tok = blockIdx.x;
+  const int lane = threadIdx.x & 31, l = lane & 15;
+  const int warps = SPLIT ? (int)gridDim.y * WPT : WPT;   // of the token, and this one among them
+  const int warp = (int)(threadIdx.x >> 5) % WPT + (SPLIT ? (int)blockIdx.y * WPT : 0);
+  const unsigned tok = blockIdx.x * (kRopeWarps / WPT) + threadIdx.x / (32 * WPT);
+  if (WPT < kRopeWarps && tok >= tokens) return;   // whole warps
   __nv_bfloat16* at = qkv + (long long)tok * ld + l * 8;
   const long long row = (long long)(tok % (unsigned)seq) * 64 + (l & 7) * 8;   // tables [seq, 64]
   const uint4 cu = load_oct<A16>(cos_t + row), su = load_oct<A16>(sin_t + row);
@@ -115,9 +121,9 @@ __global__ void __launch_bounds__(kRopeWarps * 32) qk_norm_rope_kernel(__nv_bflo
   int h = warp * 2 + (lane >> 4);
   uint4 cur = make_uint4(0u, 0u, 0u, 0u);
   if (h < heads) cur = load_oct<A16>(at + (long long)h * 128);
-  for (int h0 = warp * 2; h0 < heads; h0 += kRopeWarps * 2, h += kRopeWarps * 2) {   // the same trips for both halves of the warp
+  for (int h0 = warp * 2; h0 < heads; h0 += warps * 2, h += warps * 2) {   // the same trips for both halves of the warp
     uint4 nxt = make_uint4(0u, 0u, 0u, 0u);
-    if (h + kRopeWarps * 2 < heads) nxt = load_oct<A16>(at + (long long)(h + kRopeWarps * 2) * 128);
+    if (h + warps * 2 < heads) nxt = load_oct<A16>(at + (long long)(h + warps * 2) * 128);
     const uint32_t u[4] = {cur.x, cur.y, cur.z, cur.w};
     float2 f[4];
     float s[2];
@@ -189,9 +195,21 @@ extern "C" int i4tc_qk_norm_rope(void* qkv, int64_t tokens, int64_t ld, int64_t 
   I4TC_CUDA(guard.err);
   const bool a16 = aligned_to(qkv, 16) && ld % 8 == 0 && aligned_to(q_weight, 16) && aligned_to(k_weight, 16) &&
                    aligned_to(cos_table, 16) && aligned_to(sin_table, 16);
-  I4TC_CUDA(launch_kernel(true, a16 ? qk_norm_rope_kernel<true> : qk_norm_rope_kernel<false>, dim3((unsigned)tokens), kRopeWarps * 32, 0,
-                          static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(qkv), ld, (int)q_heads, (int)heads, (int)seq,
-                          static_cast<const __nv_bfloat16*>(q_weight), static_cast<const __nv_bfloat16*>(k_weight),
+  // A token's heads: one warp for two, two warps for four, else a block.  [16384, 1 head] 10.0 us with three idle warps a block, 4.6 so.
+  // Up to 64 tokens do not fill the device with a block each: one for every eight heads ([1, 72 heads] 3.3 -> 1.5 us).
+  const bool split = tokens <= 64 && heads > 8;
+  const int wpt = heads <= 2 ? 1 : heads <= 4 ? 2 : kRopeWarps;
+  const dim3 grid((unsigned)((tokens * wpt + kRopeWarps - 1) / kRopeWarps), split ? (unsigned)((heads + 7) / 8) : 1u);
+  auto pick = [&](auto a) {
+    constexpr bool A16 = decltype(a)::value;
+    return split      ? qk_norm_rope_kernel<A16, kRopeWarps, true>
+           : wpt == 1 ? qk_norm_rope_kernel<A16, 1, false>
+           : wpt == 2 ? qk_norm_rope_kernel<A16, 2, false>
+                      : qk_norm_rope_kernel<A16, kRopeWarps, false>;
+  };
+  I4TC_CUDA(launch_kernel(true, a16 ? pick(std::true_type{}) : pick(std::false_type{}), grid, kRopeWarps * 32, 0,
+                          static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(qkv), (unsigned)tokens, ld, (int)q_heads,
+                          (int)heads, (int)seq, static_cast<const __nv_bfloat16*>(q_weight), static_cast<const __nv_bfloat16*>(k_weight),
                           static_cast<const __nv_bfloat16*>(cos_table), static_cast<const __nv_bfloat16*>(sin_table), eps));
   return I4TC_OK;
 }

@@ -28,6 +28,28 @@ def launches(fn) -> int:
     return sum(rt.cudaGraphNodeGetType(n)[1] == rt.cudaGraphNodeType.cudaGraphNodeTypeKernel for n in nodes)
 
 
+def device_us(fn, n: int = 20) -> float:
+    """Device time of fn() in a captured graph of n calls, the best of nine replays."""
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        fn()
+    side.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        for _ in range(n):
+            fn()
+    best = float("inf")
+    for _ in range(10):
+        start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        start.record()
+        graph.replay()
+        end.record()
+        end.synchronize()
+        best = min(best, start.elapsed_time(end) * 1e3 / n)
+    return best
+
+
 def dev_packed(codes: np.ndarray) -> torch.Tensor:
     return torch.from_numpy(O.pack_int4(codes)).cuda()
 
