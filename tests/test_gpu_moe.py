@@ -91,6 +91,25 @@ def test_combine_alone(moe):
     assert torch.equal(got.cpu(), ref.to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("k", [1, 2, 3, 5, 9])
+def test_combine_any_number_of_rows(moe, k):
+    """One, two or four rows in flight, and what is left over: one fused multiply-add per slot in ascending order, one rounding."""
+    rng = np.random.RandomState(k)
+    T, H = 19, 136
+    y = torch.from_numpy(rng.randn(T * k, H).astype(np.float32)).to(torch.bfloat16)
+    inv = torch.from_numpy(rng.permutation(T * k).astype(np.int32))
+    inv[::7] = -1
+    w = torch.from_numpy(rng.rand(T, k).astype(np.float32))
+    got = moe.moe_combine(y.cuda(), inv.cuda(), w.cuda(), T, k)
+    ref = torch.zeros(T, H, dtype=torch.float64)
+    for j in range(k):
+        rows = inv.view(T, k)[:, j].long()
+        term = w[:, j:j + 1].double() * y[rows.clamp(min=0)].double()
+        # the product is exact in 64 bits (24 + 8 bits), so is the sum but for exponents 20 apart: one rounding to fp32, as the FMA's
+        ref = (ref + torch.where((rows >= 0)[:, None], term, torch.zeros_like(term))).float().double()
+    assert torch.equal(got.cpu(), ref.to(torch.bfloat16))
+
+
 def test_gather_quant_and_silu_quant(moe):
     from fp8_inference_toolkit_b200 import synthetic
 
