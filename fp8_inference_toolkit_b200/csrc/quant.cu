@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(quant_rows<MODE>() * 32, MODE == 3 ? 8 : MODE 
 }
 
 // Tokens quantised once and written to every row that wants them: token t's codes and scales go to rows inv[t * top_k + j] of the
-// group-major [G, R, 64] / [G, R] destination (none for a negative index).  The layout of the kernel above, group size 128.
+// group-major [G, R, 64] / [G, R] destination (none for an index that is negative or past it).  The layout of the kernel above, group size 128.
 // As a quantiser and a copy of its packed rows [4096 tokens, 2048] x 8 took 6.4 + 13.8 us and two launches; here 11.4.
 __global__ void __launch_bounds__(256) quant_fanout_kernel(const __nv_bfloat16* x, int64_t rows, int K, int64_t ldx,
                                                            const int32_t* inv, int top_k, int64_t R,
@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(256) quant_fanout_kernel(const __nv_bfloat16* 
     const int mine = j0 + lane < top_k ? __ldg(inv + r * top_k + j0 + lane) : -1;
     for (int j = 0; j < min(32, top_k - j0); ++j) {
       const int64_t pos = __shfl_sync(0xffffffffu, mine, j);
-      if (pos < 0 || k >= K) continue;
+      if ((uint64_t)pos >= (uint64_t)R || k >= K) continue;
       *reinterpret_cast<uint4*>(packed + (g * R + pos) * 64 + (lane & 3) * 16) = w;
       if ((lane & 3) == 0) scale[g * R + pos] = sc;
     }

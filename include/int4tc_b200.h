@@ -279,7 +279,7 @@ int i4tc_moe_gather_quant(const void* x, int dtype, int64_t num_tokens, int64_t 
                           uint8_t* packed, float* scale, int device, void* stream);
 
 /* Every token of bf16 x quantised once (gs=128, activation role) and written to rows inv_pairs[t * top_k + j], j < top_k, of
- * packed [K/128, num_rows, 64] / scale [K/128, num_rows]; a negative index writes nothing. */
+ * packed [K/128, num_rows, 64] / scale [K/128, num_rows]; an index outside [0, num_rows) writes nothing. */
 int i4tc_moe_quant_fanout(const void* x, int64_t num_tokens, int64_t K, int64_t ldx, const int32_t* inv_pairs, int64_t top_k,
                           int64_t num_rows, uint8_t* packed, float* scale, int device, void* stream);
 

@@ -22,6 +22,25 @@ def test_same_rows_as_the_copy(T, K, top_k):
     ops.check_status()
 
 
+def test_rows_past_the_destination_are_not_written():
+    from fp8_inference_toolkit_b200 import moe, ops
+
+    T, K, R = 5, 256, 7
+    x = torch.randn(T, K, device="cuda").to(torch.bfloat16)
+    inv = torch.tensor([0, 2, 4, 7, 2 ** 31 - 1, -1, -(2 ** 31), 1, 3, 6], dtype=torch.int32, device="cuda")
+    p = torch.full((K // 128, R, 64), 0x5A, dtype=torch.uint8, device="cuda")
+    s = torch.full((K // 128, R), -1.0, device="cuda")
+    ops.check(ops.lib.i4tc_moe_quant_fanout(x.data_ptr(), T, K, K, inv.data_ptr(), 2, R, p.data_ptr(), s.data_ptr(), 0,
+                                            torch.cuda.current_stream().cuda_stream), "moe_quant_fanout")
+    want_p, want_s = ops.dynamic_int4_quant_grouped(x, 128)
+    rows = {0: 0, 2: 0, 4: 1, 1: 3, 3: 4, 6: 4}
+    for r in range(R):
+        if r in rows:
+            assert torch.equal(p[:, r], want_p[:, rows[r]]) and torch.equal(s[:, r], want_s[:, rows[r]])
+        else:
+            assert (p[:, r] == 0x5A).all() and (s[:, r] == -1.0).all()
+
+
 @pytest.mark.parametrize("T", [3, 64, 300, 700])
 def test_layers_back_to_back(T):
     """300 and 700 tokens: the register-fed and the tile kernel."""
