@@ -611,13 +611,14 @@ int launch_grouped_ext(bool asym, const void* x, int dtype, int64_t rows, int64_
 // Row-wise kernel.  One 256-thread block per row; the row is cached in registers
 // (NCH chunks of 2048 elements, 8 per thread per chunk), so HBM is read once.
 // ------------------------------------------------------------------------------------------
-template <typename T, int NCH, bool GIVEN>
+// TRIGGER: a GEMM behind it may start early.
+template <typename T, int NCH, bool GIVEN, bool TRIGGER>
 __global__ void __launch_bounds__(256) quant_rowwise_kernel(const T* __restrict__ x, int K, int64_t ldx,
                                                             const float* __restrict__ given_scale,
                                                             uint8_t* __restrict__ packed,
                                                             float* __restrict__ scale, int role) {
   __shared__ float s_max[8];
-  pdl_trigger();
+  if (TRIGGER) pdl_trigger();
   const int64_t r = blockIdx.x;
   const T* src = x + r * ldx;
   const int t = threadIdx.x;
@@ -648,6 +649,7 @@ __global__ void __launch_bounds__(256) quant_rowwise_kernel(const T* __restrict_
     absmax = s_max[0];
 #pragma unroll
     for (int i = 1; i < 8; ++i) absmax = fmaxf(absmax, s_max[i]);
+    if (t * 8 >= K) return;   // (short rows: no division in warps that have no element)
     const float s = __fdiv_rn(absmax, 7.0f);
     if (t == 0) scale[r] = scale_out(absmax, s, role);
     store(AbsmaxCodes<T>(absmax, s));
@@ -835,13 +837,16 @@ static int launch_rowwise_t(const T* x, int64_t rows, int64_t K, int64_t ldx, co
   if (!vec_ok) {
     quant_rowwise_generic_kernel<T, GIVEN><<<grid, 256, 0, st>>>(x, K, ldx, given, packed, scale, role);
   } else if (K <= 2048) {
-    quant_rowwise_kernel<T, 1, GIVEN><<<grid, 256, 0, st>>>(x, (int)K, ldx, given, packed, scale, role);
+    // A trigger in each of many short blocks costs more than a GEMM's early start gives: [8192, 128] 9.8 us with it, 7.3 without, [16384, 1024]
+    // 18.4 and 13.9, [8192, 2048] 10.8 and 10.4; with the GEMM, [2048, 1024] x [1024, 1024] 11.4 and 11.6, [4096, 1024] x [1024, 1024] 17.6 and 17.0.
+    if (rows > 2048) quant_rowwise_kernel<T, 1, GIVEN, false><<<grid, 256, 0, st>>>(x, (int)K, ldx, given, packed, scale, role);
+    else quant_rowwise_kernel<T, 1, GIVEN, true><<<grid, 256, 0, st>>>(x, (int)K, ldx, given, packed, scale, role);
   } else if (K <= 4096) {
-    quant_rowwise_kernel<T, 2, GIVEN><<<grid, 256, 0, st>>>(x, (int)K, ldx, given, packed, scale, role);
+    quant_rowwise_kernel<T, 2, GIVEN, true><<<grid, 256, 0, st>>>(x, (int)K, ldx, given, packed, scale, role);
   } else if (K <= 8192) {
-    quant_rowwise_kernel<T, 4, GIVEN><<<grid, 256, 0, st>>>(x, (int)K, ldx, given, packed, scale, role);
+    quant_rowwise_kernel<T, 4, GIVEN, true><<<grid, 256, 0, st>>>(x, (int)K, ldx, given, packed, scale, role);
   } else {
-    quant_rowwise_kernel<T, 8, GIVEN><<<grid, 256, 0, st>>>(x, (int)K, ldx, given, packed, scale, role);
+    quant_rowwise_kernel<T, 8, GIVEN, true><<<grid, 256, 0, st>>>(x, (int)K, ldx, given, packed, scale, role);
   }
   I4TC_CUDA(cudaGetLastError());
   return I4TC_OK;

@@ -7,6 +7,7 @@ import pytest
 import torch
 
 from oracle import w4a4_oracle as O
+from tests.helpers import device_us
 
 pytestmark = pytest.mark.gpu
 
@@ -39,6 +40,25 @@ def test_rowwise_bit_exact(tc, M, K, role):
     assert scale.shape == (M,) and scale.dtype == torch.float32
     assert np.array_equal(packed.cpu().numpy(), O.pack_int4(codes))
     assert np.array_equal(scale.cpu().numpy(), s)
+
+
+@pytest.mark.parametrize("M,K", [(2048, 128), (2049, 64), (2049, 264), (2500, 2048), (2049, 2056)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_rowwise_many_short_rows(tc, M, K, dtype):
+    """Both sides of the row count from which short rows do not announce a successor, and rows that leave warps of a block empty."""
+    x = _x(M, K, 11, dtype, zero_rows=(0, M - 1))
+    packed, scale = tc.dynamic_int4_quant(x.cuda())
+    codes, s = O.quant_rowwise(x, "activation")
+    assert np.array_equal(packed.cpu().numpy(), O.pack_int4(codes))
+    assert np.array_equal(scale.cpu().numpy(), s)
+
+
+def test_many_short_rows_cost_no_more_than_their_blocks(tc):
+    """[16384, 256] takes 0.63 of the time of [16384, 2048], eight times the bytes in as many blocks (0.91 when every block announced a
+    successor)."""
+    x = torch.randn(16384, 2048, device="cuda").to(torch.bfloat16)
+    short = x[:, :256].contiguous()
+    assert device_us(lambda: tc.dynamic_int4_quant(short)) < 0.8 * device_us(lambda: tc.dynamic_int4_quant(x))
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
