@@ -220,8 +220,12 @@ int launch_ext(const void* x, int dtype, int64_t rows, int64_t K, int64_t ldx, i
   DeviceGuard guard(device);
   I4TC_CUDA(guard.err);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // the 128-bit kernel does the same arithmetic at a fraction of the instructions
-  if ((smooth == nullptr || ASYM) && K % 32 == 0 && (dtype == I4TC_BF16 || dtype == I4TC_FP16) &&
+  // The 128-bit kernel does the same arithmetic at a fraction of the instructions.  It gives a lane 32 elements of a row, so that short
+  // rows leave lanes without any, and with factors those go through the divisions all the same: many short rows keep the kernel
+  // that fills its warps ([16384, 256] 11.6 us, 128-bit 22.9; [8192, 512] 11.5 and 14.0, [8192, 640] 13.9 and 14.5, [16384, 640] 26.1
+  // and 24.7; groups of 64 [8192, 256] 9.2 and 13.2, [8192, 512] 15.0 and 14.3; up to 2048 rows a launch is the bound).
+  const bool short_rows = smooth != nullptr && rows > 2048 && K <= (group_size == 64 ? 384 : rows <= 8192 ? 640 : 512);
+  if ((smooth == nullptr || ASYM) && !short_rows && K % 32 == 0 && (dtype == I4TC_BF16 || dtype == I4TC_FP16) &&
       grouped_ext_fast_ok(x, ldx, smooth, packed))
     return launch_grouped_ext(ASYM, x, dtype, rows, K, ldx, (int)group_size, (float)clip_ratio, smooth, packed, scale, azp_adj,
                               st);

@@ -53,3 +53,25 @@ def test_extreme_elements(factor, value, dtype):
     sm[37] = factor
     _check(x, sm)
     _check(torch.zeros_like(x), sm)
+
+
+@pytest.mark.parametrize("M,K,gs", [(2048, 256, 128), (2049, 256, 128), (2049, 640, 128), (2049, 768, 128), (2049, 384, 64), (2049, 448, 64)])
+def test_many_short_rows(M, K, gs):
+    """Both sides of the line beyond which short rows keep the general kernel."""
+    gen = torch.Generator(device="cuda").manual_seed(K)
+    _check((torch.randn(M, K, device="cuda", generator=gen) + 0.75).to(torch.bfloat16),
+           (torch.rand(K, device="cuda", generator=gen) + 0.5).to(torch.bfloat16), gs)
+
+
+def test_many_short_rows_are_not_slowed_down():
+    """16384 rows of 256: no slower than rows that the 128-bit kernel cannot take (it needed twice as long)."""
+    from fp8_inference_toolkit_b200 import ops
+    from tests.helpers import device_us
+
+    M, K = 16384, 256
+    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    off = torch.empty(M, K + 8, dtype=x.dtype, device="cuda")[:, 1 : K + 1]
+    off.copy_(x)
+    sm = torch.ones(K, dtype=torch.bfloat16, device="cuda")
+    us = [device_us(lambda: ops.dynamic_int4_quant_asymmetric_clipped_grouped(t, 128, 0.95, sm)) for t in (x, off)]
+    assert us[0] < 1.2 * us[1], us
