@@ -35,9 +35,10 @@ struct Shape {
 // weights); otherwise the candidate with the fewest cost-weighted waves wins.  Weights = measured time per output
 // column relative to 256-wide pair tiles at M = 8192 (per-group | per-channel epilogue): 192-wide pair tiles 1.10 | 1.30,
 // 256-wide single tiles 1.05 | 1.20, 128-wide single tiles 1.25 | 1.45.
-// int8 operands (i8_groups = their K groups, else 0): 192-wide pair tiles 1.10, 256-wide single 1.20, 128-wide single 1.60, pairs from 129
-// rows on, and 1.5 us more for a launch of pairs at 1.3 ns per column and group; over 110 sizes the choice costs 0.7 % against the
-// fastest of the four, with the per-channel weights it was 3.6 %.
+// int8 operands (i8_groups = their K groups, else 0; pairs from 129 rows on): microseconds of a launch, per wave and K group, and per
+// million outputs, fitted to the four shapes at 224 sizes (M 129..4096, N 1000..24576, K 1024..12288).  The choice costs 0.1 % on average
+// and 4 % at most against the fastest of the four.  With weights per column only, few groups, whose tiles are mostly fill and
+// drain, got the wide shapes: 4.0 and 35 % ([4096, 1024] x [4096, 1024] 29.7 us with 256-wide pairs, 22.0 with 192).
 static Shape choose_shape(long long M, long long N, int sms, bool allow_swap, bool group_mode, bool pairs_allowed,
                           double* cost_out = nullptr, int i8_groups = 0) {
   Shape s;
@@ -68,9 +69,9 @@ static Shape choose_shape(long long M, long long N, int sms, bool allow_swap, bo
     s.bn = N >= 16384 ? 256 : 128;
     return s;
   }
-  struct Cand { int bn; bool pair; double w_group, w_channel, w_i8; };
-  const Cand cands[4] = {{256, true, 1.00, 1.00, 1.00}, {192, true, 1.10, 1.30, 1.10}, {256, false, 1.05, 1.20, 1.20},
-                         {128, false, 1.25, 1.45, 1.60}};
+  struct Cand { int bn; bool pair; double w_group, w_channel, i8_launch, i8_group, i8_out; };
+  const Cand cands[4] = {{256, true, 1.00, 1.00, 8.54, 0.274, 0.426}, {192, true, 1.10, 1.30, 6.37, 0.2345, 0.375},
+                         {256, false, 1.05, 1.20, 7.75, 0.321, 0.43}, {128, false, 1.25, 1.45, 4.95, 0.2545, 0.371}};
   double best = 1e30;
   s.bn = 256;
   for (const Cand& c : cands) {
@@ -80,8 +81,8 @@ static Shape choose_shape(long long M, long long N, int sms, bool allow_swap, bo
     const long long units = c.pair ? sms / 2 : sms;
     const long long tiles = rows * ((N + c.bn - 1) / c.bn);
     const long long waves = (tiles + units - 1) / units;
-    double cost = (double)waves * c.bn * (i8_groups ? c.w_i8 : group_mode ? c.w_group : c.w_channel);
-    if (i8_groups && c.pair) cost += 1.5 / (0.0013 * i8_groups);
+    const double cost = i8_groups ? c.i8_launch + (double)waves * i8_groups * c.i8_group + (double)M * N * 1e-6 * c.i8_out
+                                  : (double)waves * c.bn * (group_mode ? c.w_group : c.w_channel);
     if (cost < best) {
       best = cost;
       s.bn = c.bn;

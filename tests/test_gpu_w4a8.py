@@ -111,3 +111,32 @@ def test_full_path_reference_test_14(tc, ops):
     full = x.float() @ w.float().T
     cos = torch.nn.functional.cosine_similarity(out.float().cpu().flatten(), full.flatten(), dim=0)
     assert cos > 0.97
+
+
+@pytest.mark.parametrize("M,K,N", [(300, 1024, 16000), (700, 1024, 4096), (4096, 1024, 4096), (512, 12288, 4096), (257, 1536, 12000)])
+def test_tile_shape_is_near_the_fastest(M, K, N):
+    """Bits do not depend on the tile shape, and the chosen one is within 15 % of the fastest (with few K groups it was up to 35 % off)."""
+    from fp8_inference_toolkit_b200 import ops
+    from tests.helpers import device_us
+
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    a, b = (torch.randint(-127, 128, s, device="cuda", generator=gen).to(torch.int8) for s in ((M, K), (N, K)))
+    sa, sb = (torch.rand(n, device="cuda", generator=gen) for n in (M, N))
+
+    def timed():
+        out = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+        return device_us(lambda: ops.cutlass_w4a8_scaled_mm(a, b, sa, sb, out, M, N, K), 10), out
+
+    chosen, want = timed()
+    best = chosen
+    for width, pairs in ((256, 1), (192, 1), (256, 0), (128, 0)):
+        ops.set_tuning(width, 0)
+        ops.set_cta_pairs(pairs)
+        try:
+            us, out = timed()
+        finally:
+            ops.set_tuning()
+            ops.set_cta_pairs(-1)
+        best = min(best, us)
+        assert torch.equal(out, want)
+    assert chosen < 1.15 * best, (chosen, best)
