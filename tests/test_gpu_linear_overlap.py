@@ -18,9 +18,11 @@ def _separate(x, lin, per_channel):
     out = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
     if per_channel:
         p, s = ops.dynamic_int4_quant(x)
+        torch.cuda.synchronize()
         ops.cutlass_int4_scaled_mm(p, lin.weight_int4, s, lin.weight_scale, out, M, N, K)
     else:
         p, s = ops.dynamic_int4_quant_grouped(x, 128)
+        torch.cuda.synchronize()
         ops.cutlass_int4_fused_grouped_gemm(p, lin.weight_int4, s, lin.weight_scale, out, M, N, 128, K // 128)
     return out
 
@@ -92,6 +94,7 @@ def test_asymmetric_back_to_back(M, K, N, smooth):
     for x in xs:
         out = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
         p, s, z = ops.dynamic_int4_quant_asymmetric_clipped_grouped(x, 128, 0.95, sm)
+        torch.cuda.synchronize()
         ops.cutlass_int4_fused_grouped_gemm_azp(p, wp, s, ws, out, z, cs, M, N, 128, K // 128)
         want.append(out)
     torch.cuda.synchronize()
@@ -112,22 +115,24 @@ def test_weights_written_in_front(M, K, N):
     xp, xs = ops.dynamic_int4_quant_grouped(x, 128)
     x8, x8s = ops.dynamic_int8_quant(x)
 
-    def grouped(w):
+    def grouped(w, between=lambda: None):
         out = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
         p, s = ops.static_int4_weight_quant_grouped(w, 128)
+        between()
         ops.cutlass_int4_fused_grouped_gemm(xp, p, xs, s, out, M, N, 128, K // 128)
         return out
 
-    def int8(w):   # (the int8 rows of the weight stand for the unpacked codes)
+    def int8(w, between=lambda: None):   # (the int8 rows of the weight stand for the unpacked codes)
         out = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
         q, s = ops.dynamic_int8_quant(w)
+        between()
         ops.cutlass_w4a8_scaled_mm(x8, q, x8s, s, out, M, N, K)
         return out
 
     for run in (grouped, int8):
         want = []
         for w in ws:
-            want.append(run(w))
+            want.append(run(w, torch.cuda.synchronize))   # the weights are complete before the GEMM is launched
             torch.cuda.synchronize()
         got = [run(ws[i % 3]) for i in range(12)]   # the packed weights of a call take the memory of the ones before
         for i, out in enumerate(got):

@@ -41,6 +41,25 @@ def test_rows_past_the_destination_are_not_written():
             assert (p[:, r] == 0x5A).all() and (s[:, r] == -1.0).all()
 
 
+def _stage_by_stage(x, ids, wt, w):
+    """The layer with nothing beside anything: every kernel ends before the next is launched, the rows by quantise and copy."""
+    from fp8_inference_toolkit_b200 import moe
+
+    def done(result):
+        torch.cuda.synchronize()
+        return result
+
+    T, k = ids.shape
+    sp, inv, off = done(moe.moe_sort_tokens(ids, w.num_experts))
+    a, sa = done(moe.moe_gather_quant(x, sp, k))
+    h = torch.empty(T * k, 2 * w.inter, dtype=torch.bfloat16, device="cuda")
+    done(moe.moe_w4a4_grouped_gemm(a, sa, w.gate_up_packed, w.gate_up_scale, off, h, 2 * w.inter, w.hidden // 128, w.num_experts))
+    b, sb = done(moe.moe_silu_mul_quant(h))
+    y = torch.empty(T * k, w.hidden, dtype=torch.bfloat16, device="cuda")
+    done(moe.moe_w4a4_grouped_gemm(b, sb, w.down_packed, w.down_scale, off, y, w.hidden, w.inter // 128, w.num_experts))
+    return done(moe.moe_combine(y, inv, wt.contiguous(), T, k))
+
+
 @pytest.mark.parametrize("T", [3, 64, 300, 700])
 def test_layers_back_to_back(T):
     """300 and 700 tokens: the register-fed and the tile kernel."""
@@ -52,10 +71,7 @@ def test_layers_back_to_back(T):
                                 (torch.randn(E, H, I, device="cuda", generator=gen) * 0.02).to(torch.bfloat16))
     xs = [torch.randn(T, H, device="cuda", generator=gen).mul_(2.0 ** i).to(torch.bfloat16) for i in range(4)]
     routes = [moe.moe_route(torch.randn(T, E, device="cuda", generator=gen), k) for _ in range(4)]
-    want = []
-    for x, (ids, wt) in zip(xs, routes):
-        want.append(moe.moe_layer(x, ids, wt, w))
-        torch.cuda.synchronize()
+    want = [_stage_by_stage(x, ids, wt, w) for x, (ids, wt) in zip(xs, routes)]
     got = [moe.moe_layer(xs[i % 4], *routes[i % 4], w) for i in range(24)]
     for i, out in enumerate(got):
         assert torch.equal(out, want[i % 4])
