@@ -64,7 +64,8 @@ def moe_gather_quant(x: torch.Tensor, sorted_pairs: torch.Tensor, top_k: int):
 def moe_quant_gather(x: torch.Tensor, sorted_pairs: torch.Tensor, top_k: int):
     """The result of ``moe_gather_quant`` by quantising every token once and copying its packed row to each of its
     (token, slot) pairs: the quantiser works on whole rows, so the codes and scales are the same, with ``top_k`` times
-    less arithmetic.  Rows of pairs the sort left out (index -1) are left unwritten: no later stage reads them."""
+    less arithmetic.  Rows of pairs the sort left out (index -1) are left unwritten: no later stage reads them.
+    ``moe_layer`` does both in one kernel, ``moe_quant_fanout``."""
     from .ops import dynamic_int4_quant_grouped
 
     _require(x.is_cuda and x.dim() == 2 and x.is_contiguous() and x.dtype == torch.bfloat16,
