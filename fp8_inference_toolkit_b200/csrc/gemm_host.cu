@@ -97,12 +97,14 @@ static Shape choose_shape(long long M, long long N, int sms, bool allow_swap, bo
 // inside the GEMM is the better choice.  Both sides are estimated from measured times (B200, 1965 MHz): columns of tile
 // that an SM pair works through one after another x groups x 2.40 ns (192 / 128-column tiles: 5 / 7 % more) here,
 // 3.78 ns per cost unit of choose_shape there, 1.30 and 1.53 times that with the zero-point term and 2 ns a column here;
-// the expansion moves 1.5 bytes per code at 7.1 TB/s (part of it in L2) and is one more launch.  Fitted to both kernels
-// at 712 sizes (M 129..8192, N 264..24576, K 256..12288, with and without zero points): the choice costs 0.5 % on
-// average against the faster of the two.  Around the line (expanded, best width | in-kernel):
-// [256, 4096] x [6144, 4096] 27.5 | 28.1 us, with zero points 31.2 | 39.4; [256, 4096] x [24576, 4096] 65 | 70 and one row
-// more 92 | 74; [512, 4096] x [24576, 4096] 93 | 99, with zero points 114 | 152; [1000, 1024] x [1000, 1024] 14.8 | 13.1,
-// with zero points 14.8 | 15.9.
+// the expansion moves 1.5 bytes per code at 7.1 TB/s (part of it in L2) and is one more launch.  The constants were fitted to
+// kernels that did not yet start under the end of their predecessors.  With those that do, over 154 sizes (M 129..4096,
+// N 1000..24576, K 512..12288; i4tc_linear | with zero points | the GEMM by itself | with zero points), the choice costs
+// against the fastest kernel and width 0.0 | 0.0 | 0.0 | 0.1 % on average for K above 2048 (at most 3.4) and
+// 14 | 9 | 10 | 7 % for K up to 2048, where fill, drain and the hidden expansion count for more than columns.  Whole calls
+// around the line (expanded, best width | in-kernel): [256, 4096] x [6144, 4096] 23.6 | 26.6 us, with zero points 28.7 | 38.2;
+// [256, 4096] x [24576, 4096] 64 | 68 and one row more 91 | 73; [512, 4096] x [24576, 4096] 92 | 102, with zero points
+// 113 | 150; [1000, 1024] x [1000, 1024] 11.9 | 14.0 (in-kernel is chosen), with zero points 14.7 | 18.4.
 static int choose_f8(long long M, long long N, int G, const DeviceInfo& dev, bool azp) {
   const int sms = dev.sm_count;
   if (g_force_bn != 0 || g_force_swap >= 0 || g_force_splits != 0 || g_cta_pairs >= 0 || g_epi_warps != 0 ||
