@@ -36,8 +36,8 @@ struct Shape {
 // column relative to 256-wide pair tiles at M = 8192 (per-group | per-channel epilogue): 192-wide pair tiles 1.10 | 1.30,
 // 256-wide single tiles 1.05 | 1.20, 128-wide single tiles 1.25 | 1.45.
 // int8 operands (i8_groups = their K groups, else 0; pairs from 129 rows on): microseconds of a launch, per wave and K group, and per
-// million outputs, fitted to the four shapes at 224 sizes (M 129..4096, N 1000..24576, K 1024..12288).  The choice costs 0.1 % on average
-// and 4 % at most against the fastest of the four.  With weights per column only, few groups, whose tiles are mostly fill and
+// million outputs, fitted to the four shapes at 224 sizes (M 129..4096, N 1000..24576, K 1024..12288).  The choice costs 0.2 % on average
+// and 8 % at most against the fastest of the four.  With weights per column only, few groups, whose tiles are mostly fill and
 // drain, got the wide shapes: 4.0 and 35 % ([4096, 1024] x [4096, 1024] 29.7 us with 256-wide pairs, 22.0 with 192).
 static Shape choose_shape(long long M, long long N, int sms, bool allow_swap, bool group_mode, bool pairs_allowed,
                           double* cost_out = nullptr, int i8_groups = 0) {
@@ -70,8 +70,8 @@ static Shape choose_shape(long long M, long long N, int sms, bool allow_swap, bo
     return s;
   }
   struct Cand { int bn; bool pair; double w_group, w_channel, i8_launch, i8_group, i8_out; };
-  const Cand cands[4] = {{256, true, 1.00, 1.00, 8.54, 0.274, 0.426}, {192, true, 1.10, 1.30, 6.37, 0.2345, 0.375},
-                         {256, false, 1.05, 1.20, 7.75, 0.321, 0.43}, {128, false, 1.25, 1.45, 4.95, 0.2545, 0.371}};
+  const Cand cands[4] = {{256, true, 1.00, 1.00, 8.74, 0.280, 0.417}, {192, true, 1.10, 1.30, 6.20, 0.240, 0.368},
+                         {256, false, 1.05, 1.20, 8.09, 0.324, 0.412}, {128, false, 1.25, 1.45, 5.15, 0.251, 0.364}};
   double best = 1e30;
   s.bn = 256;
   for (const Cand& c : cands) {
