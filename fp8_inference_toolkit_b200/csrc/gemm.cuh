@@ -62,10 +62,10 @@ struct GemmParams {
 };
 
 // out[i] = bf16(sum_s ws[s * stride + i]), s ascending.
-int launch_split_reduce(const float* ws, long long stride, int splits, long long n, void* out, bool overlap, cudaStream_t st);
+int launch_split_reduce(const float* ws, long long stride, int splits, long long n, void* out, cudaStream_t st);
 // out[m, n] = cast((sum_s ws[s * stride + m * N + n] * sb[n]) * sa[m]): the ranges hold exact integer sums.
 int launch_split_reduce_scaled(const float* ws, long long stride, int splits, long long M, long long N, const float* sa,
-                               const float* sb, void* out, int out_dtype, bool overlap, cudaStream_t st);
+                               const float* sb, void* out, int out_dtype, cudaStream_t st);
 
 // What became of a launch of CTA pairs (clusters of two) that did not succeed.
 struct PairLaunch {

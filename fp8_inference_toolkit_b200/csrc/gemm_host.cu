@@ -300,9 +300,9 @@ static int run_dense(const DenseArgs& d, int device, void* stream) {
   if (int rc = launch_w4a4_gemm(p, tmP, tmQ, sh.bn, grid, false, epi_warps_for(d.epi_mode), static_cast<cudaStream_t>(stream))) return rc;
   if (p.splits > 1) {
     if (d.epi_mode == EPI_CHANNEL)
-      return launch_split_reduce_scaled(p.split_ws, p.ws_stride, p.splits, d.M, d.N, d.sa, d.sb, d.out, d.out_dtype, true,
+      return launch_split_reduce_scaled(p.split_ws, p.ws_stride, p.splits, d.M, d.N, d.sa, d.sb, d.out, d.out_dtype,
                                         static_cast<cudaStream_t>(stream));
-    return launch_split_reduce(p.split_ws, p.ws_stride, p.splits, d.M * d.N, d.out, true, static_cast<cudaStream_t>(stream));
+    return launch_split_reduce(p.split_ws, p.ws_stride, p.splits, d.M * d.N, d.out, static_cast<cudaStream_t>(stream));
   }
   return I4TC_OK;
 }
@@ -462,7 +462,7 @@ extern "C" int i4tc_gemm_grouped_scratch(const uint8_t* a, const uint8_t* b, con
 
 // One or two bf16 tokens against per-group scales, where the CUDA-core kernel is the one chosen (run_dense) and its 16-byte loads
 // suit: it quantises the tokens as well, where that pays (gemv_quant_pays).  A second launch costs the host and the device more than
-// every block's own pass over a few thousand elements: [1, 4096] x [6144, 4096] 23.9 -> 20.3 us a call.  Everything else, refused calls
+// every block's own pass over a few thousand elements: [1, 4096] x [6144, 4096] 23.0 -> 20.1 us a call.  Everything else, refused calls
 // among them, takes the two kernels.  (An output that overlaps the activations does too: blocks here end at different times.)
 static bool linear_in_one_kernel(const void* x, int dtype, int64_t M, int64_t K, int64_t ldx, const uint8_t* w, const float* w_scale,
                                  const uint8_t* x_packed, const float* x_scale, const void* out, int64_t N) {

@@ -979,19 +979,19 @@ __global__ void __launch_bounds__(256) split_reduce_scaled_kernel(const float* _
 }
 
 int launch_split_reduce_scaled(const float* ws, long long stride, int splits, long long M, long long N, const float* sa,
-                               const float* sb, void* out, int out_dtype, bool overlap, cudaStream_t st) {
+                               const float* sb, void* out, int out_dtype, cudaStream_t st) {
   const dim3 blocks((unsigned)((M * N + 255) / 256));
   if (out_dtype == I4TC_FP16)
-    I4TC_CUDA(launch_kernel(overlap, split_reduce_scaled_kernel<__half>, blocks, 256, 0, st, ws, stride, splits, M, N, sa, sb,
+    I4TC_CUDA(launch_kernel(true, split_reduce_scaled_kernel<__half>, blocks, 256, 0, st, ws, stride, splits, M, N, sa, sb,
                             static_cast<__half*>(out)));
   else
-    I4TC_CUDA(launch_kernel(overlap, split_reduce_scaled_kernel<__nv_bfloat16>, blocks, 256, 0, st, ws, stride, splits, M, N, sa, sb,
+    I4TC_CUDA(launch_kernel(true, split_reduce_scaled_kernel<__nv_bfloat16>, blocks, 256, 0, st, ws, stride, splits, M, N, sa, sb,
                             static_cast<__nv_bfloat16*>(out)));
   return I4TC_OK;
 }
 
-int launch_split_reduce(const float* ws, long long stride, int splits, long long n, void* out, bool overlap, cudaStream_t st) {
-  I4TC_CUDA(launch_kernel(overlap, split_reduce_kernel, dim3((unsigned)((n + 1023) / 1024)), 256, 0, st, ws, stride, splits, n,
+int launch_split_reduce(const float* ws, long long stride, int splits, long long n, void* out, cudaStream_t st) {
+  I4TC_CUDA(launch_kernel(true, split_reduce_kernel, dim3((unsigned)((n + 1023) / 1024)), 256, 0, st, ws, stride, splits, n,
                           static_cast<__nv_bfloat16*>(out)));
   return I4TC_OK;
 }
