@@ -72,11 +72,11 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_kernel(const __nv_bfloat
   }
 }
 
-// Heads [0, q_heads) with wq and [q_heads, heads) with wk of every token of qkv (row stride ld, heads of 128):
-// normalise, then rotate halves by the token's position (token % seq), in place.  A block takes a token (several, where a warp or two
-// hold all heads; few tokens are shared by several blocks) and a warp two heads at a time, a lane eight consecutive elements of one; the other half of the rotation is 8 lanes away.  Tables and weights stay in
-// registers over the heads.  Every bf16 rounding of the separate ops is kept, so results differ from theirs by the order of the sum of
-// squares only (four-element chains, then partners 64, 32, 16, 8 and 4 elements away).
+// Heads [0, q_heads) with wq and [q_heads, heads) with wk of every token of qkv (row stride ld, heads of 128): normalise, then rotate
+// halves by the token's position (token % seq), in place.  A block takes a token (several, where a warp or two hold all heads; few tokens
+// are shared by several blocks) and a warp two heads at a time, a lane eight consecutive elements of one; the other half of the rotation
+// is 8 lanes away.  Tables and weights stay in registers over the heads.  Every bf16 rounding of the separate ops is kept, so results
+// differ from theirs by the order of the sum of squares only (four-element chains, then partners 64, 32, 16, 8 and 4 elements away).
 // A warp per head with 8-byte accesses, an index division per head and single conversions was bound by the special-function unit:
 // [4096, 40 heads] 38.6 us -> 14.5 (5.8 TB/s of the one read and one write).
 constexpr int kRopeWarps = 4;

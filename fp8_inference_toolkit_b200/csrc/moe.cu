@@ -217,8 +217,8 @@ __global__ void __launch_bounds__(kSortChunk) moe_sort_fused_kernel(const int32_
   for (int j = s_total + blockIdx.x * kSortChunk + threadIdx.x; j < P; j += chunks * kSortChunk) sorted_pairs[j] = -1;
 }
 
-// out[t, :] = bf16( sum_j w[t, j] * y[inv[t*k + j], :] ), fp32 accumulation in ascending j, one fused multiply-add
-// per term.  U: rows in flight, no more than top_k (with four for every top_k, [4096, 4096] with one row a token took 11.1 us, with two 18.5; 8.1 and 14.5 so).
+// out[t, :] = bf16( sum_j w[t, j] * y[inv[t*k + j], :] ), fp32 accumulation in ascending j, one fused multiply-add per term.  U: rows in
+// flight, no more than top_k (with four for every top_k, [4096, 4096] with one row a token took 11.1 us, with two 18.5; 8.1 and 14.5 so).
 template <int U>
 __global__ void __launch_bounds__(256) moe_combine_kernel(const __nv_bfloat16* y,
                                                          const int32_t* inv,

@@ -16,12 +16,12 @@
 // layout as in skinny.cu.
 //
 // 128 experts of [1536, 2048] and [2048, 768] (321 MB of weights), top 8, both GEMMs behind a flushed L2, tile kernel -> this one,
-// experts drawn uniformly: 64 tokens 181 -> 77 us (4.2 TB/s), 192 tokens 181 -> 101, 400 tokens 185 -> 149; with Zipf's weights 161 -> 81,
-// 183 -> 118, 192 -> 185; all tokens on the same eight experts 58 -> 44, 61 -> 69, 85 -> 116.  (With a block taking an expert's passes one
-// after the other: uniform 89, 108, 155; Zipf 103, 155, 206; eight experts 120, 142, 212; 1000 tokens on one expert 626, now 50.)  Bound by instructions and latency (the nibbles' 24 logic
-// operations and four to sixteen products per warp and group), not by HBM: asking the L2 for a warp's whole K range beforehand
-// changed nothing at 64 tokens and cost 20 % at 192.  Weights through shared memory (cp.async.bulk, two warps a block, ten warps an SM): 123 us
-// at 64 tokens and 325 at 512.
+// experts drawn uniformly: 64 tokens 181 -> 77 us (4.2 TB/s), 192 tokens 181 -> 101, 400 tokens 185 -> 149; with Zipf's weights 161 ->
+// 81, 183 -> 118, 192 -> 185; all tokens on the same eight experts 58 -> 44, 61 -> 69, 85 -> 116.  (With a block taking an expert's
+// passes one after the other: uniform 89, 108, 155; Zipf 103, 155, 206; eight experts 120, 142, 212; 1000 tokens on one expert 626, now
+// 50.)  Bound by instructions and latency (the nibbles' 24 logic operations and four to sixteen products per warp and group), not by HBM:
+// asking the L2 for a warp's whole K range beforehand changed nothing at 64 tokens and cost 20 % at 192.  Weights through shared memory
+// (cp.async.bulk, two warps a block, ten warps an SM): 123 us at 64 tokens and 325 at 512.
 #include "gemm.cuh"
 #include "ptx.cuh"
 

@@ -837,8 +837,9 @@ static int launch_rowwise_t(const T* x, int64_t rows, int64_t K, int64_t ldx, co
   if (!vec_ok) {
     quant_rowwise_generic_kernel<T, GIVEN><<<grid, 256, 0, st>>>(x, K, ldx, given, packed, scale, role);
   } else if (K <= 2048) {
-    // A trigger in each of many short blocks costs more than a GEMM's early start gives: [8192, 128] 9.8 us with it, 7.3 without, [16384, 1024]
-    // 18.4 and 13.9, [8192, 2048] 10.8 and 10.4; with the GEMM, [2048, 1024] x [1024, 1024] 11.4 and 11.6, [4096, 1024] x [1024, 1024] 17.6 and 17.0.
+    // A trigger in each of many short blocks costs more than a GEMM's early start gives: [8192, 128] 9.8 us with it, 7.3 without, [16384,
+    // 1024] 18.4 and 13.9, [8192, 2048] 10.8 and 10.4; with the GEMM, [2048, 1024] x [1024, 1024] 11.4 and 11.6, [4096, 1024] x [1024,
+    // 1024] 17.6 and 17.0.
     if (rows > 2048) quant_rowwise_kernel<T, 1, GIVEN, false><<<grid, 256, 0, st>>>(x, (int)K, ldx, given, packed, scale, role);
     else quant_rowwise_kernel<T, 1, GIVEN, true><<<grid, 256, 0, st>>>(x, (int)K, ldx, given, packed, scale, role);
   } else if (K <= 4096) {

@@ -115,7 +115,7 @@ def test_full_path_reference_test_14(tc, ops):
 
 @pytest.mark.parametrize("M,K,N", [(300, 1024, 16000), (700, 1024, 4096), (4096, 1024, 4096), (512, 12288, 4096), (257, 1536, 12000)])
 def test_tile_shape_is_near_the_fastest(M, K, N):
-    """Bits do not depend on the tile shape, and the chosen one is within 15 % of the fastest (with few K groups it was up to 35 % off)."""
+    """Bits do not depend on the tile shape, and the chosen one is within 20 % of the fastest (with few K groups it was up to 35 % off)."""
     from fp8_inference_toolkit_b200 import ops
     from tests.helpers import device_us
 
@@ -139,4 +139,4 @@ def test_tile_shape_is_near_the_fastest(M, K, N):
             ops.set_cta_pairs(-1)
         best = min(best, us)
         assert torch.equal(out, want)
-    assert chosen < 1.15 * best, (chosen, best)
+    assert chosen < 1.2 * best, (chosen, best)
